@@ -72,8 +72,102 @@ __global__ void cb_norm_kernel(const float* cb, int M, int dsub, float* out) {
     out[idx] = acc;
 }
 
-// PQ encode: one warp per (vector, sub-quantizer); exhaustive nearest codeword under the
-// canonical fp32 distance, first minimum wins.
+// PQ encode for sub-vectors of DS = 2 .. 32 components: exhaustive nearest codeword under the canonical
+// fp32 distance (sequential fmaf over the components), first minimum wins.  A thread owns V vectors
+// of one sub-quantizer and walks the 256 codewords, which its CTA holds in shared memory as negated
+// pairs (codewords 2p and 2p + 1 side by side): every load is a broadcast, and one packed add and one
+// packed fma advance two distances, each with the rounding of the scalar instruction.
+// Bound by the fp32 pipe: 2 * 256 * DS operations per sub-vector (0.55 ms for 300 000 vectors of 16
+// sub-quantizers with DS = 8).  The warp-per-(vector, sub-quantizer) form it replaces re-read every
+// codeword from L1 for every vector: 10.9 ms there, 0.84 ms here.
+__device__ __forceinline__ uint64_t f32x2_pack(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void f32x2_unpack(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+constexpr int kEncThreads = 128;
+constexpr int enc_vectors(int ds) { return ds <= 8 ? 2 : 1; }   // per thread: 4 * DS registers of operands at V = 2
+
+template <int DS>
+__global__ void __launch_bounds__(kEncThreads)
+encode_tiled_kernel(const float* x, int64_t n, int d, int M, const float* cb, const float* centroids,
+                    const int32_t* list_no, uint8_t* codes) {
+    constexpr int V = enc_vectors(DS);
+    __shared__ __align__(16) float neg[kKsub / 2][DS][2];
+    const int m = blockIdx.y;
+    const float* cbm = cb + static_cast<int64_t>(m) * kKsub * DS;
+    for (int i = threadIdx.x; i < kKsub * DS; i += kEncThreads) {
+        const int j = i / DS, t = i % DS;
+        neg[j >> 1][t][j & 1] = -__ldg(cbm + i);
+    }
+    __syncthreads();
+    for (int64_t v0 = static_cast<int64_t>(blockIdx.x) * (kEncThreads * V) + threadIdx.x; v0 < n;
+         v0 += static_cast<int64_t>(gridDim.x) * (kEncThreads * V)) {
+        uint64_t r[V][DS];
+#pragma unroll
+        for (int u = 0; u < V; ++u) {
+            const int64_t v = min(v0 + u * kEncThreads, n - 1);   // a lane past the end repeats the last vector
+            const float* xv = x + v * d + m * DS;
+            const float* cv = centroids ? centroids + static_cast<int64_t>(__ldg(list_no + v)) * d + m * DS : nullptr;
+#pragma unroll
+            for (int t = 0; t < DS; ++t) {
+                const float e = centroids ? __ldg(xv + t) - __ldg(cv + t) : __ldg(xv + t);
+                r[u][t] = f32x2_pack(e, e);
+            }
+        }
+        float best[V];
+        int arg[V];
+#pragma unroll
+        for (int u = 0; u < V; ++u) {
+            best[u] = __int_as_float(0x7f800000);
+            arg[u] = 0;
+        }
+#pragma unroll 2
+        for (int p = 0; p < kKsub / 2; ++p) {
+            const ulonglong2* c2 = reinterpret_cast<const ulonglong2*>(&neg[p][0][0]);
+            uint64_t acc[V];
+#pragma unroll
+            for (int u = 0; u < V; ++u) acc[u] = 0ull;   // (+0, +0)
+#pragma unroll
+            for (int t = 0; t < DS; t += 2) {
+                const ulonglong2 c = c2[t >> 1];
+#pragma unroll
+                for (int u = 0; u < V; ++u) {
+                    uint64_t df = f32x2_add(r[u][t], c.x);
+                    acc[u] = f32x2_fma(df, df, acc[u]);
+                    df = f32x2_add(r[u][t + 1], c.y);
+                    acc[u] = f32x2_fma(df, df, acc[u]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < V; ++u) {
+                float lo, hi;
+                f32x2_unpack(acc[u], lo, hi);
+                if (lo < best[u]) { best[u] = lo; arg[u] = 2 * p; }
+                if (hi < best[u]) { best[u] = hi; arg[u] = 2 * p + 1; }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < V; ++u)
+            if (v0 + u * kEncThreads < n) codes[(v0 + u * kEncThreads) * M + m] = static_cast<uint8_t>(arg[u]);
+    }
+}
+
+// Any other sub-vector length: one warp per (vector, sub-quantizer).
 __global__ void encode_kernel(const float* x, int64_t n, int d, int M, int dsub, const float* cb, int by_residual,
                               const float* centroids, const int32_t* list_no, uint8_t* codes) {
     const int64_t task = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1581,6 +1675,31 @@ cudaError_t launch_collect(const ScanArgs& a, int nslots, uint32_t* cpos, uint32
 }
 
 inline unsigned blocks_for(int64_t n, int threads) { return static_cast<unsigned>((n + threads - 1) / threads); }
+// centroids: nullptr for raw encoding
+cudaError_t launch_encode(const float* x, int64_t n, int d, int M, int dsub, const float* cb, const float* centroids,
+                          const int32_t* list_no, int num_sms, uint8_t* codes, cudaStream_t st) {
+#define B200_ENC_CASE(DS)                                                                                         \
+    case DS: {                                                                                                    \
+        const int64_t per = kEncThreads * enc_vectors(DS);                                                        \
+        /* several CTAs per SM, each with enough vectors to pay for staging its codebook */                       \
+        const int64_t gx = std::min<int64_t>((n + per - 1) / per, std::max(1, 32 * num_sms / M));                 \
+        encode_tiled_kernel<DS><<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(M)), kEncThreads, 0, st>>>( \
+            x, n, d, M, cb, centroids, list_no, codes);                                                           \
+        break;                                                                                                    \
+    }
+    switch (dsub) {
+        B200_ENC_CASE(2)
+        B200_ENC_CASE(4)
+        B200_ENC_CASE(8)
+        B200_ENC_CASE(16)
+        B200_ENC_CASE(32)
+        default:
+            encode_kernel<<<blocks_for(n * M, 8), 256, 0, st>>>(x, n, d, M, dsub, cb, centroids ? 1 : 0, centroids,
+                                                                list_no, codes);
+    }
+#undef B200_ENC_CASE
+    return cudaGetLastError();
+}
 inline int pow2_ceil_int(int v) {
     int p = 1;
     while (p < v) p <<= 1;
@@ -1773,9 +1892,8 @@ void IvfpqIndex::add(int64_t n, const float* x, const int64_t* ids, bool x_on_de
         B200_CUDA_CHECK(launch_check_range_i32(ln, m, nlist_, vflag, st));
         if (read_flag()) throw std::invalid_argument("add: a vector could not be assigned to a list (distance overflow)");
         uint8_t* cd = static_cast<uint8_t*>(w_codes_.ensure(static_cast<size_t>(m) * M_));
-        encode_kernel<<<blocks_for(m * M_, 8), 256, 0, st>>>(xd, m, d_, M_, dsub_, codebooks_.as<float>(),
-                                                             by_residual_ ? 1 : 0, coarse_->rows_f32(), ln, cd);
-        B200_CUDA_CHECK(cudaGetLastError());
+        B200_CUDA_CHECK(launch_encode(xd, m, d_, M_, dsub_, codebooks_.as<float>(),
+                                      by_residual_ ? coarse_->rows_f32() : nullptr, ln, num_sms_, cd, st));
         float* t2 = nullptr;
         if (by_residual_) {
             t2 = static_cast<float*>(w_t2_.ensure(static_cast<size_t>(m) * 4));
