@@ -145,6 +145,8 @@ struct RowEpilogue {
     __half2 rq2;              // cosine: the row's query term
     AccT tau, tau_up;
     float tq;                 // FOLD append: the row's threshold, for the approximate key
+    float bias;               // FOLD append over a segmented base: what the accumulator lacks to (tau - key) / 2
+    uint32_t admit_all;       // all ones when the row's threshold admits every key (no difference to it can be formed)
     int blk_q;                // row of the open candidate block (-1: none)
     uint32_t blk_next, blk_left;
     uint32_t pre_base;        // a second block reserved ahead of need (its atomic is issued at the end of a
@@ -153,7 +155,7 @@ struct RowEpilogue {
 
     __device__ __forceinline__ explicit RowEpilogue(const GemmArgs& a_)
         : a(a_), q(-1), row_ok(false), l2(!IPONLY && a_.metric == kMetricL2),
-          tau(AccT(0)), tau_up(AccT(0)), tq(0.f),
+          tau(AccT(0)), tau_up(AccT(0)), tq(0.f), bias(0.f), admit_all(0u),
           blk_q(-1), blk_next(0), blk_left(0), pre_base(0), pre_ok(false) {}
 
     // 32 filter bits of this row for base positions col0 .. col0 + 31 (col0 is a multiple of 32).
@@ -197,9 +199,11 @@ struct RowEpilogue {
             }
             if (FOLD && !a.direct) {
                 tq = ord_to_float(to);
+                if (a.seg_bias) bias = __ldg(a.seg_bias + q);
             } else {
                 tau = K::tau(to);
                 tau_up = K::above(tau);
+                admit_all = tau == tau_up ? 0xFFFFFFFFu : 0u;
             }
         }
     }
@@ -280,6 +284,10 @@ struct RowEpilogue {
         } else {
             // (the tcgen05 kernel calls fold_mask / fold_extract itself, with the accumulator handed
             // back in between; this is the path of the CUDA-core variant)
+            if (a.seg_bias) {
+                seg_fold_extract(r, seg_fold_mask(r, nvalid), col0);
+                return;
+            }
             const uint32_t m = fold_mask(r, col0, nvalid);
             fold_extract(r, m, col0);
         }
@@ -309,6 +317,29 @@ struct RowEpilogue {
         if (a.qmask && row_ok) mask &= __brev(mask_word(col0));
         return hit ? mask : 0u;
     }
+    // Segmented base: the threshold is the candidate row's own (bias), so it joins the accumulator here.
+    // The registers keep D without it: the key is read from them directly, and with a threshold of
+    // +infinity every column whose key is a number passes, infinite keys included.
+    __device__ __forceinline__ uint32_t seg_fold_mask(const uint32_t (&r)[32], int nvalid) {
+        uint32_t m0 = 0, m1 = 0;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            m0 = __funnelshift_l(__float_as_uint(__uint_as_float(r[c]) + bias), m0, 1);
+            m1 = __funnelshift_l(__float_as_uint(__uint_as_float(r[16 + c]) + bias), m1, 1);
+        }
+        const uint32_t mask = ~((m0 << 16) | (m1 & 0xFFFFu)) & (nvalid >= 32 ? 0xFFFFFFFFu : ~(0xFFFFFFFFu >> nvalid));
+        return row_ok ? mask : 0u;
+    }
+    __device__ __forceinline__ void seg_fold_extract(const uint32_t (&r)[32], uint32_t mask, int64_t col0) {
+        while (mask) {
+            const uint32_t c = __clz(mask);
+            mask &= ~(0x80000000u >> c);
+            const float dv = __uint_as_float(pick(r, c));
+            const float key = l2 ? -2.f * dv : -dv;
+            if (key != key) continue;   // NaN
+            append(pack_cand(float_to_ord(key), static_cast<uint32_t>(col0 + c)));
+        }
+    }
     // fold_extract: appends the columns of `mask` from the registers (select tree; no TMEM access).
     __device__ __forceinline__ void fold_extract(const uint32_t (&r)[32], uint32_t mask, int64_t col0) {
         while (mask) {
@@ -334,7 +365,7 @@ struct RowEpilogue {
         uint32_t mask = (m0 << 16) | (m1 & 0xFFFFu);
         uint32_t valid = nvalid >= 32 ? 0xFFFFFFFFu : ((1u << nvalid) - 1u);
         if (a.qmask && row_ok) valid &= mask_word(col0);
-        return row_ok ? (mask & __brev(valid)) : 0u;
+        return row_ok ? ((mask | admit_all) & __brev(valid)) : 0u;
     }
     __device__ __forceinline__ void ip_extract(const uint32_t (&r)[32], uint32_t mask, int64_t col0) {
         while (mask) {
@@ -365,7 +396,7 @@ struct RowEpilogue {
         uint32_t mask = (m0 << 16) | (m1 & 0xFFFFu);
         uint32_t valid = nvalid >= 32 ? 0xFFFFFFFFu : ((1u << nvalid) - 1u);
         if (a.qmask && row_ok) valid &= mask_word(col0);
-        return row_ok ? (mask & __brev(valid)) : 0u;
+        return row_ok ? ((mask | admit_all) & __brev(valid)) : 0u;
     }
     __device__ __forceinline__ void l2_extract(const uint32_t (&r)[32], uint32_t mask, int64_t col0, const uint32_t* gn) {
         while (mask) {
@@ -484,7 +515,7 @@ struct RowEpilogue {
                 }
             }
             uint32_t mask = (m0 << 16) | (m1 & 0xFFFFu);
-            mask &= __brev(valid);   // rows past the end of the base, rows the filter excludes
+            mask = (mask | admit_all) & __brev(valid);   // rows past the end of the base, rows the filter excludes
             while (mask) {
                 const uint32_t c = __clz(mask);
                 mask &= ~(0x80000000u >> c);
@@ -867,7 +898,9 @@ dist_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
             const int64_t half_col0 = tile_col0 + half * kCols;
             // sixteen-warp L2: the generic chunk code (sample pass, direct mode) reads the norms from global memory too
             const uint32_t* hnorm = l2_global(KIND) ? gnorm + tile_col0 + half * kCols : &epi_sh.norm[ab][half * kCols];
-            const int hslot = sel * (kTileB / BURST) + half * (kCols / BURST);
+            // first burst slot: counted from the pass's first tile, or from the first tile of the segment
+            const int slot_tile = a.seg_index ? tile - static_cast<int>(cbase / kTileB) : sel;
+            const int hslot = slot_tile * (kTileB / BURST) + half * (kCols / BURST);
             uint32_t ra[32], rb[32];
             if (KIND == kKindI8Cos && MODE == kModeAppend && kCols == 64 && !a.direct) {
                 // cosine: the accumulators of both chunks become ordered fp16 scores in place (the
@@ -934,8 +967,20 @@ dist_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
                 ptx::tmem_ld_wait(ra);
                 ptx::tmem_ld_wait(rb);
                 const int64_t rem_a = n_end - half_col0, rem_b = rem_a - 32;
-                const uint32_t ma = epi.fold_mask(ra, half_col0, rem_a >= 32 ? 32 : (rem_a > 0 ? static_cast<int>(rem_a) : 0));
-                const uint32_t mb = epi.fold_mask(rb, half_col0 + 32, rem_b >= 32 ? 32 : (rem_b > 0 ? static_cast<int>(rem_b) : 0));
+                const int va = rem_a >= 32 ? 32 : (rem_a > 0 ? static_cast<int>(rem_a) : 0);
+                const int vb = rem_b >= 32 ? 32 : (rem_b > 0 ? static_cast<int>(rem_b) : 0);
+                if (a.seg_bias) {
+                    const uint32_t ma = epi.seg_fold_mask(ra, va), mb = epi.seg_fold_mask(rb, vb);
+                    ptx::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(&bar_acc_empty[ab]);
+                    epi.seg_fold_extract(ra, ma, half_col0);
+                    epi.seg_fold_extract(rb, mb, half_col0 + 32);
+                    epi.end_tile(hslot);
+                    continue;
+                }
+                const uint32_t ma = epi.fold_mask(ra, half_col0, va);
+                const uint32_t mb = epi.fold_mask(rb, half_col0 + 32, vb);
                 ptx::tc_fence_before();
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&bar_acc_empty[ab]);
@@ -1061,6 +1106,7 @@ dist_gemm_simt_kernel(const GemmArgs a) {
             cbase = a.seg_col0[tile];
             n_end = a.seg_end[tile];
         }
+        const int slot_tile = a.seg_index ? tile - static_cast<int>(cbase / kTileB) : sel;
         __syncthreads();
         for (int h = 0; h < kTileB; h += kTileQ) {
             uint32_t nv = (l2 || cosm) ? __ldg(gnorm + tile_col0 + h + threadIdx.x) : 0u;
@@ -1084,10 +1130,10 @@ dist_gemm_simt_kernel(const GemmArgs a) {
                 if (is_i8(KIND)) r[j] = static_cast<uint32_t>(acc);
                 else r[j] = __float_as_uint(acc);
             }
-            const int bslot = sel * (kTileB / BURST) + c * (32 / BURST);
+            const int bslot = slot_tile * (kTileB / BURST) + c * (32 / BURST);
             epi.chunk(r, &epi_sh.norm[0][c * 32], col0, nvalid, bslot, c, cbase);
         }
-        epi.end_tile(sel * (kTileB / BURST));
+        epi.end_tile(slot_tile * (kTileB / BURST));
     }
     epi.finish();
 }

@@ -87,12 +87,16 @@ struct GemmArgs {
     //   seg_index: which index; the candidates of (index i, query q) go to row
     //              (i - seg_first) * nq + q of cand / tau (direct mode only)
     //   seg_col0 : position of the index's first base row in the concatenated base (the slot of a
-    //              candidate is its position minus this)
+    //              candidate is its position minus this; burst minima count their slots from it too)
     //   seg_end  : position one past the index's last real base row
+    // With thresholds (direct = 0) tau, counts, cand and mins are per candidate row.  Folded operands
+    // then carry no threshold terms (those sit in the query operand, which all members share):
+    // seg_bias[row] is added to the accumulator before its sign is tested.
     const int32_t* seg_index;
     int seg_first;        // index of the first member this pass covers
     const int64_t* seg_col0;
     const int64_t* seg_end;
+    const float* seg_bias;
     int* err;             // device error word
     // optional phase profile (nullptr = off): 8 counters of SM cycles summed over CTAs
     //   0 producer wait-empty   1 mma wait-acc-empty   2 mma wait-full   3 epilogue wait-acc-full

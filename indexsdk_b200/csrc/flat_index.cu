@@ -345,6 +345,15 @@ void FlatIndex::run_page(int nq, const void* xq_raw, const void* xq_op_in, int k
     uint64_t* cand = static_cast<uint64_t*>(w_cand_.ensure(static_cast<size_t>(nq) * plan.cap * 8));
     uint32_t* counts = static_cast<uint32_t*>(w_counts_.ensure(static_cast<size_t>(nq) * 4));
 
+    TauFold fold;
+    if (dtype_ == kF32) {
+        // the full pass tests "key <= tau" inside the GEMM: the threshold joins the query operand
+        fold.qnorm = static_cast<const float*>(qnorm);
+        fold.ymax = max_norm_;
+        fold.d = d_;
+        fold.metric = metric_;
+        fold.q_bf16 = const_cast<void*>(xq_op);
+    }
     if (plan.sampled) {
         // 3a. sample pass -> per-burst minima -> threshold
         const int stride = plan.s_tiles * (kTileB / plan.burst);
@@ -357,14 +366,9 @@ void FlatIndex::run_page(int nq, const void* xq_raw, const void* xq_op_in, int k
         L.burst = plan.burst;
         a.prof = prof_ ? w_prof_.as<unsigned long long>() : nullptr;
         B200_CUDA_CHECK(launch_dist_gemm(L, a, &map_a, &map_b_, stream_));
-        B200_CUDA_CHECK(launch_kth_threshold(mins, stride, stride, nq, k, eps, tau_all, tau, stream_));
-        if (dtype_ == kF32) {
-            // the full pass tests "key <= tau" inside the GEMM: the threshold joins the query operand
-            B200_CUDA_CHECK(launch_fold_tau(tau, static_cast<const float*>(qnorm), max_norm_, nq, d_, metric_,
-                                            const_cast<void*>(xq_op), stream_));
-            stats_.kernel_launches += 1;
-        }
-        B200_CUDA_CHECK(cudaMemsetAsync(counts, 0, static_cast<size_t>(nq) * 4, stream_));
+        fold.counts = counts;
+        B200_CUDA_CHECK(launch_kth_threshold(mins, stride, stride, nq, k, eps, tau_all, tau, fold, stream_));
+        fold.counts = nullptr;
         stats_.gemm_launches += 1;
         stats_.kernel_launches += 2;
         a.direct = 0;
@@ -407,10 +411,7 @@ void FlatIndex::run_page(int nq, const void* xq_raw, const void* xq_op_in, int k
     };
     report_counts(two_stretches ? "after the first stretch" : "after the full pass");
     if (two_stretches) {
-        B200_CUDA_CHECK(launch_tighten_tau(cand, counts, plan.cap, nq, k, eps, tau, stream_));
-        if (dtype_ == kF32)
-            B200_CUDA_CHECK(launch_fold_tau(tau, static_cast<const float*>(qnorm), max_norm_, nq, d_, metric_,
-                                            const_cast<void*>(xq_op), stream_));
+        B200_CUDA_CHECK(launch_tighten_tau(cand, counts, plan.cap, nq, k, eps, tau, fold, stream_));
         a.tile_first = first_stretch;
         a.n_tiles_sel = n_tiles - first_stretch;
         a.prof = nullptr;
@@ -420,7 +421,7 @@ void FlatIndex::run_page(int nq, const void* xq_raw, const void* xq_op_in, int k
         B200_CUDA_CHECK(launch_dist_gemm(L, a, &map_a, &map_b_, stream_));
         a.trace = nullptr;
         stats_.gemm_launches += 1;
-        stats_.kernel_launches += 3;
+        stats_.kernel_launches += 2;
         report_counts("after the second stretch");
     }
     timer_.end(stream_);

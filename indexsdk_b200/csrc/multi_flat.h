@@ -23,7 +23,8 @@ class FlatGroup {
 public:
     explicit FlatGroup(int device) : device_(device) {}
     // Can these members (one device; same d / metric / dtype is the caller's contract) be searched
-    // as one group with nq queries?  Small indexes only: every key of a member is written once.
+    // as one group with nq queries?  Small indexes only: without thresholds every key of a member is
+    // written once.
     static bool eligible(const std::vector<FlatIndex*>& members, int64_t nq, int k);
     // xq: device pointer, float rows (kF32 / kF16 members) or int8 rows.  D / I: device pointers
     // [members][nq][k].  Work is queued on `stream`; returns after synchronising it.
@@ -34,6 +35,9 @@ public:
 
 private:
     void refresh(const std::vector<FlatIndex*>& members, cudaStream_t stream);
+    // All members' passes, with a threshold per (member, query) or with every key kept.
+    void run_passes(bool with_tau, int nq, const void* xq, const void* xq_op, const CUtensorMap& map_a, const void* qnorm,
+                    int k, float* D, int64_t* I, cudaStream_t stream);
 
     int device_;
     std::vector<const FlatIndex*> cur_;
@@ -46,7 +50,8 @@ private:
     bool use_simt_ = false;
     CUtensorMap map_b_;
     DeviceBuffer xop_, x32_, norms_, labels_, seg_index_, seg_col0_, seg_end_;
-    DeviceBuffer w_qop_, w_qnorm_, w_eps_, w_tau_, w_cand_, w_sel_, w_err_;
+    DeviceBuffer w_qop_, w_qnorm_, w_eps_, w_tau_, w_mins_, w_cand_, w_sel_, w_err_;
+    PinnedBuffer h_flags_;
     uint64_t launches_ = 0, rebuilds_ = 0;
 };
 

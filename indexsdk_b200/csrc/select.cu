@@ -13,6 +13,47 @@ namespace {
 constexpr int kSelThreads = 256;
 constexpr int kSmallSet = 512;   // candidate sets up to this size are sorted in shared memory
 
+// Three bf16 terms whose sum reproduces v to 24 significant bits (an infinite v stays in the
+// first term).
+__device__ __forceinline__ void split3_bf16(float v, __nv_bfloat16* out) {
+    const __nv_bfloat16 h = __float2bfloat16_rn(v);
+    float r = isfinite(v) ? v - __bfloat162float(h) : 0.f;
+    const __nv_bfloat16 m = __float2bfloat16_rn(r);
+    r -= __bfloat162float(m);
+    out[0] = h;
+    out[1] = m;
+    out[2] = __float2bfloat16_rn(r);
+}
+
+// Writes the threshold of candidate row q and what else becomes known with it, so that no launch of
+// its own is spent on either (a launch in the chain of a single query costs about 3.5 us):
+//   fold.counts : the row's candidate counter starts at zero
+//   fold.q_bf16 / fold.bias : the threshold in the form the folded GEMM tests, c = tau / 2 (L2) or tau
+//     (inner product), as three bf16 terms of the query operand or, for a segmented base, as one float
+//     per candidate row.  c is first raised by a margin for the fp32 accumulation inside the tensor core:
+//     d + 16 additions of terms whose partial sums stay below M = |q||y|max + |y|max^2 / 2 + |tau| perturb
+//     a key by less than 2^-14.8 M in either pass, and 2^-12 M covers the sample pass, the full pass and
+//     the threshold's own term together, so no key <= tau is missed.
+__device__ __forceinline__ void store_tau(int q, uint32_t ord, uint32_t* tau, const TauFold& fold) {
+    tau[q] = ord;
+    if (fold.counts) fold.counts[q] = 0u;
+    if (!fold.qnorm) return;
+    const float t = ord_to_float(ord);
+    const float qn = fold.qnorm[fold.q_mod > 0 ? q % fold.q_mod : q];
+    const float m = sqrtf(qn) * fold.ymax + 0.5f * fold.ymax * fold.ymax + fabsf(t);
+    float c = t + 0.000244140625f * m;
+    if (fold.metric == kMetricL2) c *= 0.5f;
+    if (fold.bias) {
+        fold.bias[q] = c;
+    } else {
+        const int dp = fold.d + kFoldCols;
+        // columns d + 3 .. d + 5 lie in one 8-column group (d is a multiple of 16), so they are
+        // consecutive in the packed layout as well
+        split3_bf16(c, static_cast<__nv_bfloat16*>(fold.q_bf16) +
+                           operand_elem(packed_operands(kKindBF16, dp), q, fold.d + 3, dp, kTileQ));
+    }
+}
+
 // Inclusive scan of a 256-bin histogram held in shared memory; returns through `bucket`/`below`
 // the bin that contains rank r (1-based) and the number of elements in lower bins.
 __device__ __forceinline__ void find_bucket(uint32_t* hist, uint32_t* scan, uint32_t r, uint32_t* bucket,
@@ -61,11 +102,11 @@ __device__ KeyT block_radix_kth(const KeyT* in, uint32_t n, uint32_t r, uint32_t
 
 __global__ void __launch_bounds__(kSelThreads)
 kth_threshold_kernel(const uint32_t* mins, int stride, int n, int k, const float* eps, uint32_t tau_all,
-                     uint32_t* tau) {
+                     uint32_t* tau, const TauFold fold) {
     __shared__ uint32_t hist[256], scan[256], sh_bucket, sh_below;
     const int q = blockIdx.x;
     if (n < k) {
-        if (threadIdx.x == 0) tau[q] = tau_all;
+        if (threadIdx.x == 0) store_tau(q, tau_all, tau, fold);
         return;
     }
     uint32_t kth = block_radix_kth<uint32_t>(mins + static_cast<int64_t>(q) * stride, n, k, hist, scan, &sh_bucket,
@@ -73,12 +114,11 @@ kth_threshold_kernel(const uint32_t* mins, int stride, int n, int k, const float
     if (threadIdx.x == 0) {
         if (eps) {
             float f = ord_to_float(kth);
-            f = f + 2.f * eps[q];
+            f = f + 2.f * eps[fold.q_mod > 0 ? q % fold.q_mod : q];
             f = f + fabsf(f) * 9.5367431640625e-07f;  // one part in 2^20 against the rounding of the adds
             kth = (f != f) ? tau_all : float_to_ord(f);
-            if (kth > tau_all) kth = tau_all;
         }
-        tau[q] = kth;
+        store_tau(q, kth > tau_all ? tau_all : kth, tau, fold);
     }
 }
 
@@ -97,7 +137,7 @@ constexpr int kPruneKeep = 2048;    // survivors staged for the in-place compact
 // approximate)).  Rows whose list overflowed or holds fewer than k candidates keep their threshold.
 __global__ void __launch_bounds__(kSelThreads)
 tighten_tau_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int k, const float* eps,
-                   uint32_t* tau) {
+                   uint32_t* tau, const TauFold fold) {
     __shared__ uint32_t hist[256], scan[256], sh_bucket, sh_below;
     __shared__ uint32_t keys[kPruneKeys];
     const int q = blockIdx.x;
@@ -116,7 +156,7 @@ tighten_tau_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t cap, i
             if (f != f) return;
             kth = float_to_ord(f);
         }
-        if (kth < tau[q]) tau[q] = kth;
+        if (kth < tau[q]) store_tau(q, kth, tau, fold);
     }
 }
 
@@ -176,12 +216,12 @@ prune_candidates_kernel(uint64_t* cand, uint32_t* counts, uint32_t cap, int k, c
 template <int NPL>
 __global__ void __launch_bounds__(128)
 kth_threshold_warp_kernel(const uint32_t* mins, int stride, int n, int nq, int k, const float* eps, uint32_t tau_all,
-                          uint32_t* tau) {
+                          uint32_t* tau, const TauFold fold) {
     const int lane = threadIdx.x & 31;
     const int q = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (q >= nq) return;
     if (n < k) {
-        if (lane == 0) tau[q] = tau_all;
+        if (lane == 0) store_tau(q, tau_all, tau, fold);
         return;
     }
     uint32_t v[NPL];
@@ -208,12 +248,11 @@ kth_threshold_warp_kernel(const uint32_t* mins, int stride, int n, int nq, int k
         uint32_t kth = prefix;
         if (eps) {
             float f = ord_to_float(kth);
-            f = f + 2.f * eps[q];
+            f = f + 2.f * eps[fold.q_mod > 0 ? q % fold.q_mod : q];
             f = f + fabsf(f) * 9.5367431640625e-07f;  // one part in 2^20 against the rounding of the adds
             kth = (f != f) ? tau_all : float_to_ord(f);
-            if (kth > tau_all) kth = tau_all;
         }
-        tau[q] = kth;
+        store_tau(q, kth > tau_all ? tau_all : kth, tau, fold);
     }
 }
 
@@ -237,13 +276,14 @@ __device__ __forceinline__ void bitonic_sort_u64(uint64_t* s, int P) {
 
 __global__ void __launch_bounds__(kSelThreads)
 select_topk_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int k, int P,
-                   uint64_t* out, uint8_t* overflow) {
+                   uint64_t* out, uint8_t* overflow, uint32_t* any_overflow) {
     extern __shared__ uint64_t sorted[];  // P entries
     __shared__ uint32_t hist[256], scan[256], sh_bucket, sh_below, sh_fill;
     const int q = blockIdx.x;
     const uint64_t* row = cand + static_cast<int64_t>(q) * cap;
     uint32_t n = counts ? counts[q] : n_fixed;
     if (overflow && threadIdx.x == 0) overflow[q] = n > cap ? 1 : 0;
+    if (any_overflow && threadIdx.x == 0 && n > cap) atomicOr(any_overflow, 1u);
     if (n > cap) n = cap;
     uint64_t* orow_fast = out + static_cast<int64_t>(q) * k;
     if (n <= static_cast<uint32_t>(kSmallSet)) {
@@ -555,18 +595,6 @@ __device__ __forceinline__ int warp_sum_i(int v) {
     return v;
 }
 
-// Three bf16 terms whose sum reproduces v to 24 significant bits (an infinite v stays in the
-// first term).
-__device__ __forceinline__ void split3_bf16(float v, __nv_bfloat16* out) {
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    float r = isfinite(v) ? v - __bfloat162float(h) : 0.f;
-    const __nv_bfloat16 m = __float2bfloat16_rn(r);
-    r -= __bfloat162float(m);
-    out[0] = h;
-    out[1] = m;
-    out[2] = __float2bfloat16_rn(r);
-}
-
 // Query operand rows of d + kFoldCols bf16: the query, three ones (they pick up the base row's
 // folded norm), three zeros (the threshold terms, written by fold_tau_kernel once the threshold is
 // known) and zero padding.
@@ -599,25 +627,6 @@ __global__ void prep_queries_f32_kernel(const float* xq, int nq, int d, int metr
         else e = c * qn * ymax + g * qn * ymax;
         eps[q] = e;
     }
-}
-
-// Writes the threshold terms of the folded query rows: c = tau / 2 (L2) or tau (inner product).
-// tau is first raised by a margin for the fp32 accumulation inside the tensor core: d + 16
-// additions of terms whose partial sums stay below M = |q||y|max + |y|max^2 / 2 + |tau| perturb a
-// key by less than 2^-14.8 M in either pass, and 2^-12 M covers the sample pass, the full pass and
-// the threshold's own term together, so no key <= tau is missed.
-__global__ void fold_tau_kernel(const uint32_t* tau, const float* qnorm, float ymax, int nq, int d, int metric,
-                                __nv_bfloat16* qb) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nq) return;
-    const float t = ord_to_float(tau[q]);
-    const float m = sqrtf(qnorm[q]) * ymax + 0.5f * ymax * ymax + fabsf(t);
-    float c = t + 0.000244140625f * m;
-    if (metric == kMetricL2) c *= 0.5f;
-    const int dp = d + kFoldCols;
-    // columns d + 3 .. d + 5 lie in one 8-column group (d is a multiple of 16), so they are
-    // consecutive in the packed layout as well
-    split3_bf16(c, qb + operand_elem(packed_operands(kKindBF16, dp), q, d + 3, dp, kTileQ));
 }
 
 __global__ void prep_queries_f16_kernel(const __half* xq, int nq, int d, float* qnorm) {
@@ -736,19 +745,19 @@ inline int next_pow2(int v) {
 }  // namespace
 
 cudaError_t launch_kth_threshold(const uint32_t* mins, int stride, int n, int nq, int k, const float* eps,
-                                 uint32_t tau_all, uint32_t* tau, cudaStream_t stream) {
+                                 uint32_t tau_all, uint32_t* tau, const TauFold& fold, cudaStream_t stream) {
     if (nq <= 0) return cudaSuccess;
     if (n <= 512)
-        kth_threshold_warp_kernel<16><<<(nq + 3) / 4, 128, 0, stream>>>(mins, stride, n, nq, k, eps, tau_all, tau);
+        kth_threshold_warp_kernel<16><<<(nq + 3) / 4, 128, 0, stream>>>(mins, stride, n, nq, k, eps, tau_all, tau, fold);
     else if (n <= 1024)
-        kth_threshold_warp_kernel<32><<<(nq + 3) / 4, 128, 0, stream>>>(mins, stride, n, nq, k, eps, tau_all, tau);
+        kth_threshold_warp_kernel<32><<<(nq + 3) / 4, 128, 0, stream>>>(mins, stride, n, nq, k, eps, tau_all, tau, fold);
     else
-        kth_threshold_kernel<<<nq, kSelThreads, 0, stream>>>(mins, stride, n, k, eps, tau_all, tau);
+        kth_threshold_kernel<<<nq, kSelThreads, 0, stream>>>(mins, stride, n, k, eps, tau_all, tau, fold);
     return cudaGetLastError();
 }
 
 cudaError_t launch_select_topk(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int nq,
-                               int k, uint64_t* out, uint8_t* overflow, cudaStream_t stream) {
+                               int k, uint64_t* out, uint8_t* overflow, cudaStream_t stream, uint32_t* any_overflow) {
     if (nq <= 0) return cudaSuccess;
     int P = next_pow2(k < 32 ? 32 : k);
     size_t smem = static_cast<size_t>(P) * sizeof(uint64_t);
@@ -757,14 +766,14 @@ cudaError_t launch_select_topk(const uint64_t* cand, const uint32_t* counts, uin
                                              static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
-    select_topk_kernel<<<nq, kSelThreads, smem, stream>>>(cand, counts, n_fixed, cap, k, P, out, overflow);
+    select_topk_kernel<<<nq, kSelThreads, smem, stream>>>(cand, counts, n_fixed, cap, k, P, out, overflow, any_overflow);
     return cudaGetLastError();
 }
 
 cudaError_t launch_tighten_tau(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int nq, int k,
-                               const float* eps, uint32_t* tau, cudaStream_t stream) {
+                               const float* eps, uint32_t* tau, const TauFold& fold, cudaStream_t stream) {
     if (nq <= 0) return cudaSuccess;
-    tighten_tau_kernel<<<nq, kSelThreads, 0, stream>>>(cand, counts, cap, k, eps, tau);
+    tighten_tau_kernel<<<nq, kSelThreads, 0, stream>>>(cand, counts, cap, k, eps, tau, fold);
     return cudaGetLastError();
 }
 
@@ -840,13 +849,6 @@ cudaError_t launch_base_prep_f32(const float* x, int64_t n, int d, int metric, v
     if (n <= 0) return cudaSuccess;
     base_prep_f32_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, stream>>>(
         x, n, d, metric, static_cast<__nv_bfloat16*>(x_bf16), row0, norms, max_norm_sq);
-    return cudaGetLastError();
-}
-cudaError_t launch_fold_tau(const uint32_t* tau, const float* qnorm, float base_max_norm, int nq, int d, int metric,
-                            void* q_bf16, cudaStream_t stream) {
-    if (nq <= 0) return cudaSuccess;
-    fold_tau_kernel<<<(nq + 255) / 256, 256, 0, stream>>>(tau, qnorm, base_max_norm, nq, d, metric,
-                                                          static_cast<__nv_bfloat16*>(q_bf16));
     return cudaGetLastError();
 }
 cudaError_t launch_base_prep_f16(const void* x, int64_t n, int d, float* norms, cudaStream_t stream) {

@@ -8,18 +8,31 @@
 
 namespace b200 {
 
+// What the kernels that fix a threshold write besides it (see store_tau in select.cu); all optional.
+struct TauFold {
+    uint32_t* counts = nullptr;     // set to zero per row
+    const float* qnorm = nullptr;   // fp32 indexes: squared query norms; the folded threshold is written as well
+    float ymax = 0.f;               // largest norm of a base row
+    int d = 0, metric = 0;
+    void* q_bf16 = nullptr;         // query operand that takes the threshold terms ...
+    float* bias = nullptr;          // ... or one float per candidate row (segmented base)
+    int q_mod = 0;                  // > 0: candidate row r belongs to query r % q_mod (eps and qnorm are per query)
+};
+
 // tau[q] = k-th smallest (1-based) of mins[q][0..n) as an ordered key; when eps != nullptr the
 // key is widened in the float domain by 2*eps[q] (filter-and-refine slack).  n < k gives the
 // "accept everything" threshold tau_all.
 cudaError_t launch_kth_threshold(const uint32_t* mins, int stride, int n, int nq, int k, const float* eps,
-                                 uint32_t tau_all, uint32_t* tau, cudaStream_t stream);
+                                 uint32_t tau_all, uint32_t* tau, const TauFold& fold, cudaStream_t stream);
 
 // Per query: the k smallest of cand[q][0..min(counts[q],cap)) in ascending order into
 // out[q][0..k), padded with kCandInvalid.  counts == nullptr means every row holds n_fixed
 // candidates.  overflow[q] is set to 1 when counts[q] > cap (the row's result is then not
-// trustworthy and the caller re-runs it without a threshold).
+// trustworthy and the caller re-runs it without a threshold); *any_overflow is set to 1 when that
+// happens to any row.
 cudaError_t launch_select_topk(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int nq,
-                               int k, uint64_t* out, uint8_t* overflow, cudaStream_t stream);
+                               int k, uint64_t* out, uint8_t* overflow, cudaStream_t stream,
+                               uint32_t* any_overflow = nullptr);
 
 // fp32 refinement: replaces the key of every candidate by the canonical fp32 distance
 // (sequential fmaf over the dimension) computed from the fp32 rows; L2 -> distance,
@@ -27,7 +40,7 @@ cudaError_t launch_select_topk(const uint64_t* cand, const uint32_t* counts, uin
 // thresholded path, between two stretches of the full pass: tau[row] = min(tau[row], k-th smallest
 // key among the row's candidates so far (+ 2 eps[row] where eps is given: approximate keys))
 cudaError_t launch_tighten_tau(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int nq, int k,
-                               const float* eps, uint32_t* tau, cudaStream_t stream);
+                               const float* eps, uint32_t* tau, const TauFold& fold, cudaStream_t stream);
 // fp32 index, thresholded path: removes candidates whose approximate key exceeds the k-th smallest
 // approximate key of the row by more than 2 eps[row] (they cannot be in the exact top-k); the row
 // is compacted and counts[row] updated
@@ -74,9 +87,6 @@ cudaError_t launch_prep_queries_i8(const int8_t* xq, int nq, int d, int32_t* qno
 // in it; norms points at the norms of the rows being added.
 cudaError_t launch_base_prep_f32(const float* x, int64_t n, int d, int metric, void* x_bf16, int64_t row0,
                                  float* norms, float* max_norm_sq, cudaStream_t stream);
-// threshold terms of the folded query rows, from the ordered-key thresholds tau[nq]
-cudaError_t launch_fold_tau(const uint32_t* tau, const float* qnorm, float base_max_norm, int nq, int d, int metric,
-                            void* q_bf16, cudaStream_t stream);
 cudaError_t launch_base_prep_f16(const void* x_f16, int64_t n, int d, float* norms, cudaStream_t stream);
 cudaError_t launch_base_prep_i8(const int8_t* x, int64_t n, int d, int32_t* norms, cudaStream_t stream);
 cudaError_t launch_f32_to_f16(const float* x, int64_t count, void* out, cudaStream_t stream);
