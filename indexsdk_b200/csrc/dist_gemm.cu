@@ -723,8 +723,9 @@ dist_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
                     ptx::mbar_expect_tx(full, stage_bytes);
                     uint8_t* st = ring + static_cast<size_t>(r * nst + s) * stage_bytes;
                     if (packed) {
-                        ptx::bulk_load_1d(st, static_cast<const uint8_t*>(a.B) + static_cast<size_t>(tile) * stage_bytes,
-                                          stage_bytes, full);
+                        const void* src = a.seg_tile ? a.seg_tile[tile]
+                                                     : static_cast<const uint8_t*>(a.B) + static_cast<size_t>(tile) * stage_bytes;
+                        ptx::bulk_load_1d(st, src, stage_bytes, full);
                         if (++rs == nst) { rs = 0; rph ^= 1u; }
                         continue;
                     }

@@ -97,6 +97,7 @@ struct GemmArgs {
     const int64_t* seg_col0;
     const int64_t* seg_end;
     const float* seg_bias;
+    const void* const* seg_tile;   // packed operands: address of every tile's image, read where the index keeps it
     int* err;             // device error word
     // optional phase profile (nullptr = off): 8 counters of SM cycles summed over CTAs
     //   0 producer wait-empty   1 mma wait-acc-empty   2 mma wait-full   3 epilogue wait-acc-full

@@ -5,8 +5,8 @@
 // (block -> index, label offset) tables (FR/ascendhost/src/index/IndexFlatL2Aicpu.cpp:307-444 driver,
 // FR/ops/cpukernel/impl/topk_multisearch_cpu_kernel.cpp:316-430 segmented heap select,
 // FR/ascenddaemon/impl/IndexFlat.cpp:813-847 tables); its API admits 10 000 indexes
-// (FR/ascend/AscendMultiIndexSearch.cpp:38-41).  Here the bases of the member indexes are kept
-// concatenated (every member starts on a tile boundary) beside a tile -> index table, and one
+// (FR/ascend/AscendMultiIndexSearch.cpp:38-41).  Here the members' rows get positions in one common
+// space (every member starts on a tile boundary), with a tile -> index table, and one
 // distance GEMM walks all tiles with every query block: the epilogue sends the keys of a tile to
 // the candidate rows of the tile's index.  Refinement, selection and emission then run over
 // [index][query] rows, so the number of kernel launches does not depend on the number of indexes.
@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "flat_index.h"
+#include "select.cuh"
 
 namespace b200 {
 
@@ -31,7 +32,7 @@ public:
     void search_device(const std::vector<FlatIndex*>& members, int64_t nq, const void* xq, int k, float* D, int64_t* I,
                        cudaStream_t stream);
     uint64_t launches() const { return launches_; }   // kernels launched by searches so far
-    uint64_t rebuilds() const { return rebuilds_; }   // times the concatenation was (re)built
+    uint64_t rebuilds() const { return rebuilds_; }   // times the members' tables were (re)built
 
 private:
     void refresh(const std::vector<FlatIndex*>& members, cudaStream_t stream);
@@ -40,16 +41,24 @@ private:
                     int k, float* D, int64_t* I, cudaStream_t stream);
 
     int device_;
-    std::vector<const FlatIndex*> cur_;
+    std::vector<const FlatIndex*> cur_;   // the members the tables below describe, with their contents' generations
     std::vector<uint64_t> cur_gen_;
-    std::vector<int64_t> seg_start_;      // first position of every member in the concatenation (+ total at the end)
-    int64_t total_rows_ = 0;              // padded rows of the concatenation
+    std::vector<int64_t> seg_start_;      // first position of every member (+ total at the end)
+    int64_t total_rows_ = 0;              // padded rows of all members
+    bool in_place_ = false;               // packed operands are read where the members keep them
     uint32_t cap_ = 0;                    // largest padded member
     float max_norm_ = 0.f;
     int d_ = 0, metric_ = 0, dtype_ = 0, op_cols_ = 0, kind_ = 0, num_sms_ = 0;
     bool use_simt_ = false;
     CUtensorMap map_b_;
-    DeviceBuffer xop_, x32_, norms_, labels_, seg_index_, seg_col0_, seg_end_;
+    DeviceBuffer xop_, norms_;            // gathered operand rows (row-major operands: one tensor map covers them)
+    DeviceBuffer tables_;                 // device copy of h_tables_, in which the pointers below lie
+    PinnedBuffer h_tables_;
+    const MemberView* members_ = nullptr;
+    const void* const* seg_tile_ = nullptr;
+    const int64_t* seg_col0_ = nullptr;
+    const int64_t* seg_end_ = nullptr;
+    const int32_t* seg_index_ = nullptr;
     DeviceBuffer w_qop_, w_qnorm_, w_eps_, w_tau_, w_mins_, w_cand_, w_sel_, w_err_;
     PinnedBuffer h_flags_;
     uint64_t launches_ = 0, rebuilds_ = 0;

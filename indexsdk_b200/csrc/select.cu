@@ -341,7 +341,7 @@ constexpr int kRefPitch = kRefChunk + 4;
 constexpr uint32_t kRefWindow = 512;   // candidate slots compacted at a time
 __global__ void __launch_bounds__(128)
 refine_f32_kernel(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int d, int metric,
-                  const float* xq, const float* xb, int q_first, int q_mod) {
+                  const float* xq, const float* xb, int q_first, int q_mod, const MemberView* members) {
     extern __shared__ __align__(16) float ref_sm[];
     float* qs = ref_sm;                                              // [d]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -353,6 +353,12 @@ refine_f32_kernel(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint
     uint32_t n = counts ? counts[q] : n_fixed;
     if (n > cap) n = cap;
     if (blockIdx.x * kRefWindow >= n) return;
+    uint32_t pos_first = 0;   // position of xb's first row
+    if (members) {
+        const MemberView& mv = members[(q_first + q) / q_mod];
+        xb = mv.rows_f32;
+        pos_first = static_cast<uint32_t>(mv.first);
+    }
     for (int i = threadIdx.x; i < d / 4; i += 128)
         reinterpret_cast<float4*>(qs)[i] = __ldg(reinterpret_cast<const float4*>(xq + static_cast<int64_t>(qrow) * d) + i);
     __syncthreads();
@@ -372,7 +378,7 @@ refine_f32_kernel(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint
         if (c != kCandInvalid) {
             const uint32_t j = atomicAdd(&s_cnt, 1u);
             s_slot[j] = i;
-            s_pos[j] = static_cast<uint32_t>(c);
+            s_pos[j] = static_cast<uint32_t>(c) - pos_first;
         }
     }
     __syncthreads();
@@ -488,7 +494,7 @@ refine_f32_kernel(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint
             __syncwarp();
         }
         if (metric != kMetricL2) acc = -acc;
-        if (live) row[i] = pack_cand(float_to_ord(acc), pos);
+        if (live) row[i] = pack_cand(float_to_ord(acc), pos + pos_first);
     }
     __syncthreads();   // the window's lists are reused
     }
@@ -508,7 +514,12 @@ __global__ void emit_kernel(const EmitArgs e) {
         label = -1;
     } else {
         const uint32_t ok = static_cast<uint32_t>(c >> 32), pos = static_cast<uint32_t>(c);
-        label = e.labels ? e.labels[pos] : static_cast<int64_t>(pos);
+        if (e.members) {
+            const MemberView& mv = e.members[q / e.q_mod];
+            label = mv.labels[static_cast<int64_t>(pos) - mv.first];
+        } else {
+            label = e.labels ? e.labels[pos] : static_cast<int64_t>(pos);
+        }
         if (e.mode == 2) {
             int32_t kv = ord_to_int(ok);
             if (e.metric == kMetricL2) dist = static_cast<float>(kv + static_cast<const int32_t*>(e.qnorm)[qn]);
@@ -785,7 +796,8 @@ cudaError_t launch_prune_candidates(uint64_t* cand, uint32_t* counts, uint32_t c
 }
 
 cudaError_t launch_refine_f32(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int nq, int d,
-                              int metric, const float* xq, const float* xb, cudaStream_t stream, int q_mod) {
+                              int metric, const float* xq, const float* xb, cudaStream_t stream, int q_mod,
+                              const MemberView* members) {
     if (nq <= 0) return cudaSuccess;
     uint32_t per_row = counts ? cap : (n_fixed < cap ? n_fixed : cap);
     // Blocks stride over a row's candidates, so a few thousand blocks in total keep the machine
@@ -805,7 +817,7 @@ cudaError_t launch_refine_f32(uint64_t* cand, const uint32_t* counts, uint32_t n
         const int nqq = nq - q0 < 65535 ? nq - q0 : 65535;
         refine_f32_kernel<<<dim3(gx, nqq), 128, smem, stream>>>(cand + static_cast<int64_t>(q0) * cap,
                                                             counts ? counts + q0 : nullptr, n_fixed, cap, d, metric,
-                                                            xq, xb, q0, q_mod);
+                                                            xq, xb, q0, q_mod, members);
     }
     return cudaGetLastError();
 }

@@ -8,6 +8,16 @@
 
 namespace b200 {
 
+// One member of a multi-index search over a common position space: where its rows lie and the position
+// of its first row.
+struct MemberView {
+    const float* rows_f32;     // fp32 members
+    const int64_t* labels;
+    const void* operand;       // tensor-core operand rows (or packed tiles)
+    const void* norms;
+    int64_t first, n;
+};
+
 // What the kernels that fix a threshold write besides it (see store_tau in select.cu); all optional.
 struct TauFold {
     uint32_t* counts = nullptr;     // set to zero per row
@@ -47,8 +57,10 @@ cudaError_t launch_tighten_tau(const uint64_t* cand, const uint32_t* counts, uin
 cudaError_t launch_prune_candidates(uint64_t* cand, uint32_t* counts, uint32_t cap, int nq, int k,
                                     const float* eps, cudaStream_t stream);
 // q_mod > 0: candidate row r belongs to query r % q_mod (rows = [index][query] of a multi-index search)
+// and, where members (a device array) is given instead of xb, to member r / q_mod
 cudaError_t launch_refine_f32(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int nq, int d,
-                              int metric, const float* xq, const float* xb, cudaStream_t stream, int q_mod = 0);
+                              int metric, const float* xq, const float* xb, cudaStream_t stream, int q_mod = 0,
+                              const MemberView* members = nullptr);
 
 struct EmitArgs {
     const uint64_t* sel;     // [nq][k] sorted candidates
@@ -62,6 +74,7 @@ struct EmitArgs {
     int ldk;
     const int32_t* qmap;     // optional: output row = qmap[q] (fallback re-runs scatter into place)
     int q_mod;               // > 0: row q uses the query norm of row q % q_mod (multi-index search)
+    const MemberView* members;   // with q_mod: row q's labels are those of member q / q_mod (device array, or nullptr)
 };
 cudaError_t launch_emit(const EmitArgs& e, cudaStream_t stream);
 
