@@ -43,6 +43,7 @@
 #include <cub/cub.cuh>
 #include <unordered_set>
 
+#include "ivfpq_short_scan.cuh"
 #include "ivfpq_tc_scan.cuh"
 #include "kmeans.h"
 #include "ptx_sm100.cuh"
@@ -2095,6 +2096,56 @@ void IvfpqIndex::search_preassigned_device(int64_t nq, const float* xq, int k, c
 
 // pre_cD / pre_cI: [nq][nprobe] probe distances and list ids computed elsewhere (nullptr: run the
 // coarse stage here).
+// Short codes (ivfpq_short_scan.cu): the queries of a page in groups whose candidate rows fit 1 GB.
+// Returns the queries that need the exact scan (more candidates than a row holds).
+std::vector<int32_t> IvfpqIndex::search_short(const ShortScanArgs& a, int64_t m, cudaStream_t st) {
+    int64_t longest = 0;
+    for (int64_t l : lens_host_) longest = std::max(longest, l);
+    ShortScanArgs s = a;
+    s.cap = static_cast<uint32_t>(std::min<int64_t>(kShortMaxCap, std::max<int64_t>(32, longest * a.nprobe)));
+    const int64_t visited = longest * a.nprobe;
+    s.n1_max = static_cast<uint32_t>(std::min<int64_t>(
+        kShortMaxBound, std::max<int64_t>(1, std::min(visited, std::max<int64_t>({visited / 16, 4LL * a.k, 2048})))));
+    const int64_t group = std::min<int64_t>(4096, std::max<int64_t>(1, (int64_t(1) << 30) / (static_cast<int64_t>(s.cap) * 8)));
+    const int64_t g = std::min(group, m);
+    s.cand = static_cast<uint2*>(w_cpos_.ensure(static_cast<size_t>(g) * s.cap * 8));
+    s.lut = static_cast<float*>(w_fd_.ensure(static_cast<size_t>(g) * a.M * kKsub * 4));
+    s.label_max = static_cast<uint64_t*>(w_fth_.ensure(static_cast<size_t>(g) * 12));
+    s.thr = reinterpret_cast<float*>(s.label_max + g);
+    s.count = static_cast<uint32_t*>(w_ccount_.ensure(static_cast<size_t>(g) * 4));
+    uint8_t* flag = static_cast<uint8_t*>(w_flag_.ensure(static_cast<size_t>(m)));
+    for (int64_t g0 = 0; g0 < m; g0 += group) {
+        s.nq = std::min(group, m - g0);
+        s.cI = a.cI + g0 * a.nprobe;
+        s.cD = a.cD + g0 * a.nprobe;
+        s.xq = a.xq + g0 * a.d;
+        s.outD = a.outD + g0 * a.k;
+        s.outI = a.outI + g0 * a.k;
+        s.flag = flag + g0;
+        B200_CUDA_CHECK(launch_short_scan(s, num_sms_, st));
+        stats_.kernel_launches += 3;
+    }
+    uint8_t* hf = static_cast<uint8_t*>(h_flag_.ensure(static_cast<size_t>(m)));
+    B200_CUDA_CHECK(cudaMemcpyAsync(hf, flag, static_cast<size_t>(m), cudaMemcpyDeviceToHost, st));
+    B200_CUDA_CHECK(cudaStreamSynchronize(st));
+    std::vector<int32_t> bad;
+    for (int64_t i = 0; i < m; ++i)
+        if (hf[i]) bad.push_back(static_cast<int32_t>(i));
+    return bad;
+}
+
+// Error bound of the filter arithmetic relative to the canonical value:
+//   raw      : re-ordering a sum of M non-negative fp32 terms -> (2M + 8) ulp of the sum
+//   residual : every rounding acts on a partial sum bounded by
+//              B = |coarse| + |t2|max + 2 |q| cbnorm + |result|, about 2M + 2 dsub + 16 of them
+float IvfpqIndex::filter_err_rel() const {
+    const float ulp = 5.9604645e-08f;
+    return by_residual_ ? (2.f * M_ + 2.f * dsub_ + 16.f) * ulp : (2.f * M_ + 8.f) * ulp;
+}
+float IvfpqIndex::t2_bound() const {
+    return cb_norm_bound_ * cb_norm_bound_ + 2.f * coarse_->raw_view().max_norm * cb_norm_bound_;
+}
+
 void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int64_t* I, const float* pre_cD,
                                const int64_t* pre_cI) {
     if (nq <= 0) return;
@@ -2109,6 +2160,8 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
     int kpt = 1;
     while (kpt * 32 < k + 16) kpt <<= 1;
     const bool fast = rotated_ && !force_exact_ && kpt <= 32;
+    const bool short_codes = !rotated_ && !force_exact_ &&
+                             use_short_scan(M_, by_residual_, static_cast<double>(nprobe) * n_ / nlist_, nprobe, k);
     const int kprime = 32 * kpt;
     const int64_t page = 16384;
     unsigned long long scanned = stats_.scan_codes;
@@ -2158,6 +2211,45 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
         a.scanned = w_tmp_.as<unsigned long long>();
         a.qlist = nullptr;
 
+        if (short_codes) {
+            timer_.begin(kStageScan, st);
+            ShortScanArgs s{};
+            s.cI = a.cI;
+            s.cD = a.cD;
+            s.nprobe = nprobe;
+            s.nlist = nlist_;
+            s.k = k;
+            s.M = M_;
+            s.d = d_;
+            s.dsub = dsub_;
+            s.offsets = a.offsets;
+            s.lens = a.lens;
+            s.codes = a.codes;
+            s.ids = a.ids;
+            s.t2 = a.t2;
+            s.by_residual = a.by_residual;
+            s.xq = xp;
+            s.centroids = a.centroids;
+            s.codebooks = a.codebooks;
+            s.err_rel = filter_err_rel();
+            s.t2_bound = t2_bound();
+            s.cb_bound = cb_norm_bound_;
+            s.outD = a.outD;
+            s.outI = a.outI;
+            s.scanned = a.scanned;
+            std::vector<int32_t> bad = search_short(s, m, st);
+            if (!bad.empty()) {
+                stats_.fallback_queries += bad.size();
+                int32_t* ql = static_cast<int32_t*>(w_qlist_.ensure(bad.size() * 4));
+                B200_CUDA_CHECK(cudaMemcpyAsync(ql, bad.data(), bad.size() * 4, cudaMemcpyHostToDevice, st));
+                a.qlist = ql;
+                B200_CUDA_CHECK(launch_exact(a, static_cast<int>(bad.size()), st));
+                stats_.kernel_launches += 1;
+            }
+            timer_.end(st);
+            idle = false;
+            continue;
+        }
         if (!fast) {
             timer_.begin(kStageScan, st);
             B200_CUDA_CHECK(launch_exact(a, static_cast<int>(m), st));
@@ -2181,15 +2273,9 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
         a.fp = static_cast<uint32_t*>(w_fp_.ensure(static_cast<size_t>(m) * S * kprime * 4));
         a.fth = static_cast<float*>(w_fth_.ensure(static_cast<size_t>(m) * S * 4));
         a.flag = static_cast<uint8_t*>(w_flag_.ensure(static_cast<size_t>(m)));
-        // error bound of the filter arithmetic relative to the canonical value:
-        //   raw      : re-ordering a sum of M non-negative fp32 terms -> (2M + 8) ulp of the sum
-        //   residual : every rounding acts on a partial sum bounded by
-        //              B = |coarse| + |t2|max + 2 |q| cbnorm + |result|, about 2M + 2 dsub + 16 of them
-        const float ulp = 5.9604645e-08f;
-        a.err_rel = by_residual_ ? (2.f * M_ + 2.f * dsub_ + 16.f) * ulp : (2.f * M_ + 8.f) * ulp;
+        a.err_rel = filter_err_rel();
         a.cb_bound = cb_norm_bound_;
-        const float cmax = coarse_->raw_view().max_norm;
-        a.t2_bound = cb_norm_bound_ * cb_norm_bound_ + 2.f * cmax * cb_norm_bound_;
+        a.t2_bound = t2_bound();
         // very large batches of residual codes: every probed list is decoded once and multiplied with
         // all of its queries on the tensor cores (ivfpq_tc_scan.cu)
         const bool tc = persist && tc_scan_ && tc_cb_ok_ && by_residual_ && d_ == kTcDim && M_ == kTcM && kpt == 1 &&

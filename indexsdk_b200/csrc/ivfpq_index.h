@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "flat_index.h"
+#include "ivfpq_short_scan.cuh"
 
 namespace b200 {
 
@@ -77,6 +78,9 @@ private:
     int nprobe_ = 1;
     int64_t n_ = 0;                       // vectors stored
     int64_t n_pad_ = 0;                   // storage slots in use: every list padded to a multiple of 32
+    std::vector<int32_t> search_short(const ShortScanArgs& a, int64_t m, cudaStream_t st);
+    float filter_err_rel() const;
+    float t2_bound() const;
     void search_stages(int64_t nq, const float* xq, int k, float* D, int64_t* I, const float* pre_cD,
                        const int64_t* pre_cI);
     bool has_centroids_ = false, has_codebooks_ = false;

@@ -1,0 +1,79 @@
+"""IVFPQ search of short codes (M = 4 and 8): bound, collection and exact order against the oracle.
+Where it can go wrong: k against what the nearest lists hold, lists shorter than a block's unit or
+empty, ties that outgrow the sort (2 048 pairs) and the candidate row (32 768), duplicate-free
+ordering by label, several shares per query."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import assert_exact
+from indexsdk_b200 import datasets
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(b200, xb, ids, cent, cb, resid, xq, nprobe, k):
+    nlist, M = cent.shape[0], cb.shape[0]
+    ix = b200.IndexIVFPQ(xb.shape[1], nlist, M, 8, by_residual=resid)
+    ix.set_centroids(cent)
+    ix.set_codebooks(cb)
+    ix.add_with_ids(xb, ids)
+    ix.nprobe = nprobe
+    D, I = ix.search(xq, k)
+    ln = oracle.ivf_assign(cent, xb)
+    off, cs, idl = oracle.build_lists(ln, oracle.pq_encode(cb, xb, resid, cent, ln), ids, nlist)
+    Dr, Ir = oracle.ivfpq_search(cent, cb, resid, off, cs, idl, xq, nprobe, k)
+    assert_exact(D, I, Dr, Ir)
+    return ix
+
+
+@pytest.mark.parametrize("resid", [False, True])
+@pytest.mark.parametrize("M,d,nlist,n,nq,nprobe,k", [
+    (4, 64, 16, 3000, 1, 16, 1),           # one query, many shares of it
+    (4, 128, 8, 40000, 3, 8, 300),
+    (8, 64, 512, 5000, 70, 40, 100),       # lists of about ten vectors, some empty
+    (8, 128, 8, 33000, 5, 5, 1024),
+    (4, 64, 4, 900, 2, 2, 1024),           # fewer vectors than k
+    (8, 96, 1300, 2600, 9, 1024, 10),      # the largest number of staged probes
+])
+def test_short_codes_vs_oracle(b200, resid, M, d, nlist, n, nq, nprobe, k):
+    xb, _ = datasets.mixture(n, d, max(nlist // 3, 4), seed=4)
+    xq, _ = datasets.mixture(nq, d, max(nlist // 3, 4), seed=5, centers_seed=4)
+    rng = np.random.default_rng(1)
+    ids = rng.permutation(n).astype(np.int64) * 3 - 1000     # unordered, some negative
+    cent, cb = datasets.train_ivfpq(xb[:8000], min(nlist, 512), M, resid, niter=3)
+    if nlist > 512:                                          # more lists than were trained: shifted copies
+        cent = np.concatenate([cent + np.float32(0.01 * i) for i in range(3)])[:nlist]
+    _check(b200, xb, ids, cent, cb, resid, xq, nprobe, k)
+
+
+@pytest.mark.parametrize("resid", [False, True])
+@pytest.mark.parametrize("copies", [3000, 40000])
+def test_ties_beyond_the_sort_and_beyond_the_row(b200, resid, copies):
+    """`copies` equal vectors in one list: the labels decide.  40 000 do not fit a candidate row, which
+    residual encoding answers with the exact scan and raw encoding with a bound on the labels."""
+    d, M, nlist, k = 64, 4, 4, 50
+    xb, _ = datasets.mixture(2000, d, 4, seed=4)
+    cent, cb = datasets.train_ivfpq(xb, nlist, M, resid, niter=3)
+    xb = np.concatenate([xb, np.repeat(xb[:1], copies, axis=0)])
+    ids = np.random.default_rng(2).permutation(len(xb)).astype(np.int64) - 500
+    ix = _check(b200, xb, ids, cent, cb, resid, xb[:3], 4, k)
+    assert (ix.stats()["fallback_queries"] > 0) == (copies == 40000 and resid)
+
+
+def test_queries_that_hold_nan_or_infinity_find_what_the_exact_scan_finds(b200, monkeypatch):
+    d, M, nlist = 64, 8, 8
+    xb, _ = datasets.mixture(4000, d, 8, seed=4)
+    cent, cb = datasets.train_ivfpq(xb, nlist, M, False, niter=3)
+    xq = xb[:4].copy()
+    xq[1, 3], xq[2, 5], xq[3] = np.nan, np.inf, 1e30
+    out = []
+    for exact in ("0", "1"):
+        monkeypatch.setenv("B200IDX_IVFPQ_EXACT", exact)
+        ix = b200.IndexIVFPQ(d, nlist, M, 8, by_residual=False)
+        ix.set_centroids(cent)
+        ix.set_codebooks(cb)
+        ix.add(xb)
+        ix.nprobe = 4
+        out.append(ix.search(xq, 20))
+    assert_exact(out[0][0], out[0][1], out[1][0], out[1][1])
