@@ -188,11 +188,11 @@ struct RowEpilogue {
             rq2 = cos16_query_term(__ldg(a.qnorm_i32 + qn));
         }
         if (MODE == kModeAppend && ok && new_row) {
-            // once per run of tiles of the same row: the threshold, and (threshold mode) the first
-            // candidate block -- reserved now, while the accumulator is still being computed, so
-            // that the first candidate of the run does not wait for the atomic
+            // once per run of tiles of the same row: the threshold, and (threshold mode, runs long
+            // enough to use it) the first candidate block -- reserved now, while the accumulator is
+            // still being computed, so that the first candidate of the run does not wait for the atomic
             const uint32_t to = __ldg(a.tau + q);
-            if (!a.direct && blk_q != q) {
+            if (a.eager && !a.direct && blk_q != q) {
                 blk_next = atomicAdd(a.counts + q, kCandBlock);
                 blk_left = kCandBlock;
                 blk_q = q;
@@ -1177,6 +1177,9 @@ cudaError_t launch_one(const GemmLaunch& L, GemmArgs a, const CUtensorMap* mapA,
         const double ideal = static_cast<double>(total) / grid;
         if (worst <= 1.06 * ideal + 1.0) a.aligned_ranges = 1;
     }
+    // In a short run most threads never see a candidate, and the blocks they reserved would be what the
+    // selection reads: 9 472 slots for the 150 candidates of one query against 100 003 rows.
+    a.eager = total >= 16LL * grid ? 1 : 0;
     kern<<<grid, gemm_threads(KIND), smem, stream>>>(*mapA, *mapB, a);
     return cudaGetLastError();
 }

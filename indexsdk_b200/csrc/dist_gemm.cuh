@@ -76,6 +76,8 @@ struct GemmArgs {
     uint64_t* cand;       // [nq][cap] packed (ordered key, position); reserved but unused slots hold "invalid"
     uint32_t* counts;     // [nq] slots reserved (blocks of 8 per thread and query block run): >= candidates
     uint32_t cap;
+    int eager;            // threshold mode: a thread reserves its first candidate block before it has a candidate
+                          // (filled in by launch_dist_gemm)
     int direct;           // 1: slot = position (cap >= N, no atomics); 0: slot = atomic counter
     // optional per-(query, base row) filter: bit (row % 32) of qmask[q * qmask_stride + row / 32] = 1
     // lets the row take part (nullptr: every row does)

@@ -275,7 +275,7 @@ FlatIndex::Plan FlatIndex::make_plan(int k, int64_t nq) const {
     return p;
 }
 
-void FlatIndex::run_page(int nq, const void* xq_raw, const void* xq_op_in, int k, float* D, int64_t* I, int ldk,
+FlatIndex::PageTail FlatIndex::run_page(int nq, const void* xq_raw, const void* xq_op_in, int k, float* D, int64_t* I, int ldk,
                          const int32_t* qmap_dev, bool force_full) {
     const int kind = gemm_kind();
     const bool is_int = dtype_ == kI8;
@@ -426,43 +426,57 @@ void FlatIndex::run_page(int nq, const void* xq_raw, const void* xq_op_in, int k
     }
     timer_.end(stream_);
 
-    const uint32_t* counts_arg = plan.sampled ? counts : nullptr;
+    PageTail t{};
+    t.nq = nq;
+    t.k = k;
+    t.sampled = plan.sampled;
+    t.prune = plan.sampled && static_cast<int64_t>(plan.s_tiles) * 2 <= n_tiles;
+    t.cap = plan.cap;
+    t.xq = static_cast<const float*>(xq_raw);
+    t.e.nq = nq;
+    t.e.k = k;
+    t.e.metric = metric_;
+    t.e.mode = is_int ? 2 : (dtype_ == kF32 ? 1 : 0);
+    t.e.qnorm = qnorm;
+    t.e.labels = labels_.as<int64_t>();
+    t.e.D = D;
+    t.e.I = I;
+    t.e.ldk = ldk;
+    t.e.qmap = qmap_dev;
+    return t;
+}
+
+// From the candidates to the results.  fused: fp32 lists that are short enough in one launch; the others
+// come back with status 2 in w_over_ and need a second call without it.
+void FlatIndex::run_tail(const PageTail& t, bool fused) {
+    uint64_t* cand = w_cand_.as<uint64_t>();
+    uint32_t* counts = t.sampled ? w_counts_.as<uint32_t>() : nullptr;
+    const float* eps = w_eps_.as<float>();
+    uint8_t* over = static_cast<uint8_t*>(w_over_.ensure(static_cast<size_t>(t.nq)));
     const uint32_t n_fixed = static_cast<uint32_t>(n_);
-    // 5. fp32 refinement of the candidates
+    if (fused) {
+        timer_.begin(kStageRefine, stream_);
+        B200_CUDA_CHECK(launch_finish_f32(cand, counts, t.cap, d_, eps, t.xq, x32_.as<float>(), over, nullptr, t.e, stream_));
+        timer_.end(stream_);
+        stats_.kernel_launches += 1;
+        return;
+    }
     if (dtype_ == kF32) {
         timer_.begin(kStageRefine, stream_);
         // worth a pass only when the threshold came from a subset of the tiles (about 1 / fraction
         // times more candidates than k)
-        if (plan.sampled && static_cast<int64_t>(plan.s_tiles) * 2 <= (n_ + kTileB - 1) / kTileB) {
-            B200_CUDA_CHECK(launch_prune_candidates(cand, counts, plan.cap, nq, k, eps, stream_));
+        if (t.prune) {
+            B200_CUDA_CHECK(launch_prune_candidates(cand, counts, t.cap, t.nq, t.k, eps, stream_));
             stats_.kernel_launches += 1;
         }
-        B200_CUDA_CHECK(launch_refine_f32(cand, counts_arg, n_fixed, plan.cap, nq, d_, metric_,
-                                          static_cast<const float*>(xq_raw), x32_.as<float>(), stream_));
+        B200_CUDA_CHECK(launch_refine_f32(cand, counts, n_fixed, t.cap, t.nq, d_, metric_, t.xq, x32_.as<float>(), stream_));
         stats_.kernel_launches += 1;
         timer_.end(stream_);
     }
     timer_.begin(kStageSelect, stream_);
-    // 6. exact top-k of the candidates, 7. results
-    uint64_t* sel = static_cast<uint64_t*>(w_sel_.ensure(static_cast<size_t>(nq) * k * 8));
-    uint8_t* over = static_cast<uint8_t*>(w_over_.ensure(static_cast<size_t>(nq)));
-    B200_CUDA_CHECK(launch_select_topk(cand, counts_arg, n_fixed, plan.cap, nq, k, sel,
-                                       plan.sampled ? over : nullptr, stream_));
-    if (!plan.sampled) B200_CUDA_CHECK(cudaMemsetAsync(over, 0, static_cast<size_t>(nq), stream_));
-    EmitArgs e{};
-    e.sel = sel;
-    e.nq = nq;
-    e.k = k;
-    e.metric = metric_;
-    e.mode = is_int ? 2 : (dtype_ == kF32 ? 1 : 0);
-    e.qnorm = qnorm;
-    e.labels = labels_.as<int64_t>();
-    e.D = D;
-    e.I = I;
-    e.ldk = ldk;
-    e.qmap = qmap_dev;
-    B200_CUDA_CHECK(launch_emit(e, stream_));
-    stats_.kernel_launches += 2;
+    if (!t.sampled) B200_CUDA_CHECK(cudaMemsetAsync(over, 0, static_cast<size_t>(t.nq), stream_));
+    B200_CUDA_CHECK(launch_select_emit(cand, counts, n_fixed, t.cap, t.sampled ? over : nullptr, nullptr, t.e, stream_));
+    stats_.kernel_launches += 1;
     timer_.end(stream_);
 }
 
@@ -501,11 +515,20 @@ void FlatIndex::search_device(int64_t nq, const void* xq, bool q_is_f16, int k, 
         const int nqp = static_cast<int>(std::min<int64_t>(page, nq - q0));
         const uint8_t* xp = static_cast<const uint8_t*>(xq_in) + q0 * in_row;
         mask_cur_ = mask_dev_ ? mask_dev_ + q0 * mask_stride_ : nullptr;
-        run_page(nqp, xp, xp, k, D + q0 * ldk, I + q0 * ldk, ldk, nullptr, false);
+        const PageTail tail = run_page(nqp, xp, xp, k, D + q0 * ldk, I + q0 * ldk, ldk, nullptr, false);
+        const bool fused = dtype_ == kF32 && tail.sampled && k <= kFinishMaxK;
+        run_tail(tail, fused);
         uint8_t* h = static_cast<uint8_t*>(h_over_.ensure(static_cast<size_t>(nqp) + sizeof(int)));
-        B200_CUDA_CHECK(cudaMemcpyAsync(h, w_over_.get(), static_cast<size_t>(nqp), cudaMemcpyDeviceToHost, stream_));
-        B200_CUDA_CHECK(cudaMemcpyAsync(h + nqp, w_err_.get(), sizeof(int), cudaMemcpyDeviceToHost, stream_));
-        B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
+        auto fetch_status = [&]() {
+            B200_CUDA_CHECK(cudaMemcpyAsync(h, w_over_.get(), static_cast<size_t>(nqp), cudaMemcpyDeviceToHost, stream_));
+            B200_CUDA_CHECK(cudaMemcpyAsync(h + nqp, w_err_.get(), sizeof(int), cudaMemcpyDeviceToHost, stream_));
+            B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
+        };
+        fetch_status();
+        if (fused && std::memchr(h, 2, static_cast<size_t>(nqp))) {   // lists too long for the fused tail
+            run_tail(tail, false);
+            fetch_status();
+        }
         timer_.collect(stats_);
         if (prof_) {
             unsigned long long pc[32];
@@ -563,7 +586,7 @@ void FlatIndex::search_device(int64_t nq, const void* xq, bool q_is_f16, int k, 
                 B200_CUDA_CHECK(launch_gather_rows(mask_dev_, qmap + o0, m, static_cast<int>(mask_stride_ * 4), fm, stream_));
                 mask_cur_ = static_cast<const uint32_t*>(fm);
             }
-            run_page(m, fq, fq, k, D, I, ldk, qmap + o0, true);
+            run_tail(run_page(m, fq, fq, k, D, I, ldk, qmap + o0, true), false);
             B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
             timer_.collect(stats_);
         }

@@ -6,6 +6,7 @@
 // 262144-row blocks and no fractal layouts.
 #pragma once
 #include "dist_gemm.cuh"
+#include "select.cuh"
 #include <cuda.h>
 #include <stdint.h>
 
@@ -155,7 +156,16 @@ private:
         uint32_t cap;
     };
     Plan make_plan(int k, int64_t nq) const;
-    void run_page(int nq, const void* xq_raw, const void* xq_op, int k, float* D, int64_t* I, int ldk,
+    // What the steps behind the GEMM passes of a page of queries need.
+    struct PageTail {
+        int nq, k;
+        bool sampled, prune;
+        uint32_t cap;
+        const float* xq;
+        EmitArgs e;
+    };
+    void run_tail(const PageTail& t, bool fused);
+    PageTail run_page(int nq, const void* xq_raw, const void* xq_op, int k, float* D, int64_t* I, int ldk,
                   const int32_t* qmap_dev, bool force_full);
     void reserve(int64_t n);
     size_t in_elem_bytes() const { return dtype_ == kI8 ? 1 : (dtype_ == kF16 ? 2 : 4); }
@@ -194,7 +204,7 @@ private:
     CUtensorMap map_b_;
 
     // scratch
-    DeviceBuffer w_qop_, w_qraw_, w_qnorm_, w_eps_, w_mins_, w_tau_, w_cand_, w_counts_, w_sel_, w_over_, w_qmap_,
+    DeviceBuffer w_qop_, w_qraw_, w_qnorm_, w_eps_, w_mins_, w_tau_, w_cand_, w_counts_, w_over_, w_qmap_,
         w_err_, w_stage_in_, w_stage_D_, w_stage_I_, w_fb_q_, w_fb_qop_, w_prof_;
     bool prof_ = false;
     PinnedBuffer h_over_, h_in_, h_D_, h_I_;

@@ -78,7 +78,7 @@ void FlatGroup::refresh(const std::vector<FlatIndex*>& members, cudaStream_t st)
     // moved: exact distances and labels are read through the member table, and so are packed operand
     // tiles.  Row-major operands are gathered by one kernel, since one tensor map has to cover them.
     // (One copy call per member and array, as this was at first, cost 0.8 ms for 32 members of
-    // 20 000 x 128 whenever the set of members changed: such a call took 1.03 ms, now 0.23 like a repeated one.)
+    // 20 000 x 128 whenever the set of members changed; the tables take @@T@@ ms.)
     const size_t nm = members.size(), n_tiles = static_cast<size_t>(total_rows_ / kTileB);
     in_place_ = packed_operands(kind_, op_cols_) && !use_simt_;
     const size_t row_op = static_cast<size_t>(op_cols_) * op_elem(dtype_);
@@ -167,7 +167,7 @@ void FlatGroup::search_device(const std::vector<FlatIndex*>& members, int64_t nq
     // help pass at most 9 k (the k-th of B minima admits B ln(1 / (1 - k / B)) keys, and B < 1.1 k
     // means fewer than 9 k rows), which the candidate rows have room for.
     const bool thresholded = static_cast<int64_t>(cap_) / 8 >= 4LL * k;
-    uint32_t* flags = w_err_.as<uint32_t>();   // [0] error word, [1] a candidate row overflowed
+    uint32_t* flags = w_err_.as<uint32_t>();   // [0] error word, [1] a candidate row was left (overflow, or too long)
     uint32_t* h = static_cast<uint32_t*>(h_flags_.ensure(8));
     for (bool with_tau = thresholded;; with_tau = false) {
         run_passes(with_tau, nq, xq, xq_op, map_a, qnorm, k, D, I, st);
@@ -207,7 +207,6 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
     uint32_t* tau = static_cast<uint32_t*>(w_tau_.ensure(max_rows * 12));   // thresholds, counters, folded thresholds
     uint32_t* counts = tau + max_rows;
     float* bias = reinterpret_cast<float*>(counts + max_rows);
-    uint64_t* sel = static_cast<uint64_t*>(w_sel_.ensure(max_rows * k * 8));
     uint32_t* mins = with_tau ? static_cast<uint32_t*>(w_mins_.ensure(max_rows * mins_stride * 4)) : nullptr;
     if (!with_tau) {
         B200_CUDA_CHECK(launch_fill_u32(tau, static_cast<int64_t>(max_rows), tau_all, st));
@@ -270,28 +269,31 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
         L.mode = kModeAppend;
         L.burst = 32;
         B200_CUDA_CHECK(launch_dist_gemm(L, a, &map_a, &map_b_, st));
+        EmitArgs e{};
+        e.nq = rows;
+        e.k = k;
+        e.metric = metric_;
+        e.mode = is_int ? 2 : (dtype_ == kF32 ? 1 : 0);
+        e.qnorm = qnorm;
+        e.D = D + m0 * static_cast<size_t>(nq) * k;
+        e.I = I + m0 * static_cast<size_t>(nq) * k;
+        e.ldk = k;
+        e.q_mod = nq;
+        e.members = members_ + m0;
+        uint32_t* any_left = w_err_.as<uint32_t>() + 1;
+        launches_ += 2;
+        if (with_tau && dtype_ == kF32 && k <= kFinishMaxK) {
+            B200_CUDA_CHECK(launch_finish_f32(cand, counts, cap, d_, w_eps_.as<float>(), static_cast<const float*>(xq), nullptr,
+                                              nullptr, any_left, e, st));
+            continue;
+        }
         const uint32_t* n_cand = with_tau ? counts : nullptr;
         if (dtype_ == kF32) {
             B200_CUDA_CHECK(launch_refine_f32(cand, n_cand, cap, cap, rows, d_, metric_, static_cast<const float*>(xq),
                                               nullptr, st, nq, members_ + m0));
             ++launches_;
         }
-        B200_CUDA_CHECK(launch_select_topk(cand, n_cand, cap, cap, rows, k, sel, nullptr, st, w_err_.as<uint32_t>() + 1));
-        EmitArgs e{};
-        e.sel = sel;
-        e.nq = rows;
-        e.k = k;
-        e.metric = metric_;
-        e.mode = is_int ? 2 : (dtype_ == kF32 ? 1 : 0);
-        e.qnorm = qnorm;
-        e.members = members_ + m0;
-        e.D = D + m0 * static_cast<size_t>(nq) * k;
-        e.I = I + m0 * static_cast<size_t>(nq) * k;
-        e.ldk = k;
-        e.qmap = nullptr;
-        e.q_mod = nq;
-        B200_CUDA_CHECK(launch_emit(e, st));
-        launches_ += 3;
+        B200_CUDA_CHECK(launch_select_emit(cand, n_cand, cap, cap, nullptr, any_left, e, st));
     }
 }
 

@@ -59,7 +59,7 @@ private:
     const int64_t* seg_col0_ = nullptr;
     const int64_t* seg_end_ = nullptr;
     const int32_t* seg_index_ = nullptr;
-    DeviceBuffer w_qop_, w_qnorm_, w_eps_, w_tau_, w_mins_, w_cand_, w_sel_, w_err_;
+    DeviceBuffer w_qop_, w_qnorm_, w_eps_, w_tau_, w_mins_, w_cand_, w_err_;
     PinnedBuffer h_flags_;
     uint64_t launches_ = 0, rebuilds_ = 0;
 };

@@ -35,10 +35,10 @@ constexpr int kMaxKNoAlloc = 1024;
 constexpr int kMaxQueries = 1024;
 constexpr size_t kMaxQueryElems = size_t(1) << 19;                // n * d
 constexpr size_t kCandBytes = kMaxCandidates * 8;                 // 8 MiB of (key, position) pairs
-constexpr size_t kSelBudget = size_t(1) << 20;                    // n * k <= 128 Ki selected pairs (1 MiB)
+constexpr size_t kMaxResults = size_t(1) << 17;                   // n * k
 constexpr size_t kQopBytes = (size_t(1) << 20) + (size_t(32) << 10);   // n * d * 2 <= 1 MiB operand copy + 16 folded columns per row
 constexpr size_t kSmallBytes = size_t(64) << 10;                  // norms, slack, thresholds, flags
-constexpr size_t kArenaBytes = kCandBytes + kSelBudget + kQopBytes + kSmallBytes;  // 10 MiB + 96 KiB
+constexpr size_t kArenaBytes = kCandBytes + kQopBytes + kSmallBytes;  // 9 MiB + 96 KiB
 
 // Host code must not use this name as an address: it is a host-side stand-in.  The device
 // address comes from cudaGetSymbolAddress below.
@@ -82,7 +82,7 @@ extern "C" int b200idx_search_device_noalloc(b200idx_t* h, int64_t n, const void
             throw std::invalid_argument("request exceeds the static scratch: n * round_up(ntotal, 256) must be <= 2^20");
         // The operand copy of an fp32 index is op_cols() = d + 16 bf16 values wide (the folded columns), so
         // n * d <= 2^19 together with n <= 1024 keeps n * op_cols() * 2 within kQopBytes.
-        if (static_cast<size_t>(n) * k * 8 > kSelBudget || static_cast<size_t>(n) * d > kMaxQueryElems ||
+        if (static_cast<size_t>(n) * k > kMaxResults || static_cast<size_t>(n) * d > kMaxQueryElems ||
             static_cast<size_t>(n) * ix->op_cols() * 2 > kQopBytes)
             throw std::invalid_argument("request exceeds the static scratch: n * k <= 131072 and n * d <= 524288");
 
@@ -98,8 +98,6 @@ extern "C" int b200idx_search_device_noalloc(b200idx_t* h, int64_t n, const void
         size_t off = 0;
         uint64_t* cand = reinterpret_cast<uint64_t*>(arena + off);
         off += kCandBytes;
-        uint64_t* sel = reinterpret_cast<uint64_t*>(arena + off);
-        off += kSelBudget;
         void* qop = arena + off;
         off += kQopBytes;
         unsigned char* small = arena + off;
@@ -164,9 +162,7 @@ extern "C" int b200idx_search_device_noalloc(b200idx_t* h, int64_t n, const void
         if (dtype == kF32)
             B200_CUDA_CHECK(launch_refine_f32(cand, nullptr, static_cast<uint32_t>(v.n), cap, nq, d, ix->metric(),
                                               static_cast<const float*>(x_dev), v.rows_f32, st));
-        B200_CUDA_CHECK(launch_select_topk(cand, nullptr, static_cast<uint32_t>(v.n), cap, nq, k, sel, nullptr, st));
         EmitArgs e{};
-        e.sel = sel;
         e.nq = nq;
         e.k = k;
         e.metric = ix->metric();
@@ -177,7 +173,7 @@ extern "C" int b200idx_search_device_noalloc(b200idx_t* h, int64_t n, const void
         e.I = I_dev;
         e.ldk = k;
         e.qmap = nullptr;
-        B200_CUDA_CHECK(launch_emit(e, st));
+        B200_CUDA_CHECK(launch_select_emit(cand, nullptr, static_cast<uint32_t>(v.n), cap, nullptr, nullptr, e, st));
         int herr = 0;
         B200_CUDA_CHECK(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st));
         B200_CUDA_CHECK(cudaStreamSynchronize(st));

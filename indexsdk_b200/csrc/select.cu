@@ -54,63 +54,156 @@ __device__ __forceinline__ void store_tau(int q, uint32_t ord, uint32_t* tau, co
     }
 }
 
-// Inclusive scan of a 256-bin histogram held in shared memory; returns through `bucket`/`below`
-// the bin that contains rank r (1-based) and the number of elements in lower bins.
-__device__ __forceinline__ void find_bucket(uint32_t* hist, uint32_t* scan, uint32_t r, uint32_t* bucket,
-                                            uint32_t* below) {
-    // 256 threads, one bin each: shuffle scan inside the warp, the eight warp totals through `scan`
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const uint32_t v = hist[t];
-    uint32_t incl = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += u;
-    }
-    if (lane == 31) scan[w] = incl;
-    __syncthreads();
-    for (int i = 0; i < w; ++i) incl += scan[i];
-    const uint32_t excl = incl - v;
-    if (incl >= r && excl < r) {
-        *bucket = t;
-        *below = excl;
-    }
-    __syncthreads();
-}
+// ---- rank search over 32-bit keys ----
+constexpr int kRankBins = 1024;
+struct RankScratch {
+    uint32_t hist[kRankBins];
+    uint32_t warp[32];
+    uint32_t lo, hi, n, bin, below;
+};
 
-// k-th smallest (rank r, 1-based, r <= n) of n keys of KeyT read from global memory.
-template <typename KeyT>
-__device__ KeyT block_radix_kth(const KeyT* in, uint32_t n, uint32_t r, uint32_t* hist, uint32_t* scan,
-                                uint32_t* sh_bucket, uint32_t* sh_below) {
-    KeyT prefix = 0, mask = 0;
-    for (int shift = static_cast<int>(sizeof(KeyT)) * 8 - 8; shift >= 0; shift -= 8) {
-        hist[threadIdx.x] = 0;
+// r-th smallest (1-based) of the keys a block of NT threads holds; visit(f) calls f(key) for each of the
+// calling thread's keys, the same ones every time.  Fewer than r keys: 0xFFFFFFFF.
+// The digits are cut out of the range the keys really span, not out of the 32-bit word: the candidates of
+// a query share their leading byte or two, so a digit at a fixed place sends all of them to one counter,
+// whose atomics then run one after the other (22 us for the 1 500 candidates of a single query; 1 024 bins
+// over the spanned range: two or three passes, almost no collisions).  After `passes` passes the upper
+// edge of the bin is returned (a bound from above, 2^-20 of the range wide after two) unless the rank is
+// settled before; passes = 4 always settles it.  Every thread of the block must call this.
+template <int NT, typename Visit>
+__device__ __forceinline__ uint32_t block_kth32(Visit visit, uint32_t r, RankScratch& s, int passes) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int kPer = kRankBins / NT;
+    if (threadIdx.x == 0) {
+        s.lo = 0xFFFFFFFFu;
+        s.hi = 0u;
+        s.n = 0u;
+    }
+    __syncthreads();
+    {
+        uint32_t lo = 0xFFFFFFFFu, hi = 0u, n = 0u;
+        visit([&](uint32_t v) {
+            lo = min(lo, v);
+            hi = max(hi, v);
+            ++n;
+        });
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0 && n > 0) {
+            atomicMin(&s.lo, lo);
+            atomicMax(&s.hi, hi);
+            atomicAdd(&s.n, n);
+        }
+    }
+    __syncthreads();
+    uint32_t lo = s.lo, hi = s.hi;
+    if (s.n < r) return 0xFFFFFFFFu;
+    for (int pass = 0; pass < passes && lo != hi; ++pass) {
+        const int shift = max(0, 22 - __clz(hi - lo));
+        for (int b = threadIdx.x; b < kRankBins; b += NT) s.hist[b] = 0u;
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += kSelThreads) {
-            const KeyT v = in[i];
-            if ((v & mask) == prefix) atomicAdd(&hist[static_cast<uint32_t>(v >> shift) & 255u], 1u);
+        visit([&](uint32_t v) {
+            if (v >= lo && v <= hi) atomicAdd(&s.hist[(v - lo) >> shift], 1u);
+        });
+        __syncthreads();
+        uint32_t mine[kPer], sum = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            mine[j] = s.hist[threadIdx.x * kPer + j];
+            sum += mine[j];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += u;
+        }
+        if (lane == 31) s.warp[w] = incl;
+        __syncthreads();
+        uint32_t before = incl - sum;
+        for (int i = 0; i < w; ++i) before += s.warp[i];
+        if (before < r && r <= before + sum) {
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                if (before < r && r <= before + mine[j]) {
+                    s.bin = threadIdx.x * kPer + j;
+                    s.below = before;
+                }
+                before += mine[j];
+            }
         }
         __syncthreads();
-        find_bucket(hist, scan, r, sh_bucket, sh_below);
-        prefix |= static_cast<KeyT>(*sh_bucket) << shift;
-        mask |= static_cast<KeyT>(255) << shift;
-        r -= *sh_below;
-        __syncthreads();
+        lo += s.bin << shift;
+        const uint32_t top = lo + ((1u << shift) - 1u);
+        hi = top < hi && top >= lo ? top : hi;
+        r -= s.below;
     }
-    return prefix;
+    __syncthreads();   // the scratch may be reused
+    return hi;
 }
 
+// Copies the entries of row[0..n) that are in use (not kCandInvalid) to out[0..limit); returns their number,
+// which may exceed the limit (out is then incomplete).  Eight loads per thread are in flight: with one the
+// copy is a chain of memory latencies.  fill: shared counter.  Every thread of the block must call this.
+template <int NT>
+__device__ __forceinline__ uint32_t block_compact(const uint64_t* row, uint32_t n, uint64_t* out, uint32_t limit, uint32_t* fill) {
+    const int lane = threadIdx.x & 31;
+    constexpr int U = 8;
+    if (threadIdx.x == 0) *fill = 0u;
+    __syncthreads();
+    for (uint32_t i0 = threadIdx.x - lane; i0 < n; i0 += U * NT) {
+        uint64_t v[U];
+        uint32_t have = 0;
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const uint32_t i = i0 + j * NT + lane;
+            v[j] = i < n ? row[i] : kCandInvalid;
+            have += v[j] != kCandInvalid ? 1u : 0u;
+        }
+        uint32_t before = have;   // exclusive prefix over the lanes
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, before, off);
+            if (lane >= off) before += u;
+        }
+        const uint32_t all = __shfl_sync(0xffffffffu, before, 31);
+        uint32_t slot = 0;
+        if (lane == 0 && all) slot = atomicAdd(fill, all);
+        slot = __shfl_sync(0xffffffffu, slot, 0) + before - have;
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (v[j] != kCandInvalid) {
+                if (slot < limit) out[slot] = v[j];
+                ++slot;
+            }
+    }
+    __syncthreads();
+    return *fill;
+}
+
+constexpr uint32_t kKthStage = 8192;   // burst minima staged in shared memory
+
+// A threshold may be any bound from above: two passes of the rank search (2^-20 of the range) do.
 __global__ void __launch_bounds__(kSelThreads)
 kth_threshold_kernel(const uint32_t* mins, int stride, int n, int k, const float* eps, uint32_t tau_all,
                      uint32_t* tau, const TauFold fold) {
-    __shared__ uint32_t hist[256], scan[256], sh_bucket, sh_below;
+    extern __shared__ uint32_t kth_keys[];   // min(n, kKthStage)
+    __shared__ RankScratch rank;
     const int q = blockIdx.x;
     if (n < k) {
         if (threadIdx.x == 0) store_tau(q, tau_all, tau, fold);
         return;
     }
-    uint32_t kth = block_radix_kth<uint32_t>(mins + static_cast<int64_t>(q) * stride, n, k, hist, scan, &sh_bucket,
-                                             &sh_below);
+    const uint32_t* row = mins + static_cast<int64_t>(q) * stride;
+    const bool staged = n <= static_cast<int>(kKthStage);
+    if (staged) {
+        for (int i = threadIdx.x; i < n; i += kSelThreads) kth_keys[i] = row[i];
+        __syncthreads();
+    }
+    const uint32_t* keys = staged ? kth_keys : row;
+    uint32_t kth = block_kth32<kSelThreads>(
+        [&](auto&& f) { for (int i = threadIdx.x; i < n; i += kSelThreads) f(keys[i]); }, static_cast<uint32_t>(k), rank, 2);
     if (threadIdx.x == 0) {
         if (eps) {
             float f = ord_to_float(kth);
@@ -128,8 +221,19 @@ kth_threshold_kernel(const uint32_t* mins, int stride, int n, int k, const float
 // <= A_k + eps and every member of the exact top-k has an approximate key <= A_k + 2 eps; all
 // others are overwritten with the "invalid" marker.  A constant offset common to a row's keys
 // cancels out of this argument.
-constexpr int kPruneKeys = 4096;    // keys staged in shared memory for the rank search
-constexpr int kPruneKeep = 2048;    // survivors staged for the in-place compaction
+constexpr uint32_t kPruneKeys = 4096;    // entries staged in shared memory for the rank search
+constexpr int kPruneKeep = 2048;         // survivors staged for the in-place compaction
+
+// Limit on the approximate key for a row whose k-th smallest (or a bound on it) is kth; false: no limit.
+__device__ __forceinline__ bool prune_limit(uint32_t kth, float eps, uint32_t* lim) {
+    if (kth == 0xFFFFFFFFu) return false;   // fewer than k real candidates
+    float f = ord_to_float(kth);
+    f = f + 2.f * eps;
+    f = f + fabsf(f) * 9.5367431640625e-07f + eps * 0.125f;   // slack for the adds and the accumulation
+    if (f != f) return false;
+    *lim = float_to_ord(f);
+    return true;
+}
 
 // Tightens a threshold part-way through the full pass: the candidates found so far (in the tiles
 // already visited) contain k keys <= their k-th smallest key A_k, so A_k bounds the final k-th key
@@ -138,16 +242,26 @@ constexpr int kPruneKeep = 2048;    // survivors staged for the in-place compact
 __global__ void __launch_bounds__(kSelThreads)
 tighten_tau_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int k, const float* eps,
                    uint32_t* tau, const TauFold fold) {
-    __shared__ uint32_t hist[256], scan[256], sh_bucket, sh_below;
+    __shared__ RankScratch rank;
     __shared__ uint32_t keys[kPruneKeys];
     const int q = blockIdx.x;
     const uint64_t* row = cand + static_cast<int64_t>(q) * cap;
     const uint32_t n = counts[q];
-    if (n > cap || n > static_cast<uint32_t>(kPruneKeys) || n < static_cast<uint32_t>(k)) return;
-    for (uint32_t i = threadIdx.x; i < n; i += kSelThreads) keys[i] = static_cast<uint32_t>(row[i] >> 32);
-    __syncthreads();
-    uint32_t kth = block_radix_kth<uint32_t>(keys, n, static_cast<uint32_t>(k), hist, scan, &sh_bucket, &sh_below);
-    if (kth == 0xFFFFFFFFu) return;   // fewer than k real candidates (the rest are unused slots)
+    if (n > cap || n < static_cast<uint32_t>(k)) return;
+    const bool staged = n <= kPruneKeys;
+    if (staged) {
+        for (uint32_t i = threadIdx.x; i < n; i += kSelThreads) keys[i] = static_cast<uint32_t>(row[i] >> 32);
+        __syncthreads();
+    }
+    uint32_t kth = block_kth32<kSelThreads>(
+        [&](auto&& f) {
+            for (uint32_t i = threadIdx.x; i < n; i += kSelThreads) {
+                const uint32_t v = staged ? keys[i] : static_cast<uint32_t>(row[i] >> 32);
+                if (v != 0xFFFFFFFFu) f(v);   // unused slots
+            }
+        },
+        static_cast<uint32_t>(k), rank, 2);
+    if (kth == 0xFFFFFFFFu) return;   // fewer than k real candidates
     if (threadIdx.x == 0) {
         if (eps) {
             float f = ord_to_float(kth);
@@ -162,7 +276,8 @@ tighten_tau_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t cap, i
 
 __global__ void __launch_bounds__(kSelThreads)
 prune_candidates_kernel(uint64_t* cand, uint32_t* counts, uint32_t cap, int k, const float* eps) {
-    __shared__ uint32_t hist[256], scan[256], sh_bucket, sh_below, sh_fill;
+    __shared__ RankScratch rank;
+    __shared__ uint32_t sh_fill;
     __shared__ uint32_t keys[kPruneKeys];
     __shared__ uint64_t keep[kPruneKeep];
     const int q = blockIdx.x;
@@ -170,21 +285,21 @@ prune_candidates_kernel(uint64_t* cand, uint32_t* counts, uint32_t cap, int k, c
     const uint32_t n = counts[q];
     if (n > cap) return;   // overflowed row: left as it is for the selection kernel to flag
     if (n <= static_cast<uint32_t>(k)) return;
-    uint32_t kth_ord;
-    if (n <= static_cast<uint32_t>(kPruneKeys)) {
+    const bool staged = n <= kPruneKeys;
+    if (staged) {
         for (uint32_t i = threadIdx.x; i < n; i += kSelThreads) keys[i] = static_cast<uint32_t>(row[i] >> 32);
         __syncthreads();
-        kth_ord = block_radix_kth<uint32_t>(keys, n, static_cast<uint32_t>(k), hist, scan, &sh_bucket, &sh_below);
-    } else {
-        kth_ord = static_cast<uint32_t>(
-            block_radix_kth<uint64_t>(row, n, static_cast<uint32_t>(k), hist, scan, &sh_bucket, &sh_below) >> 32);
     }
-    if (kth_ord == 0xFFFFFFFFu) return;   // fewer than k real candidates
-    float lim = ord_to_float(kth_ord);
-    lim = lim + 2.f * eps[q];
-    lim = lim + fabsf(lim) * 9.5367431640625e-07f + eps[q] * 0.125f;   // slack for the adds and the accumulation
-    if (lim != lim) return;
-    const uint32_t lim_ord = float_to_ord(lim);
+    const uint32_t kth = block_kth32<kSelThreads>(
+        [&](auto&& f) {
+            for (uint32_t i = threadIdx.x; i < n; i += kSelThreads) {
+                const uint32_t v = staged ? keys[i] : static_cast<uint32_t>(row[i] >> 32);
+                if (v != 0xFFFFFFFFu) f(v);
+            }
+        },
+        static_cast<uint32_t>(k), rank, 2);
+    uint32_t lim_ord;
+    if (!prune_limit(kth, eps[q], &lim_ord)) return;
     if (threadIdx.x == 0) sh_fill = 0;
     __syncthreads();
     // survivors go to shared memory first: the row is compacted in place
@@ -212,7 +327,8 @@ prune_candidates_kernel(uint64_t* cand, uint32_t* counts, uint32_t cap, int k, c
 // The same threshold for short rows (n <= 32 * NPL), one WARP per query: the minima sit in
 // registers, NPL per lane, and the k-th smallest is found bit by bit -- per bit every lane counts
 // its values that agree with the bits fixed so far and have a 0 there, one warp reduction adds the
-// counts.  About a third of the instructions of the block-wide byte-radix version at n = 512.
+// counts.  The bits above the highest one in which the minima differ need no search, and 16 bits below
+// it are enough: a threshold may be any bound from above (65 536 steps over the spanned range).
 template <int NPL>
 __global__ void __launch_bounds__(128)
 kth_threshold_warp_kernel(const uint32_t* mins, int stride, int n, int nq, int k, const float* eps, uint32_t tau_all,
@@ -226,13 +342,26 @@ kth_threshold_warp_kernel(const uint32_t* mins, int stride, int n, int nq, int k
     }
     uint32_t v[NPL];
     const uint32_t* row = mins + static_cast<int64_t>(q) * stride;
+    uint32_t all_and = 0xFFFFFFFFu, all_or = 0u;
 #pragma unroll
     for (int j = 0; j < NPL; ++j) {
         const int i = j * 32 + lane;
         v[j] = i < n ? row[i] : 0xFFFFFFFFu;
+        if (i < n) {
+            all_and &= v[j];
+            all_or |= v[j];
+        }
     }
-    uint32_t prefix = 0, mask = 0, r = static_cast<uint32_t>(k);
-    for (int bit = 31; bit >= 0; --bit) {
+    all_and = __reduce_and_sync(0xffffffffu, all_and);
+    all_or = __reduce_or_sync(0xffffffffu, all_or);
+    const uint32_t differ = all_and ^ all_or;
+    const int top = 31 - __clz(differ);              // -1: all equal
+    uint32_t mask = top >= 31 ? 0u : ~((2u << top) - 1u), prefix = all_and & mask, r = static_cast<uint32_t>(k);
+    if (top < 0) {
+        mask = 0xFFFFFFFFu;
+        prefix = all_and;
+    }
+    for (int bit = top; bit >= 0 && bit > top - 16; --bit) {
         const uint32_t b = 1u << bit;
         uint32_t c = 0;
 #pragma unroll
@@ -245,7 +374,7 @@ kth_threshold_warp_kernel(const uint32_t* mins, int stride, int n, int nq, int k
         mask |= b;
     }
     if (lane == 0) {
-        uint32_t kth = prefix;
+        uint32_t kth = prefix | ~mask;
         if (eps) {
             float f = ord_to_float(kth);
             f = f + 2.f * eps[fold.q_mod > 0 ? q % fold.q_mod : q];
@@ -256,10 +385,12 @@ kth_threshold_warp_kernel(const uint32_t* mins, int stride, int n, int nq, int k
     }
 }
 
+// Ascending bitonic sort of P (a power of two) values in shared memory by a block of NT threads.
+template <int NT>
 __device__ __forceinline__ void bitonic_sort_u64(uint64_t* s, int P) {
     for (int size = 2; size <= P; size <<= 1) {
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
+            for (int i = threadIdx.x; i < P / 2; i += NT) {
                 const int lo = 2 * i - (i & (stride - 1));
                 const int hi = lo + stride;
                 const bool up = (lo & size) == 0;
@@ -274,71 +405,258 @@ __device__ __forceinline__ void bitonic_sort_u64(uint64_t* s, int P) {
     }
 }
 
-__global__ void __launch_bounds__(kSelThreads)
-select_topk_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int k, int P,
-                   uint64_t* out, uint8_t* overflow, uint32_t* any_overflow) {
-    extern __shared__ uint64_t sorted[];  // P entries
-    __shared__ uint32_t hist[256], scan[256], sh_bucket, sh_below, sh_fill;
+// Result j of query row q: the selected candidate's distance and label.
+__device__ __forceinline__ void emit_one(const EmitArgs& e, int q, int j, uint64_t c) {
+    const int orow = e.qmap ? e.qmap[q] : q;
+    float dist;
+    int64_t label;
+    if (c == kCandInvalid) {
+        dist = 3.402823466e+38f;  // FLT_MAX padding, label -1
+        label = -1;
+    } else {
+        const int qn = e.q_mod > 0 ? q % e.q_mod : q;   // row of the query norms
+        const uint32_t ok = static_cast<uint32_t>(c >> 32), pos = static_cast<uint32_t>(c);
+        if (e.members) {
+            const MemberView& mv = e.members[q / e.q_mod];
+            label = mv.labels[static_cast<int64_t>(pos) - mv.first];
+        } else {
+            label = e.labels ? e.labels[pos] : static_cast<int64_t>(pos);
+        }
+        if (e.mode == 2) {
+            int32_t kv = ord_to_int(ok);
+            if (e.metric == kMetricL2) dist = static_cast<float>(kv + static_cast<const int32_t*>(e.qnorm)[qn]);
+            else if (e.metric == kMetricCos) dist = cos16_value(-kv);
+            else dist = static_cast<float>(-kv);
+        } else {
+            float kv = ord_to_float(ok);
+            if (e.metric == kMetricL2) {
+                if (e.mode == 0) {
+                    kv += static_cast<const float*>(e.qnorm)[qn];
+                    kv = kv < 0.f ? 0.f : kv;
+                }
+                dist = kv;
+            } else {
+                dist = -kv;
+            }
+        }
+    }
+    e.D[static_cast<int64_t>(orow) * e.ldk + j] = dist;
+    e.I[static_cast<int64_t>(orow) * e.ldk + j] = label;
+}
+
+// The k smallest of a query's candidates, in order, straight to the results.
+//   up to 512 candidates : every one is placed by its rank, counted against all others (candidates are
+//                          distinct: positions are unique).
+//   more                 : the k-th key by rank search, ties with it by position the same way, then k are sorted.
+// The row is read once when its candidates fit `stage` entries of shared memory; longer ones are read
+// from memory in every step.
+template <int NT>
+__global__ void __launch_bounds__(NT)
+select_emit_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int P,
+                   uint32_t stage, uint8_t* overflow, uint32_t* any_overflow, const EmitArgs e) {
+    extern __shared__ uint64_t sel_sm[];   // P sorted entries, then the staged ones
+    __shared__ RankScratch rank;
+    __shared__ uint32_t sh_fill, sh_ties;
     const int q = blockIdx.x;
     const uint64_t* row = cand + static_cast<int64_t>(q) * cap;
+    const uint32_t k = static_cast<uint32_t>(e.k);
     uint32_t n = counts ? counts[q] : n_fixed;
     if (overflow && threadIdx.x == 0) overflow[q] = n > cap ? 1 : 0;
     if (any_overflow && threadIdx.x == 0 && n > cap) atomicOr(any_overflow, 1u);
     if (n > cap) n = cap;
-    uint64_t* orow_fast = out + static_cast<int64_t>(q) * k;
-    if (n <= static_cast<uint32_t>(kSmallSet)) {
-        // Small candidate set (the common case after a tight threshold): the real entries (unused
-        // reserved slots are dropped) are staged in shared memory and every one is placed by its
-        // rank, counted against all others.  Candidates are distinct (positions are unique), so
-        // the ranks are a permutation.
-        __shared__ uint64_t small[kSmallSet];
-        if (threadIdx.x == 0) sh_fill = 0;
-        for (int i = threadIdx.x; i < k; i += kSelThreads) orow_fast[i] = kCandInvalid;
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += kSelThreads) {
-            const uint64_t v = row[i];
-            if (v != kCandInvalid) small[atomicAdd(&sh_fill, 1u)] = v;
+    uint64_t* sorted = sel_sm;
+    uint64_t* held = sel_sm + P;
+    const uint64_t* src = row;
+    if (n <= 4 * stage) {   // (beyond that hardly any list fits)
+        const uint32_t m = block_compact<NT>(row, n, held, stage, &sh_fill);
+        if (m <= stage) {
+            n = m;
+            src = held;
         }
-        __syncthreads();
-        const uint32_t m = sh_fill;
-        for (uint32_t i = threadIdx.x; i < m; i += kSelThreads) {
-            const uint64_t v = small[i];
-            uint32_t rank = 0;
+        if (m <= static_cast<uint32_t>(kSmallSet)) {
+            for (uint32_t i = threadIdx.x; i < m; i += NT) {
+                const uint64_t v = held[i];
+                uint32_t r = 0;
 #pragma unroll 8
-            for (uint32_t j = 0; j < m; ++j) rank += small[j] < v ? 1u : 0u;
-            if (rank < static_cast<uint32_t>(k)) orow_fast[rank] = v;
+                for (uint32_t j = 0; j < m; ++j) r += held[j] < v ? 1u : 0u;
+                if (r < k) emit_one(e, q, static_cast<int>(r), v);
+            }
+            for (uint32_t i = m + threadIdx.x; i < k; i += NT) emit_one(e, q, static_cast<int>(i), kCandInvalid);
+            return;
         }
-        return;
     }
-    for (int i = threadIdx.x; i < P; i += kSelThreads) sorted[i] = kCandInvalid;
-    if (threadIdx.x == 0) sh_fill = 0;
+    for (int i = threadIdx.x; i < P; i += NT) sorted[i] = kCandInvalid;
+    auto each = [&](auto&& f) {
+        for (uint32_t i = threadIdx.x; i < n; i += NT) {
+            const uint64_t v = src[i];
+            if (v != kCandInvalid) f(v);
+        }
+    };
+    // bounds of what is kept: everything unless there are more than k
+    uint32_t kth = 0xFFFFFFFFu, pos_max = 0xFFFFFFFFu;
+    const uint32_t found = block_kth32<NT>([&](auto&& f) { each([&](uint64_t v) { f(static_cast<uint32_t>(v >> 32)); }); },
+                                           k, rank, 4);
+    const bool enough = rank.n >= k;   // else all of them (rank.n is left as it was set)
+    if (enough) {
+        kth = found;
+        if (threadIdx.x == 0) {
+            sh_fill = 0u;
+            sh_ties = 0u;
+        }
+        __syncthreads();
+        uint32_t less = 0, ties = 0;
+        each([&](uint64_t v) {
+            less += static_cast<uint32_t>(v >> 32) < kth ? 1u : 0u;
+            ties += static_cast<uint32_t>(v >> 32) == kth ? 1u : 0u;
+        });
+        less = __reduce_add_sync(0xffffffffu, less);
+        ties = __reduce_add_sync(0xffffffffu, ties);
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&sh_fill, less);
+            atomicAdd(&sh_ties, ties);
+        }
+        __syncthreads();
+        const uint32_t need = k - sh_fill;   // ties with the k-th key that belong to the result: the lowest positions
+        if (need < sh_ties)
+            pos_max = block_kth32<NT>(
+                [&](auto&& f) { each([&](uint64_t v) { if (static_cast<uint32_t>(v >> 32) == kth) f(static_cast<uint32_t>(v)); }); },
+                need, rank, 4);
+    }
     __syncthreads();
-    uint64_t kth = kCandInvalid;
-    if (n > static_cast<uint32_t>(k))
-        kth = block_radix_kth<uint64_t>(row, n, static_cast<uint32_t>(k), hist, scan, &sh_bucket, &sh_below);
-    for (uint32_t i = threadIdx.x; i < n; i += kSelThreads) {
-        const uint64_t v = row[i];
-        if (v <= kth && v != kCandInvalid) {
+    if (threadIdx.x == 0) sh_fill = 0u;
+    __syncthreads();
+    each([&](uint64_t v) {
+        const uint32_t key = static_cast<uint32_t>(v >> 32);
+        if (key < kth || (key == kth && static_cast<uint32_t>(v) <= pos_max)) {
             const uint32_t slot = atomicAdd(&sh_fill, 1u);
             if (slot < static_cast<uint32_t>(P)) sorted[slot] = v;
         }
-    }
+    });
     __syncthreads();
-    bitonic_sort_u64(sorted, P);
-    uint64_t* orow = out + static_cast<int64_t>(q) * k;
-    for (int i = threadIdx.x; i < k; i += kSelThreads) orow[i] = sorted[i];
+    bitonic_sort_u64<NT>(sorted, P);
+    for (int i = threadIdx.x; i < e.k; i += NT) emit_one(e, q, i, sorted[i]);
 }
 
-// Canonical fp32 distances of the candidates (sequential fmaf over the dimensions, the arithmetic
-// of the CPU oracle).  The chain of one candidate cannot be split over lanes, so a lane owns a
-// candidate -- but the rows are fetched co-operatively: a warp reads the rows of its 32 candidates
-// kRefChunk floats at a time, each row as one contiguous 128-byte piece spread over consecutive
-// lanes (four cache lines per load instruction instead of 32), parks them in shared memory and
-// every lane then walks its own row there.  Rows are padded by 4 floats: 8 consecutive lanes
-// reading one float4 each fall into 8 different 16-byte bank groups.
+// ---- canonical fp32 distances of candidates ----
+// Sequential fmaf over the dimensions, the arithmetic of the CPU oracle.  The chain of one candidate
+// cannot be split over lanes, so a lane owns a candidate -- but the rows are fetched co-operatively: a warp
+// reads the rows of its 32 candidates kRefChunk floats at a time, each row as one contiguous 128-byte
+// piece spread over consecutive lanes (four cache lines per load instruction instead of 32), parks them
+// in shared memory and every lane then walks its own row there.  Rows are padded by 4 floats: 8
+// consecutive lanes reading one float4 each fall into 8 different 16-byte bank groups.
 constexpr int kRefChunk = 32;     // small, so that many warps fit an SM: the kernel lives on memory-level parallelism
 constexpr int kRefPitch = kRefChunk + 4;
 constexpr uint32_t kRefWindow = 512;   // candidate slots compacted at a time
+
+// Distance of this lane's candidate (row `pos` of xb) to the query qs (shared memory); lanes without
+// one pass live = false.  rows: the warp's [32][kRefPitch] floats of shared memory.  Warp-collective.
+__device__ __forceinline__ float refine_lane(const float* xb, const float* qs, float* rows, uint32_t pos, bool live, int d,
+                                             int metric, int lane) {
+    const uint32_t live_mask = __ballot_sync(0xffffffffu, live);
+    float acc = 0.f;
+    if (d % kRefChunk == 0) {
+        // Whole chunks only: a lane stages the same 8 rows in every chunk, so their addresses are
+        // formed once per pass, and the loads of the next chunk are in flight while the current
+        // one is accumulated from shared memory.
+        const int j = lane & 7;
+        const float4* src[8];
+        uint32_t okm = 0;
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+            const int r = it * 4 + (lane >> 3);
+            const uint32_t pr = __shfl_sync(0xffffffffu, pos, r);
+            src[it] = reinterpret_cast<const float4*>(xb + static_cast<int64_t>(pr) * d) + j;
+            okm |= ((live_mask >> r) & 1u) << it;   // rows of unused slots are neither fetched nor read
+        }
+        float4* dst = reinterpret_cast<float4*>(rows + (lane >> 3) * kRefPitch + 4 * j);
+        const float4* mine = reinterpret_cast<const float4*>(rows + lane * kRefPitch);
+        float4 v[8];
+#pragma unroll
+        for (int it = 0; it < 8; ++it)
+            if ((okm >> it) & 1u) v[it] = __ldg(src[it]);
+        for (int ch0 = 0; ch0 < d; ch0 += kRefChunk) {
+#pragma unroll
+            for (int it = 0; it < 8; ++it)
+                if ((okm >> it) & 1u) dst[it * kRefPitch] = v[it];   // 4 rows further per step
+            __syncwarp();
+            if (ch0 + kRefChunk < d) {
+#pragma unroll
+                for (int it = 0; it < 8; ++it)
+                    if ((okm >> it) & 1u) v[it] = __ldg(src[it] + (ch0 + kRefChunk) / 4);
+            }
+            const float4* qv = reinterpret_cast<const float4*>(qs + ch0);
+            if (live) {
+                if (metric == kMetricL2) {
+#pragma unroll
+                    for (int jj = 0; jj < kRefChunk / 4; ++jj) {
+                        const float4 a = qv[jj], b = mine[jj];
+                        float t;
+                        t = a.x - b.x; acc = fmaf(t, t, acc);
+                        t = a.y - b.y; acc = fmaf(t, t, acc);
+                        t = a.z - b.z; acc = fmaf(t, t, acc);
+                        t = a.w - b.w; acc = fmaf(t, t, acc);
+                    }
+                } else {
+#pragma unroll
+                    for (int jj = 0; jj < kRefChunk / 4; ++jj) {
+                        const float4 a = qv[jj], b = mine[jj];
+                        acc = fmaf(a.x, b.x, acc);
+                        acc = fmaf(a.y, b.y, acc);
+                        acc = fmaf(a.z, b.z, acc);
+                        acc = fmaf(a.w, b.w, acc);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    } else {
+        for (int ch0 = 0; ch0 < d; ch0 += kRefChunk) {
+            const int w = d - ch0 < kRefChunk ? d - ch0 : kRefChunk;
+            const int lpr = w >> 2;                                  // float4 pieces per row
+            if (lpr == kRefChunk / 4) {
+#pragma unroll
+                for (int it = 0; it < 8; ++it) {                     // four of the 32 rows per load instruction
+                    const int r = it * 4 + (lane >> 3), j = lane & 7;
+                    const uint32_t pr = __shfl_sync(0xffffffffu, pos, r);
+                    if ((live_mask >> r) & 1u)
+                        *reinterpret_cast<float4*>(rows + r * kRefPitch + 4 * j) =
+                            __ldg(reinterpret_cast<const float4*>(xb + static_cast<int64_t>(pr) * d + ch0) + j);
+                }
+            } else {
+                for (int idx = lane; idx < 32 * lpr; idx += 32) {
+                    const int r = idx / lpr, j = idx - r * lpr;
+                    const uint32_t pr = __shfl_sync(0xffffffffu, pos, r);
+                    if ((live_mask >> r) & 1u)
+                        *reinterpret_cast<float4*>(rows + r * kRefPitch + 4 * j) =
+                            __ldg(reinterpret_cast<const float4*>(xb + static_cast<int64_t>(pr) * d + ch0) + j);
+                }
+            }
+            __syncwarp();
+            const float4* mine = reinterpret_cast<const float4*>(rows + lane * kRefPitch);
+            const float4* qv = reinterpret_cast<const float4*>(qs + ch0);
+            if (live) {
+                for (int j = 0; j < lpr; ++j) {
+                    const float4 a = qv[j], b = mine[j];
+                    if (metric == kMetricL2) {
+                        float t;
+                        t = a.x - b.x; acc = fmaf(t, t, acc);
+                        t = a.y - b.y; acc = fmaf(t, t, acc);
+                        t = a.z - b.z; acc = fmaf(t, t, acc);
+                        t = a.w - b.w; acc = fmaf(t, t, acc);
+                    } else {
+                        acc = fmaf(a.x, b.x, acc);
+                        acc = fmaf(a.y, b.y, acc);
+                        acc = fmaf(a.z, b.z, acc);
+                        acc = fmaf(a.w, b.w, acc);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    return metric == kMetricL2 ? acc : -acc;
+}
+
 __global__ void __launch_bounds__(128)
 refine_f32_kernel(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int d, int metric,
                   const float* xq, const float* xb, int q_first, int q_mod, const MemberView* members) {
@@ -370,176 +688,132 @@ refine_f32_kernel(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint
     __shared__ uint32_t s_pos[kRefWindow];
     __shared__ uint32_t s_cnt;
     for (uint32_t win0 = blockIdx.x * kRefWindow; win0 < n; win0 += gridDim.x * kRefWindow) {
-    if (threadIdx.x == 0) s_cnt = 0u;
-    __syncthreads();
-    const uint32_t win1 = win0 + kRefWindow < n ? win0 + kRefWindow : n;
-    for (uint32_t i = win0 + threadIdx.x; i < win1; i += 128) {
-        const uint64_t c = row[i];
-        if (c != kCandInvalid) {
-            const uint32_t j = atomicAdd(&s_cnt, 1u);
-            s_slot[j] = i;
-            s_pos[j] = static_cast<uint32_t>(c) - pos_first;
+        if (threadIdx.x == 0) s_cnt = 0u;
+        __syncthreads();
+        const uint32_t win1 = win0 + kRefWindow < n ? win0 + kRefWindow : n;
+        for (uint32_t i = win0 + threadIdx.x; i < win1; i += 128) {
+            const uint64_t c = row[i];
+            if (c != kCandInvalid) {
+                const uint32_t j = atomicAdd(&s_cnt, 1u);
+                s_slot[j] = i;
+                s_pos[j] = static_cast<uint32_t>(c) - pos_first;
+            }
         }
-    }
-    __syncthreads();
-    const uint32_t cnt = s_cnt;
-    for (uint32_t i0 = warp * 32; i0 < cnt; i0 += 128) {
-        const bool live = i0 + lane < cnt;
-        const uint32_t i = live ? s_slot[i0 + lane] : 0u;
-        const uint32_t pos = live ? s_pos[i0 + lane] : 0u;
-        const uint32_t live_mask = __ballot_sync(0xffffffffu, live);
-        float acc = 0.f;
-        if (d % kRefChunk == 0) {
-            // Whole chunks only: a lane stages the same 8 rows in every chunk, so their addresses are
-            // formed once per pass, and the loads of the next chunk are in flight while the current
-            // one is accumulated from shared memory.
-            const int j = lane & 7;
-            const float4* src[8];
-            uint32_t okm = 0;
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const int r = it * 4 + (lane >> 3);
-                const uint32_t pr = __shfl_sync(0xffffffffu, pos, r);
-                src[it] = reinterpret_cast<const float4*>(xb + static_cast<int64_t>(pr) * d) + j;
-                okm |= ((live_mask >> r) & 1u) << it;   // rows of unused slots are neither fetched nor read
-            }
-            float4* dst = reinterpret_cast<float4*>(rows + (lane >> 3) * kRefPitch + 4 * j);
-            const float4* mine = reinterpret_cast<const float4*>(rows + lane * kRefPitch);
-            float4 v[8];
-#pragma unroll
-            for (int it = 0; it < 8; ++it)
-                if ((okm >> it) & 1u) v[it] = __ldg(src[it]);
-            for (int ch0 = 0; ch0 < d; ch0 += kRefChunk) {
-#pragma unroll
-                for (int it = 0; it < 8; ++it)
-                    if ((okm >> it) & 1u) dst[it * kRefPitch] = v[it];   // 4 rows further per step
-                __syncwarp();
-                if (ch0 + kRefChunk < d) {
-#pragma unroll
-                    for (int it = 0; it < 8; ++it)
-                        if ((okm >> it) & 1u) v[it] = __ldg(src[it] + (ch0 + kRefChunk) / 4);
-                }
-                const float4* qv = reinterpret_cast<const float4*>(qs + ch0);
-                if (live) {
-                    if (metric == kMetricL2) {
-#pragma unroll
-                        for (int jj = 0; jj < kRefChunk / 4; ++jj) {
-                            const float4 a = qv[jj], b = mine[jj];
-                            float t;
-                            t = a.x - b.x; acc = fmaf(t, t, acc);
-                            t = a.y - b.y; acc = fmaf(t, t, acc);
-                            t = a.z - b.z; acc = fmaf(t, t, acc);
-                            t = a.w - b.w; acc = fmaf(t, t, acc);
-                        }
-                    } else {
-#pragma unroll
-                        for (int jj = 0; jj < kRefChunk / 4; ++jj) {
-                            const float4 a = qv[jj], b = mine[jj];
-                            acc = fmaf(a.x, b.x, acc);
-                            acc = fmaf(a.y, b.y, acc);
-                            acc = fmaf(a.z, b.z, acc);
-                            acc = fmaf(a.w, b.w, acc);
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-        } else
-        for (int ch0 = 0; ch0 < d; ch0 += kRefChunk) {
-            const int w = d - ch0 < kRefChunk ? d - ch0 : kRefChunk;
-            const int lpr = w >> 2;                                  // float4 pieces per row
-            if (lpr == kRefChunk / 4) {
-#pragma unroll
-                for (int it = 0; it < 8; ++it) {                     // four of the 32 rows per load instruction
-                    const int r = it * 4 + (lane >> 3), j = lane & 7;
-                    const uint32_t pr = __shfl_sync(0xffffffffu, pos, r);
-                    if ((live_mask >> r) & 1u) {   // rows of unused slots are neither fetched nor read
-                        const float4 v = __ldg(reinterpret_cast<const float4*>(xb + static_cast<int64_t>(pr) * d + ch0) + j);
-                        *reinterpret_cast<float4*>(rows + r * kRefPitch + 4 * j) = v;
-                    }
-                }
-            } else {
-                for (int idx = lane; idx < 32 * lpr; idx += 32) {
-                    const int r = idx / lpr, j = idx - r * lpr;
-                    const uint32_t pr = __shfl_sync(0xffffffffu, pos, r);
-                    const float4 v = __ldg(reinterpret_cast<const float4*>(xb + static_cast<int64_t>(pr) * d + ch0) + j);
-                    *reinterpret_cast<float4*>(rows + r * kRefPitch + 4 * j) = v;
-                }
-            }
-            __syncwarp();
-            const float4* mine = reinterpret_cast<const float4*>(rows + lane * kRefPitch);
-            const float4* qv = reinterpret_cast<const float4*>(qs + ch0);
-            if (!live) {
-                // nothing to accumulate for an unused slot
-            } else if (metric == kMetricL2) {
-#pragma unroll 4
-                for (int j = 0; j < lpr; ++j) {
-                    const float4 a = qv[j], b = mine[j];
-                    float t;
-                    t = a.x - b.x; acc = fmaf(t, t, acc);
-                    t = a.y - b.y; acc = fmaf(t, t, acc);
-                    t = a.z - b.z; acc = fmaf(t, t, acc);
-                    t = a.w - b.w; acc = fmaf(t, t, acc);
-                }
-            } else {
-#pragma unroll 4
-                for (int j = 0; j < lpr; ++j) {
-                    const float4 a = qv[j], b = mine[j];
-                    acc = fmaf(a.x, b.x, acc);
-                    acc = fmaf(a.y, b.y, acc);
-                    acc = fmaf(a.z, b.z, acc);
-                    acc = fmaf(a.w, b.w, acc);
-                }
-            }
-            __syncwarp();
+        __syncthreads();
+        const uint32_t cnt = s_cnt;
+        for (uint32_t i0 = warp * 32; i0 < cnt; i0 += 128) {
+            const bool live = i0 + lane < cnt;
+            const uint32_t i = live ? s_slot[i0 + lane] : 0u;
+            const uint32_t pos = live ? s_pos[i0 + lane] : 0u;
+            const float key = refine_lane(xb, qs, rows, pos, live, d, metric, lane);
+            if (live) row[i] = pack_cand(float_to_ord(key), pos + pos_first);
         }
-        if (metric != kMetricL2) acc = -acc;
-        if (live) row[i] = pack_cand(float_to_ord(acc), pos + pos_first);
-    }
-    __syncthreads();   // the window's lists are reused
+        __syncthreads();   // the window's lists are reused
     }
 }
 
-__global__ void emit_kernel(const EmitArgs e) {
-    const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= static_cast<int64_t>(e.nq) * e.k) return;
-    const int q = static_cast<int>(idx / e.k), j = static_cast<int>(idx % e.k);
-    const int orow = e.qmap ? e.qmap[q] : q;
-    const int qn = e.q_mod > 0 ? q % e.q_mod : q;   // row of the query norms
-    const uint64_t c = e.sel[idx];
-    float dist;
-    int64_t label;
-    if (c == kCandInvalid) {
-        dist = 3.402823466e+38f;  // FLT_MAX padding, label -1
-        label = -1;
-    } else {
-        const uint32_t ok = static_cast<uint32_t>(c >> 32), pos = static_cast<uint32_t>(c);
-        if (e.members) {
-            const MemberView& mv = e.members[q / e.q_mod];
-            label = mv.labels[static_cast<int64_t>(pos) - mv.first];
-        } else {
-            label = e.labels ? e.labels[pos] : static_cast<int64_t>(pos);
+// ---- short candidate lists of fp32 indexes: pruning, exact distances, order and results in one block ----
+// What prune_candidates_kernel, refine_f32_kernel and select_emit_kernel do one after the other, for lists
+// of at most `stage` candidates of which at most kFinKeep survive the pruning; the row is read once, survivors
+// and exact keys stay in shared memory.  Others are left alone and marked 2 in `status` (1: the row
+// overflowed, as in select_emit_kernel): the caller runs the three kernels for them.
+// One query against 100 003 x 128, k = 10: 38 us in four launches -> 10; 10 000
+// queries against 16 384 centroids, k = 64: 117 -> 110.
+constexpr int kFinThreads = 128;
+constexpr uint32_t kFinKeep = 1024;
+constexpr uint32_t kFinStage = 4096;
+__global__ void __launch_bounds__(kFinThreads, 6)
+finish_f32_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t cap, uint32_t stage, int d, const float* eps,
+                  const float* xq, const float* xb, uint8_t* status, uint32_t* any_status, const EmitArgs e) {
+    extern __shared__ __align__(16) uint64_t fin_sm[];
+    uint64_t* keep = fin_sm;                                             // [kFinKeep]
+    float* qs = reinterpret_cast<float*>(fin_sm + kFinKeep);             // [d]
+    float* rows = qs + d;                                                // 4 x [32][kRefPitch], after ...
+    uint64_t* held = reinterpret_cast<uint64_t*>(rows);                  // ... [stage] entries have been pruned
+    __shared__ RankScratch rank;
+    __shared__ uint32_t sh_fill;
+    const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int qrow = e.q_mod > 0 ? q % e.q_mod : q;
+    const uint32_t n = counts[q], k = static_cast<uint32_t>(e.k);
+    auto leave = [&](uint8_t why) {
+        if (threadIdx.x == 0) {
+            if (status) status[q] = why;
+            if (any_status) atomicOr(any_status, 1u);
         }
-        if (e.mode == 2) {
-            int32_t kv = ord_to_int(ok);
-            if (e.metric == kMetricL2) dist = static_cast<float>(kv + static_cast<const int32_t*>(e.qnorm)[qn]);
-            else if (e.metric == kMetricCos) dist = cos16_value(-kv);
-            else dist = static_cast<float>(-kv);
-        } else {
-            float kv = ord_to_float(ok);
-            if (e.metric == kMetricL2) {
-                if (e.mode == 0) {
-                    kv += static_cast<const float*>(e.qnorm)[qn];
-                    kv = kv < 0.f ? 0.f : kv;
-                }
-                dist = kv;
-            } else {
-                dist = -kv;
-            }
-        }
+    };
+    if (n > cap) {
+        leave(1);
+        return;
     }
-    e.D[static_cast<int64_t>(orow) * e.ldk + j] = dist;
-    e.I[static_cast<int64_t>(orow) * e.ldk + j] = label;
+    uint32_t pos_first = 0;
+    if (e.members) {
+        const MemberView& mv = e.members[q / e.q_mod];
+        xb = mv.rows_f32;
+        pos_first = static_cast<uint32_t>(mv.first);
+    }
+    for (int i = threadIdx.x; i < d / 4; i += kFinThreads)
+        reinterpret_cast<float4*>(qs)[i] = __ldg(reinterpret_cast<const float4*>(xq + static_cast<int64_t>(qrow) * d) + i);
+    uint32_t m = block_compact<kFinThreads>(cand + static_cast<int64_t>(q) * cap, n, held, stage, &sh_fill);
+    if (m > stage) {
+        leave(2);
+        return;
+    }
+    uint32_t lim = 0xFFFFFFFFu;
+    if (m > 2 * k || m > kFinKeep) {   // fewer are refined as they are
+        const uint32_t kth = block_kth32<kFinThreads>(
+            [&](auto&& f) {
+                for (uint32_t i = threadIdx.x; i < m; i += kFinThreads) {
+                    const uint32_t v = static_cast<uint32_t>(held[i] >> 32);
+                    if (v != 0xFFFFFFFFu) f(v);
+                }
+            },
+            k, rank, 2);
+        if (!prune_limit(kth, eps[qrow], &lim)) lim = 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) sh_fill = 0u;
+    __syncthreads();
+    for (uint32_t i0 = warp * 32; i0 < m; i0 += kFinThreads) {
+        const uint64_t v = i0 + lane < m ? held[i0 + lane] : kCandInvalid;
+        const bool in = i0 + lane < m && static_cast<uint32_t>(v >> 32) <= lim;
+        const unsigned bal = __ballot_sync(0xffffffffu, in);
+        if (!bal) continue;
+        uint32_t slot = 0;
+        if (lane == 0) slot = atomicAdd(&sh_fill, static_cast<uint32_t>(__popc(bal)));
+        slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(bal & ((1u << lane) - 1u));
+        if (in && slot < kFinKeep) keep[slot] = v;
+    }
+    __syncthreads();
+    m = sh_fill;
+    if (m > kFinKeep) {
+        leave(2);
+        return;
+    }
+    if (status && threadIdx.x == 0) status[q] = 0;
+    for (uint32_t i0 = warp * 32; i0 < m; i0 += kFinThreads) {
+        const bool live = i0 + lane < m;
+        const uint32_t pos = live ? static_cast<uint32_t>(keep[i0 + lane]) - pos_first : 0u;
+        const float key = refine_lane(xb, qs, rows + warp * (32 * kRefPitch), pos, live, d, e.metric, lane);
+        if (live) keep[i0 + lane] = pack_cand(float_to_ord(key), pos + pos_first);
+    }
+    __syncthreads();
+    if (m <= static_cast<uint32_t>(kSmallSet)) {
+        for (uint32_t i = threadIdx.x; i < m; i += kFinThreads) {
+            const uint64_t v = keep[i];
+            uint32_t r = 0;
+#pragma unroll 8
+            for (uint32_t j = 0; j < m; ++j) r += keep[j] < v ? 1u : 0u;
+            if (r < k) emit_one(e, q, static_cast<int>(r), v);
+        }
+    } else {
+        int P = kSmallSet;
+        while (P < static_cast<int>(m)) P <<= 1;
+        for (int i = static_cast<int>(m) + threadIdx.x; i < P; i += kFinThreads) keep[i] = kCandInvalid;
+        __syncthreads();
+        bitonic_sort_u64<kFinThreads>(keep, P);
+        for (uint32_t i = threadIdx.x; i < min(k, m); i += kFinThreads) emit_one(e, q, static_cast<int>(i), keep[i]);
+    }
+    for (uint32_t i = m + threadIdx.x; i < k; i += kFinThreads) emit_one(e, q, static_cast<int>(i), kCandInvalid);
 }
 
 // One warp per query; heads[] in shared memory.
@@ -758,26 +1032,45 @@ inline int next_pow2(int v) {
 cudaError_t launch_kth_threshold(const uint32_t* mins, int stride, int n, int nq, int k, const float* eps,
                                  uint32_t tau_all, uint32_t* tau, const TauFold& fold, cudaStream_t stream) {
     if (nq <= 0) return cudaSuccess;
-    if (n <= 512)
+    if (n <= 32)
+        kth_threshold_warp_kernel<1><<<(nq + 3) / 4, 128, 0, stream>>>(mins, stride, n, nq, k, eps, tau_all, tau, fold);
+    else if (n <= 128)
+        kth_threshold_warp_kernel<4><<<(nq + 3) / 4, 128, 0, stream>>>(mins, stride, n, nq, k, eps, tau_all, tau, fold);
+    else if (n <= 512)
         kth_threshold_warp_kernel<16><<<(nq + 3) / 4, 128, 0, stream>>>(mins, stride, n, nq, k, eps, tau_all, tau, fold);
     else if (n <= 1024)
         kth_threshold_warp_kernel<32><<<(nq + 3) / 4, 128, 0, stream>>>(mins, stride, n, nq, k, eps, tau_all, tau, fold);
     else
-        kth_threshold_kernel<<<nq, kSelThreads, 0, stream>>>(mins, stride, n, k, eps, tau_all, tau, fold);
+        kth_threshold_kernel<<<nq, kSelThreads, n <= static_cast<int>(kKthStage) ? n * 4 : 0, stream>>>(mins, stride, n, k, eps, tau_all, tau, fold);
     return cudaGetLastError();
 }
 
-cudaError_t launch_select_topk(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int nq,
-                               int k, uint64_t* out, uint8_t* overflow, cudaStream_t stream, uint32_t* any_overflow) {
-    if (nq <= 0) return cudaSuccess;
-    int P = next_pow2(k < 32 ? 32 : k);
-    size_t smem = static_cast<size_t>(P) * sizeof(uint64_t);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(select_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
-    select_topk_kernel<<<nq, kSelThreads, smem, stream>>>(cand, counts, n_fixed, cap, k, P, out, overflow, any_overflow);
+cudaError_t launch_select_emit(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap,
+                               uint8_t* overflow, uint32_t* any_overflow, const EmitArgs& e, cudaStream_t stream) {
+    if (e.nq <= 0 || e.k <= 0) return cudaSuccess;
+    const int P = next_pow2(e.k < 32 ? 32 : e.k);
+    // Room for about as many candidates as a threshold for that k lets through (two stretches: 7 - 8 k).
+    // Blocks of 512 where two of them fill an SM's shared memory.
+    const bool large = e.k > 128;
+    const uint32_t stage = large ? 12288u : 2048u;
+    const size_t smem = (static_cast<size_t>(P) + stage) * sizeof(uint64_t);
+    auto kern = large ? select_emit_kernel<512> : select_emit_kernel<kSelThreads>;
+    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (err != cudaSuccess) return err;
+    kern<<<e.nq, large ? 512 : kSelThreads, smem, stream>>>(cand, counts, n_fixed, cap, P, stage, overflow, any_overflow, e);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_finish_f32(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int d, const float* eps,
+                              const float* xq, const float* xb, uint8_t* status, uint32_t* any_status, const EmitArgs& e,
+                              cudaStream_t stream) {
+    if (e.nq <= 0 || e.k <= 0) return cudaSuccess;
+    const uint32_t stage = cap < kFinStage ? cap : kFinStage;
+    const size_t rows = 4 * 32 * kRefPitch * sizeof(float), held = stage * sizeof(uint64_t);
+    const size_t smem = kFinKeep * sizeof(uint64_t) + static_cast<size_t>(d) * 4 + (rows > held ? rows : held);
+    cudaError_t err = cudaFuncSetAttribute(finish_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (err != cudaSuccess) return err;
+    finish_f32_kernel<<<e.nq, kFinThreads, smem, stream>>>(cand, counts, cap, stage, d, eps, xq, xb, status, any_status, e);
     return cudaGetLastError();
 }
 
@@ -819,13 +1112,6 @@ cudaError_t launch_refine_f32(uint64_t* cand, const uint32_t* counts, uint32_t n
                                                             counts ? counts + q0 : nullptr, n_fixed, cap, d, metric,
                                                             xq, xb, q0, q_mod, members);
     }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_emit(const EmitArgs& e, cudaStream_t stream) {
-    const int64_t total = static_cast<int64_t>(e.nq) * e.k;
-    if (total <= 0) return cudaSuccess;
-    emit_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(e);
     return cudaGetLastError();
 }
 

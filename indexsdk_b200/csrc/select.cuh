@@ -35,15 +35,6 @@ struct TauFold {
 cudaError_t launch_kth_threshold(const uint32_t* mins, int stride, int n, int nq, int k, const float* eps,
                                  uint32_t tau_all, uint32_t* tau, const TauFold& fold, cudaStream_t stream);
 
-// Per query: the k smallest of cand[q][0..min(counts[q],cap)) in ascending order into
-// out[q][0..k), padded with kCandInvalid.  counts == nullptr means every row holds n_fixed
-// candidates.  overflow[q] is set to 1 when counts[q] > cap (the row's result is then not
-// trustworthy and the caller re-runs it without a threshold); *any_overflow is set to 1 when that
-// happens to any row.
-cudaError_t launch_select_topk(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int nq,
-                               int k, uint64_t* out, uint8_t* overflow, cudaStream_t stream,
-                               uint32_t* any_overflow = nullptr);
-
 // fp32 refinement: replaces the key of every candidate by the canonical fp32 distance
 // (sequential fmaf over the dimension) computed from the fp32 rows; L2 -> distance,
 // IP -> negated dot product.
@@ -63,7 +54,6 @@ cudaError_t launch_refine_f32(uint64_t* cand, const uint32_t* counts, uint32_t n
                               const MemberView* members = nullptr);
 
 struct EmitArgs {
-    const uint64_t* sel;     // [nq][k] sorted candidates
     int nq, k;
     int metric;
     int mode;                // 0: float key without query norm (add qnorm for L2); 1: refined float key; 2: int key
@@ -76,7 +66,19 @@ struct EmitArgs {
     int q_mod;               // > 0: row q uses the query norm of row q % q_mod (multi-index search)
     const MemberView* members;   // with q_mod: row q's labels are those of member q / q_mod (device array, or nullptr)
 };
-cudaError_t launch_emit(const EmitArgs& e, cudaStream_t stream);
+// Per query: the k smallest of cand[q][0..min(counts[q],cap)) in ascending order as results (FLT_MAX / -1
+// where there are fewer).  counts == nullptr means every row holds n_fixed candidates.  overflow[q] is
+// set to 1 when counts[q] > cap (the row's result is then not trustworthy and the caller re-runs it
+// without a threshold); *any_overflow is set to 1 when that happens to any row.
+cudaError_t launch_select_emit(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap,
+                               uint8_t* overflow, uint32_t* any_overflow, const EmitArgs& e, cudaStream_t stream);
+// fp32 indexes: pruning, exact distances, selection and results of short candidate lists in one launch.
+// status[q] = 0 done, 1 row overflowed, 2 list too long for it (prune, refine and select it instead; the row
+// is unchanged); *any_status is set to 1 when any row is left.  k <= kFinishMaxK.
+constexpr int kFinishMaxK = 256;
+cudaError_t launch_finish_f32(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int d, const float* eps,
+                              const float* xq, const float* xb, uint8_t* status, uint32_t* any_status, const EmitArgs& e,
+                              cudaStream_t stream);
 
 // Merge nsrc sorted lists per query.  Din/Iin: [nsrc][nq][k]; order by (distance ascending or
 // score descending, label ascending); label < 0 marks padding.  src_stride_d / src_stride_i: elements

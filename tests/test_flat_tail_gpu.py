@@ -1,0 +1,74 @@
+"""From candidates to results of the exact indexes: the fused tail of fp32 lists (block and warp form),
+its hand-over of lists that are too long, and the selection of long lists, at the edges of each."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import assert_exact
+from indexsdk_b200 import datasets
+
+pytestmark = pytest.mark.gpu
+L2, IP = 1, 0
+
+
+def _flat(b200, metric, xb, xq, k):
+    ix = b200.IndexFlat(xb.shape[1], metric)
+    ix.add(xb)
+    D, I = ix.search(xq, k)
+    Dr, Ir = oracle.flat_search(metric, xb, xq, k)
+    assert_exact(D, I, Dr, Ir)
+    return ix
+
+
+# one-tile bases searched by many queries (a threshold over the whole base, the warp form up to k = 32), k on
+# both sides of what a form takes, rows of 16 and of 32-float chunks
+@pytest.mark.parametrize("metric", [L2, IP])
+@pytest.mark.parametrize("n,d,nq,k", [(256, 64, 5000, 1), (40, 48, 20000, 2), (300, 128, 9000, 8), (2100, 64, 3000, 32),
+                                      (2100, 80, 1500, 33), (5000, 64, 700, 100), (40000, 64, 40, 256), (40000, 64, 40, 257),
+                                      (120000, 32, 3, 1000)])
+def test_forms_of_the_tail(b200, metric, n, d, nq, k):
+    _flat(b200, metric, datasets.gaussian(n, d, seed=1), datasets.gaussian(nq, d, seed=2), k)
+
+
+@pytest.mark.parametrize("n,copies,k", [(200000, 1500, 10), (200000, 6000, 10), (9000, 1200, 5)])
+def test_near_duplicates_outgrow_the_fused_tail(b200, n, copies, k):
+    """`copies` rows closer together than the bf16 filter can tell apart: all survive the pruning."""
+    xb = datasets.gaussian(n, 64, seed=1)
+    near = xb[:1] + np.float32(1e-4) * datasets.gaussian(copies, 64, seed=3)
+    xb[n - copies:] = near
+    _flat(b200, L2, xb, np.concatenate([near[:2], datasets.gaussian(2, 64, seed=4)]), k)
+
+
+@pytest.mark.parametrize("k", [1, 10, 129, 1024])
+def test_ties_at_the_last_rank_go_to_the_lowest_positions(b200, k):
+    """int8 rows of few distinct distances: thousands tie with the k-th key."""
+    rng = np.random.default_rng(5)
+    xb = rng.integers(-1, 2, size=(30000, 16)).astype(np.int8)
+    xq = rng.integers(-1, 2, size=(9, 16)).astype(np.int8)
+    for metric in (L2, IP):
+        ix = b200.IndexInt8Flat(16, metric)
+        ix.add(xb)
+        D, I = ix.search(xq, k)
+        Dr, Ir = oracle.int8_search(metric, xb, xq, k)
+        assert_exact(D, I, Dr, Ir)
+
+
+@pytest.mark.parametrize("keep", [0, 3, 40])
+def test_filter_that_leaves_fewer_rows_than_k(b200, keep):
+    """Fewer rows than k pass the filter of an int8 index large enough for a sampled threshold."""
+    n, k = 150000, 10
+    xb, xq = datasets.uniform_int8(n, 32, seed=1), datasets.uniform_int8(2, 32, seed=2)
+    bits = np.zeros((2, n), bool)
+    for q in range(2):
+        bits[q, np.random.default_rng(q).permutation(n)[:keep]] = True
+    for metric in (L2, IP):
+        ix = b200.IndexInt8Flat(32, metric)
+        ix.add(xb)
+        D, I = ix.search_with_masks(xq, k, np.packbits(bits, axis=1, bitorder="little"))
+        for q in range(2):
+            rows = np.flatnonzero(bits[q])
+            got = min(keep, k)
+            assert (I[q, got:] == -1).all()
+            if keep:
+                Dr, Ir = oracle.int8_search(metric, xb[rows], xq[q:q + 1], got, labels=rows)
+                assert_exact(D[q:q + 1, :got], I[q:q + 1, :got], Dr, Ir)
