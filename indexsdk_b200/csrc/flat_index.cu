@@ -226,7 +226,7 @@ FlatIndex::Plan FlatIndex::make_plan(int k, int64_t nq) const {
     const int64_t n_tiles = (n_ + kTileB - 1) / kTileB;
     const int64_t need = std::max<int64_t>(4LL * k, 1024);
     p.sampled = false;
-    if (n_tiles <= 256 && n_tiles >= 8) {
+    if (n_tiles <= 256) {
         // Small base (e.g. an IVF coarse quantizer): the "sample" is the whole base, so the k-th
         // smallest burst minimum is a certain upper bound of the k-th smallest key and admits
         // little more than k candidates as long as bursts are plentiful against k (with k / bursts
@@ -258,14 +258,19 @@ FlatIndex::Plan FlatIndex::make_plan(int k, int64_t nq) const {
         const double inv_f = static_cast<double>(n_tiles) / p.s_tiles;
         uint64_t want = static_cast<uint64_t>(4.0 * k * inv_f);
         // The append epilogue reserves slots in blocks of 8 per (thread, run of tiles of one query
-        // block); a row is shared by up to four threads in each of the CTAs that walk its query block, and
-        // every one of them may leave a block partly unused.
+        // block); a row is shared by four threads in each of the CTAs that walk its query block, and
+        // every one of them may leave an open block and one reserved ahead partly unused, in each
+        // stretch of the pass (a threshold from the whole base needs one stretch).
+        const bool whole = p.s_tiles == n_tiles;
         const int64_t n_qb = (std::max<int64_t>(nq, 1) + kTileQ - 1) / kTileQ;
-        // (four threads per row in the 16-warp epilogue of the bf16 kind)
-        const uint64_t owners = 4 * static_cast<uint64_t>((num_sms_ + n_qb - 1) / n_qb + 1);
-        want += owners * 32;   // an open block and one reserved ahead, in each of the two stretches of the pass
-        p.cap = pow2_ceil(std::max<uint64_t>(p.s_tiles == n_tiles ? 512 : 2048, want));
-        if (p.cap >= static_cast<uint64_t>(n_pad)) p.sampled = false;
+        const uint64_t ctas = static_cast<uint64_t>(std::min<int64_t>((num_sms_ + n_qb - 1) / n_qb + 1, n_tiles));
+        want += 4 * ctas * (whole ? 16 : 32);
+        p.cap = pow2_ceil(std::max<uint64_t>(whole ? 256 : 2048, want));
+        // Candidate rows as long as the base itself save nothing in memory; they pay all the same once
+        // there are many keys that would otherwise be refined and selected from one by one (300 000 queries
+        // against 256 rows of d 128, k = 1: 8.6 -> 0.8 ms; the second GEMM pass and the threshold cost a
+        // small call about 10 us, as much as 0.5 M keys do).
+        if (p.cap >= static_cast<uint64_t>(n_pad) && !(whole && nq * n_pad >= (int64_t(1) << 19))) p.sampled = false;
     }
     if (!p.sampled) {
         p.burst = 32;
@@ -456,7 +461,7 @@ void FlatIndex::run_tail(const PageTail& t, bool fused) {
     const uint32_t n_fixed = static_cast<uint32_t>(n_);
     if (fused) {
         timer_.begin(kStageRefine, stream_);
-        B200_CUDA_CHECK(launch_finish_f32(cand, counts, t.cap, d_, eps, t.xq, x32_.as<float>(), over, nullptr, t.e, stream_));
+        B200_CUDA_CHECK(launch_finish_f32(cand, counts, t.cap, d_, eps, t.xq, x32_.as<float>(), over, nullptr, t.e, !t.prune && t.nq >= 4 * num_sms_, stream_));
         timer_.end(stream_);
         stats_.kernel_launches += 1;
         return;

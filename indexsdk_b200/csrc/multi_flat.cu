@@ -284,7 +284,7 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
         launches_ += 2;
         if (with_tau && dtype_ == kF32 && k <= kFinishMaxK) {
             B200_CUDA_CHECK(launch_finish_f32(cand, counts, cap, d_, w_eps_.as<float>(), static_cast<const float*>(xq), nullptr,
-                                              nullptr, any_left, e, st));
+                                              nullptr, any_left, e, false, st));
             continue;
         }
         const uint32_t* n_cand = with_tau ? counts : nullptr;

@@ -74,11 +74,12 @@ cudaError_t launch_select_emit(const uint64_t* cand, const uint32_t* counts, uin
                                uint8_t* overflow, uint32_t* any_overflow, const EmitArgs& e, cudaStream_t stream);
 // fp32 indexes: pruning, exact distances, selection and results of short candidate lists in one launch.
 // status[q] = 0 done, 1 row overflowed, 2 list too long for it (prune, refine and select it instead; the row
-// is unchanged); *any_status is set to 1 when any row is left.  k <= kFinishMaxK.
+// is unchanged); *any_status is set to 1 when any row is left.  k <= kFinishMaxK.  few: lists of little
+// more than k candidates are expected (a threshold over the whole base), no need to prune them first.
 constexpr int kFinishMaxK = 256;
 cudaError_t launch_finish_f32(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int d, const float* eps,
                               const float* xq, const float* xb, uint8_t* status, uint32_t* any_status, const EmitArgs& e,
-                              cudaStream_t stream);
+                              bool few, cudaStream_t stream);
 
 // Merge nsrc sorted lists per query.  Din/Iin: [nsrc][nq][k]; order by (distance ascending or
 // score descending, label ascending); label < 0 marks padding.  src_stride_d / src_stride_i: elements
