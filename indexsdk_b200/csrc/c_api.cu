@@ -112,6 +112,7 @@ void check_search_args(const b200idx_index* h, int64_t n, const void* x, int k, 
 struct MultiScratch {
     std::mutex mu;           // held for a whole multi-index search that uses this device
     DeviceBuffer q, D, I, allD, allI, mD, mI, gD, gI;
+    PinnedBuffer hq, hD, hI;
     std::unique_ptr<FlatGroup> group;   // concatenated copy of the small Flat indexes searched together last
 };
 MultiScratch& multi_scratch(int device) {
@@ -294,6 +295,14 @@ int b200idx_search_multi(b200idx_t* const* hs, int nh, int64_t n, const void* x,
             allD = static_cast<float*>(s0.allD.ensure(per * nh * 4));
             allI = static_cast<int64_t*>(s0.allI.ensure(per * nh * 8));
         }
+        std::unique_ptr<HostResults> merged_res;
+        if (merged) {
+            DeviceGuard g(dev0);
+            merged_res.reset(new HostResults(s0.hI, s0.hD, s0.mI, s0.mD, static_cast<int64_t>(per)));
+        }
+        HostResults* merged_out = merged_res.get();
+        bool merge_done = false;
+        bool* merge_queued = &merge_done;
         std::vector<std::string> errors(groups.size());
         std::vector<std::thread> workers;
         size_t gi = 0;
@@ -309,8 +318,7 @@ int b200idx_search_multi(b200idx_t* const* hs, int nh, int64_t n, const void* x,
                     float* dD = static_cast<float*>(sc.D.ensure(per * 4));
                     int64_t* dI = static_cast<int64_t*>(sc.I.ensure(per * 8));
                     cudaStream_t st = static_cast<cudaStream_t>(b200idx_stream(hs[members[0]]));
-                    B200_CUDA_CHECK(cudaMemcpyAsync(dq, x, static_cast<size_t>(n) * row, cudaMemcpyHostToDevice, st));
-                    B200_CUDA_CHECK(cudaStreamSynchronize(st));
+                    upload_small(dq, x, static_cast<size_t>(n) * row, sc.hq, st);
                     // Small exact indexes of one device are searched in ONE pass over their
                     // concatenated bases (segmented search): launches do not grow with their number.
                     std::vector<FlatIndex*> fm;
@@ -328,7 +336,15 @@ int b200idx_search_multi(b200idx_t* const* hs, int nh, int64_t n, const void* x,
                         const bool direct = merged && dev == dev0 && contiguous;
                         float* gD = direct ? allD + per * members[0] : static_cast<float*>(sc.gD.ensure(per * m * 4));
                         int64_t* gI = direct ? allI + per * members[0] : static_cast<int64_t*>(sc.gI.ensure(per * m * 8));
-                        sc.group->search_device(fm, n, dq, k, gD, gI, st);
+                        // all members here and merged: the merge is queued behind the search
+                        std::function<void()> then;
+                        if (direct && static_cast<int>(m) == nh) {
+                            then = [&]() {
+                                B200_CUDA_CHECK(launch_merge_topk(nh, n, k, descending_of(h0) ? 1 : 0, allD, allI, merged_out->D, merged_out->I, st));
+                            };
+                            *merge_queued = true;
+                        }
+                        sc.group->search_device(fm, n, dq, k, gD, gI, st, then);
                         if (!direct) {
                             const cudaMemcpyKind kind = merged ? cudaMemcpyDefault : cudaMemcpyDeviceToHost;
                             float* dstD = merged ? allD : D;
@@ -346,6 +362,7 @@ int b200idx_search_multi(b200idx_t* const* hs, int nh, int64_t n, const void* x,
                         }
                         return;
                     }
+                    B200_CUDA_CHECK(cudaStreamSynchronize(st));   // the members search on streams of their own
                     for (int i : members) {
                         b200idx_index* h = hs[i];
                         // with merged results on this device the member writes its slice directly
@@ -377,12 +394,11 @@ int b200idx_search_multi(b200idx_t* const* hs, int nh, int64_t n, const void* x,
         if (merged) {
             DeviceGuard g(dev0);
             cudaStream_t st = static_cast<cudaStream_t>(b200idx_stream(h0));
-            float* mD = static_cast<float*>(s0.mD.ensure(per * 4));
-            int64_t* mI = static_cast<int64_t*>(s0.mI.ensure(per * 8));
-            B200_CUDA_CHECK(launch_merge_topk(nh, n, k, descending_of(h0) ? 1 : 0, allD, allI, mD, mI, st));
-            B200_CUDA_CHECK(cudaMemcpyAsync(D, mD, per * 4, cudaMemcpyDeviceToHost, st));
-            B200_CUDA_CHECK(cudaMemcpyAsync(I, mI, per * 8, cudaMemcpyDeviceToHost, st));
-            B200_CUDA_CHECK(cudaStreamSynchronize(st));
+            if (!merge_done) {
+                B200_CUDA_CHECK(launch_merge_topk(nh, n, k, descending_of(h0) ? 1 : 0, allD, allI, merged_out->D, merged_out->I, st));
+                B200_CUDA_CHECK(cudaStreamSynchronize(st));
+            }
+            merged_out->deliver(D, I, st);
         }
     }, /*lock=*/false);
 }

@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
+#include <cstring>
 #include <stdint.h>
 
 #include "common.cuh"
@@ -102,5 +103,45 @@ struct DeviceGuard {
     }
     int prev_ = 0, dev_ = 0;
 };
+
+// Results of a search on their way to the caller's host arrays.  Up to kDirectResults of them are written by
+// the kernels straight into pinned memory and are there when the stream is idle: no copies (two blocking
+// ones and the gaps around them cost about 30 us a call), one memcpy.  More go through device memory.
+struct HostResults {
+    static constexpr int64_t kDirectResults = 32768;
+    float* D;
+    int64_t* I;
+    HostResults(PinnedBuffer& hI, PinnedBuffer& hD, DeviceBuffer& dI, DeviceBuffer& dD, int64_t count)
+        : count_(count), direct_(count <= kDirectResults) {
+        I = static_cast<int64_t*>(direct_ ? hI.ensure(static_cast<size_t>(count) * 8) : dI.ensure(static_cast<size_t>(count) * 8));
+        D = static_cast<float*>(direct_ ? hD.ensure(static_cast<size_t>(count) * 4) : dD.ensure(static_cast<size_t>(count) * 4));
+    }
+    // Call with everything that writes the results complete (direct: synchronised) or queued on st.
+    void deliver(float* outD, int64_t* outI, cudaStream_t st) const {
+        if (direct_) {
+            std::memcpy(outD, D, static_cast<size_t>(count_) * 4);
+            std::memcpy(outI, I, static_cast<size_t>(count_) * 8);
+            return;
+        }
+        B200_CUDA_CHECK(cudaMemcpyAsync(outD, D, static_cast<size_t>(count_) * 4, cudaMemcpyDeviceToHost, st));
+        B200_CUDA_CHECK(cudaMemcpyAsync(outI, I, static_cast<size_t>(count_) * 8, cudaMemcpyDeviceToHost, st));
+        B200_CUDA_CHECK(cudaStreamSynchronize(st));
+    }
+
+private:
+    int64_t count_;
+    bool direct_;
+};
+
+// Host -> device copy; a small one goes through pinned memory, which lets the call return at once.  The
+// stream has to be idle when the same staging buffer is used again.
+inline void upload_small(void* dst, const void* src, size_t bytes, PinnedBuffer& stage, cudaStream_t st) {
+    if (bytes <= (size_t(256) << 10)) {
+        void* h = stage.ensure(bytes);
+        std::memcpy(h, src, bytes);
+        src = h;
+    }
+    B200_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+}
 
 }  // namespace b200

@@ -448,16 +448,22 @@ FlatIndex::PageTail FlatIndex::run_page(int nq, const void* xq_raw, const void* 
     t.e.I = I;
     t.e.ldk = ldk;
     t.e.qmap = qmap_dev;
+    // statuses and the error word: pinned memory that the last kernels write to, and only when there is
+    // something to say (a copy and its launch cost 6 us each)
+    t.status = static_cast<uint8_t*>(h_over_.ensure(static_cast<size_t>(nq) + sizeof(int) + 8));
+    t.e.err = w_err_.as<int>();
+    t.e.err_host = reinterpret_cast<int*>(t.status + round_up(nq, 4));
     return t;
 }
 
 // From the candidates to the results.  fused: fp32 lists that are short enough in one launch; the others
-// come back with status 2 in w_over_ and need a second call without it.
+// come back with status 2 and need a second call without it.
 void FlatIndex::run_tail(const PageTail& t, bool fused) {
     uint64_t* cand = w_cand_.as<uint64_t>();
     uint32_t* counts = t.sampled ? w_counts_.as<uint32_t>() : nullptr;
     const float* eps = w_eps_.as<float>();
-    uint8_t* over = static_cast<uint8_t*>(w_over_.ensure(static_cast<size_t>(t.nq)));
+    uint8_t* over = t.status;
+    std::memset(over, 0, static_cast<size_t>(round_up(t.nq, 4)) + sizeof(int));
     const uint32_t n_fixed = static_cast<uint32_t>(n_);
     if (fused) {
         timer_.begin(kStageRefine, stream_);
@@ -479,10 +485,46 @@ void FlatIndex::run_tail(const PageTail& t, bool fused) {
         timer_.end(stream_);
     }
     timer_.begin(kStageSelect, stream_);
-    if (!t.sampled) B200_CUDA_CHECK(cudaMemsetAsync(over, 0, static_cast<size_t>(t.nq), stream_));
     B200_CUDA_CHECK(launch_select_emit(cand, counts, n_fixed, t.cap, t.sampled ? over : nullptr, nullptr, t.e, stream_));
     stats_.kernel_launches += 1;
     timer_.end(stream_);
+}
+
+// Queues a search of fp32 queries on the stream without waiting for it, where one page holds it; the
+// results are there, or padding, when the stream has got that far.  Once it has, queued_ok() says whether
+// they stand (false: search_device has to do it again).
+bool FlatIndex::queue_search(int64_t nq, const float* xq, int k, float* D, int64_t* I, int ldk) {
+    if (nq <= 0 || n_ == 0 || dtype_ != kF32) return false;
+    const Plan plan = make_plan(k, nq);
+    if (nq > page_rows(plan.cap)) return false;
+    stats_.searches += 1;
+    stats_.queries += static_cast<uint64_t>(nq);
+    mask_cur_ = nullptr;
+    queued_ = run_page(static_cast<int>(nq), xq, xq, k, D, I, ldk, nullptr, false);
+    run_tail(queued_, queued_.sampled && k <= kFinishMaxK);
+    return true;
+}
+
+bool FlatIndex::queued_ok() {
+    timer_.collect(stats_);
+    throw_on_error(queued_);
+    for (int i = 0; i < queued_.nq; ++i)
+        if (queued_.status[i]) return false;
+    return true;
+}
+
+int64_t FlatIndex::page_rows(uint32_t cap) const {
+    int64_t page = static_cast<int64_t>(kCandBudgetBytes / (static_cast<size_t>(cap) * 8));
+    if (page >= kTileQ) page = page / kTileQ * kTileQ;
+    return std::max<int64_t>(page, 1);
+}
+
+// (the stream is idle)
+void FlatIndex::throw_on_error(const PageTail& t) {
+    const int err = *t.e.err_host;
+    if (!err) return;
+    cudaMemsetAsync(w_err_.get(), 0, sizeof(int), stream_);
+    throw std::runtime_error("device pipeline reported error word " + std::to_string(err) + " (bounded wait ran out)");
 }
 
 void FlatIndex::search_device(int64_t nq, const void* xq, bool q_is_f16, int k, float* D, int64_t* I, int ldk) {
@@ -495,8 +537,8 @@ void FlatIndex::search_device(int64_t nq, const void* xq, bool q_is_f16, int k, 
         std::vector<float> dpad(static_cast<size_t>(k), 3.402823466e+38f);
         std::vector<int64_t> ipad(static_cast<size_t>(k), -1);
         for (int64_t q = 0; q < nq; ++q) {
-            B200_CUDA_CHECK(cudaMemcpyAsync(D + q * ldk, dpad.data(), k * 4, cudaMemcpyHostToDevice, stream_));
-            B200_CUDA_CHECK(cudaMemcpyAsync(I + q * ldk, ipad.data(), k * 8, cudaMemcpyHostToDevice, stream_));
+            B200_CUDA_CHECK(cudaMemcpyAsync(D + q * ldk, dpad.data(), k * 4, cudaMemcpyDefault, stream_));
+            B200_CUDA_CHECK(cudaMemcpyAsync(I + q * ldk, ipad.data(), k * 8, cudaMemcpyDefault, stream_));
         }
         B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
         return;
@@ -512,9 +554,7 @@ void FlatIndex::search_device(int64_t nq, const void* xq, bool q_is_f16, int k, 
     const size_t in_row = static_cast<size_t>(d_) * in_elem_bytes();
 
     const Plan plan = make_plan(k, nq);
-    int64_t page = static_cast<int64_t>(kCandBudgetBytes / (static_cast<size_t>(plan.cap) * 8));
-    if (page >= kTileQ) page = page / kTileQ * kTileQ;
-    if (page < 1) page = 1;
+    const int64_t page = page_rows(plan.cap);
     std::vector<int32_t> over_idx;
     for (int64_t q0 = 0; q0 < nq; q0 += page) {
         const int nqp = static_cast<int>(std::min<int64_t>(page, nq - q0));
@@ -523,16 +563,10 @@ void FlatIndex::search_device(int64_t nq, const void* xq, bool q_is_f16, int k, 
         const PageTail tail = run_page(nqp, xp, xp, k, D + q0 * ldk, I + q0 * ldk, ldk, nullptr, false);
         const bool fused = dtype_ == kF32 && tail.sampled && k <= kFinishMaxK;
         run_tail(tail, fused);
-        uint8_t* h = static_cast<uint8_t*>(h_over_.ensure(static_cast<size_t>(nqp) + sizeof(int)));
-        auto fetch_status = [&]() {
-            B200_CUDA_CHECK(cudaMemcpyAsync(h, w_over_.get(), static_cast<size_t>(nqp), cudaMemcpyDeviceToHost, stream_));
-            B200_CUDA_CHECK(cudaMemcpyAsync(h + nqp, w_err_.get(), sizeof(int), cudaMemcpyDeviceToHost, stream_));
-            B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
-        };
-        fetch_status();
-        if (fused && std::memchr(h, 2, static_cast<size_t>(nqp))) {   // lists too long for the fused tail
+        B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
+        if (fused && std::memchr(tail.status, 2, static_cast<size_t>(nqp))) {   // lists too long for the fused tail
             run_tail(tail, false);
-            fetch_status();
+            B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
         }
         timer_.collect(stats_);
         if (prof_) {
@@ -561,15 +595,9 @@ void FlatIndex::search_device(int64_t nq, const void* xq, bool q_is_f16, int k, 
                         c[4] / items, c[9] / items, c[8] / items, c[10] / items, c[5] / items, c[7] / items);
             }
         }
-        int err = 0;
-        std::memcpy(&err, h + nqp, sizeof(int));
-        if (err) {
-            cudaMemsetAsync(w_err_.get(), 0, sizeof(int), stream_);
-            throw std::runtime_error("device pipeline reported error word " + std::to_string(err) +
-                                     " (bounded wait ran out)");
-        }
+        throw_on_error(tail);
         for (int i = 0; i < nqp; ++i)
-            if (h[i]) over_idx.push_back(static_cast<int32_t>(q0 + i));
+            if (tail.status[i]) over_idx.push_back(static_cast<int32_t>(q0 + i));
     }
     if (!over_idx.empty()) {
         // Candidate overflow (heavy ties or an unrepresentative sample): re-run those queries
@@ -620,10 +648,8 @@ void FlatIndex::search_host_masked(int64_t nq, const void* xq, bool q_is_f16, in
     for (int64_t q0 = 0; q0 < nq; q0 += page) {
         const int64_t m = std::min<int64_t>(page, nq - q0);
         void* dq = w_stage_in_.ensure(static_cast<size_t>(m) * in_row);
-        float* dD = static_cast<float*>(w_stage_D_.ensure(static_cast<size_t>(m) * k * 4));
-        int64_t* dI = static_cast<int64_t*>(w_stage_I_.ensure(static_cast<size_t>(m) * k * 8));
-        B200_CUDA_CHECK(cudaMemcpyAsync(dq, static_cast<const uint8_t*>(xq) + q0 * in_row,
-                                        static_cast<size_t>(m) * in_row, cudaMemcpyHostToDevice, stream_));
+        HostResults out(h_I_, h_D_, w_stage_I_, w_stage_D_, m * k);
+        upload_small(dq, static_cast<const uint8_t*>(xq) + q0 * in_row, static_cast<size_t>(m) * in_row, h_in_, stream_);
         if (mask && n_ > 0) {
             void* dm = w_mask_.ensure(static_cast<size_t>(m) * mstride * 4);
             B200_CUDA_CHECK(cudaMemsetAsync(dm, 0, static_cast<size_t>(m) * mstride * 4, stream_));
@@ -632,12 +658,8 @@ void FlatIndex::search_host_masked(int64_t nq, const void* xq, bool q_is_f16, in
             mask_dev_ = static_cast<const uint32_t*>(dm);
             mask_stride_ = mstride;
         }
-        search_device(m, dq, q_is_f16, k, dD, dI, k);
-        B200_CUDA_CHECK(cudaMemcpyAsync(D + q0 * k, dD, static_cast<size_t>(m) * k * 4, cudaMemcpyDeviceToHost,
-                                        stream_));
-        B200_CUDA_CHECK(cudaMemcpyAsync(I + q0 * k, dI, static_cast<size_t>(m) * k * 8, cudaMemcpyDeviceToHost,
-                                        stream_));
-        B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
+        search_device(m, dq, q_is_f16, k, out.D, out.I, k);
+        out.deliver(D + q0 * k, I + q0 * k, stream_);
     }
 }
 

@@ -122,6 +122,8 @@ public:
     // int8.  D/I: device pointers with row stride ldk >= k.  Work is enqueued on stream();
     // the call synchronises that stream before returning (candidate-overflow check).
     void search_device(int64_t nq, const void* xq, bool q_is_f16, int k, float* D, int64_t* I, int ldk);
+    bool queue_search(int64_t nq, const float* xq, int k, float* D, int64_t* I, int ldk);
+    bool queued_ok();
     // Host-pointer search: pinned staging, H2D, search_device, D2H.
     void search_host(int64_t nq, const void* xq, bool q_is_f16, int k, float* D, int64_t* I);
     // mask: nq rows of ceil(ntotal / 8) bytes, bit (i % 8) of byte i / 8 = 1 lets base position i take part
@@ -162,8 +164,12 @@ private:
         bool sampled, prune;
         uint32_t cap;
         const float* xq;
+        uint8_t* status;   // per query, pinned (see EmitArgs::err_host for the error word behind it)
         EmitArgs e;
     };
+    PageTail queued_{};    // the search queue_search put on the stream
+    int64_t page_rows(uint32_t cap) const;
+    void throw_on_error(const PageTail& t);
     void run_tail(const PageTail& t, bool fused);
     PageTail run_page(int nq, const void* xq_raw, const void* xq_op, int k, float* D, int64_t* I, int ldk,
                   const int32_t* qmap_dev, bool force_full);
@@ -204,7 +210,7 @@ private:
     CUtensorMap map_b_;
 
     // scratch
-    DeviceBuffer w_qop_, w_qraw_, w_qnorm_, w_eps_, w_mins_, w_tau_, w_cand_, w_counts_, w_over_, w_qmap_,
+    DeviceBuffer w_qop_, w_qraw_, w_qnorm_, w_eps_, w_mins_, w_tau_, w_cand_, w_counts_, w_qmap_,
         w_err_, w_stage_in_, w_stage_D_, w_stage_I_, w_fb_q_, w_fb_qop_, w_prof_;
     bool prof_ = false;
     PinnedBuffer h_over_, h_in_, h_D_, h_I_;

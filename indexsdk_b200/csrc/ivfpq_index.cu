@@ -1235,7 +1235,7 @@ ivfpq_refine_kernel(const ScanArgs a, int P) {
             // fewer than k survivors although something was dropped, or the k-th is too close
             if (!have_k || !(sd[kk - 1] < a_min - eps)) bad = 1;
         }
-        a.flag[q] = bad;
+        if (bad) a.flag[q] = 1;
     }
 }
 
@@ -1312,7 +1312,7 @@ ivfpq_refine_warp_kernel(const ScanArgs a) {
             }
             if (lk == kNoLabel || !(dk < a_min - eps)) bad = 1;
         }
-        a.flag[q] = bad;
+        if (bad) a.flag[q] = 1;
     }
 }
 
@@ -2161,7 +2161,8 @@ std::vector<int32_t> IvfpqIndex::search_short(const ShortScanArgs& a, int64_t m,
     s.label_max = static_cast<uint64_t*>(w_fth_.ensure(static_cast<size_t>(g) * 12));
     s.thr = reinterpret_cast<float*>(s.label_max + g);
     s.count = static_cast<uint32_t*>(w_ccount_.ensure(static_cast<size_t>(g) * 4));
-    uint8_t* flag = static_cast<uint8_t*>(w_flag_.ensure(static_cast<size_t>(m)));
+    uint8_t* flag = static_cast<uint8_t*>(h_flag_.ensure(static_cast<size_t>(m)));
+    std::memset(flag, 0, static_cast<size_t>(m));
     for (int64_t g0 = 0; g0 < m; g0 += group) {
         s.nq = std::min(group, m - g0);
         s.cI = a.cI + g0 * a.nprobe;
@@ -2173,12 +2174,10 @@ std::vector<int32_t> IvfpqIndex::search_short(const ShortScanArgs& a, int64_t m,
         B200_CUDA_CHECK(launch_short_scan(s, num_sms_, st));
         stats_.kernel_launches += 3;
     }
-    uint8_t* hf = static_cast<uint8_t*>(h_flag_.ensure(static_cast<size_t>(m)));
-    B200_CUDA_CHECK(cudaMemcpyAsync(hf, flag, static_cast<size_t>(m), cudaMemcpyDeviceToHost, st));
     B200_CUDA_CHECK(cudaStreamSynchronize(st));
     std::vector<int32_t> bad;
     for (int64_t i = 0; i < m; ++i)
-        if (hf[i]) bad.push_back(static_cast<int32_t>(i));
+        if (flag[i]) bad.push_back(static_cast<int32_t>(i));
     return bad;
 }
 
@@ -2212,14 +2211,16 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
                              use_short_scan(M_, by_residual_, static_cast<double>(nprobe) * n_ / nlist_, nprobe, k);
     const int kprime = 32 * kpt;
     const int64_t page = 16384;
-    unsigned long long scanned = stats_.scan_codes;
-    const unsigned long long* scanned_src = &scanned;
     bool idle = true;    // the stream has been synchronised and nothing was queued since
+    scanned_known_ = false;
     for (int64_t q0 = 0; q0 < nq; q0 += page) {
         const int64_t m = std::min(page, nq - q0);
         const float* xp = xq + q0 * d_;
         const float* cD;
         const int64_t* cI;
+        // The probes of the page are queued and scanned without looking at their statuses, which are read
+        // with the scan's; in the rare case that one is not 0 (candidate overflow) the page is done again.
+        bool queued = false;
         if (pre_cI) {
             cD = pre_cD + q0 * nprobe;
             cI = pre_cI + q0 * nprobe;
@@ -2227,11 +2228,18 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
             float* wD = static_cast<float*>(w_cD_.ensure(static_cast<size_t>(m) * nprobe * 4));
             int64_t* wI = static_cast<int64_t*>(w_cI_.ensure(static_cast<size_t>(m) * nprobe * 8));
             timer_.begin(kStageCoarse, st);
-            coarse_->search_device(m, xp, false, nprobe, wD, wI, nprobe);
+            queued = coarse_->queue_search(m, xp, nprobe, wD, wI, nprobe);
+            if (!queued) coarse_->search_device(m, xp, false, nprobe, wD, wI, nprobe);
             timer_.end(st);
             cD = wD;
             cI = wI;
         }
+        auto probes_stand = [&]() {   // stream idle
+            if (!queued || coarse_->queued_ok()) return true;
+            coarse_->search_device(m, xp, false, nprobe, const_cast<float*>(cD), const_cast<int64_t*>(cI), nprobe);
+            queued = false;
+            return false;
+        };
 
         ScanArgs a{};
         a.cbT = codebooks_t_.as<float>();
@@ -2286,6 +2294,7 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
             s.outI = a.outI;
             s.scanned = a.scanned;
             std::vector<int32_t> bad = search_short(s, m, st);
+            if (!probes_stand()) bad = search_short(s, m, st);
             if (!bad.empty()) {
                 stats_.fallback_queries += bad.size();
                 int32_t* ql = static_cast<int32_t*>(w_qlist_.ensure(bad.size() * 4));
@@ -2299,10 +2308,17 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
             continue;
         }
         if (!fast) {
-            timer_.begin(kStageScan, st);
-            B200_CUDA_CHECK(launch_exact(a, static_cast<int>(m), st));
-            timer_.end(st);
-            stats_.kernel_launches += 2;
+            for (bool again = true; again;) {
+                timer_.begin(kStageScan, st);
+                B200_CUDA_CHECK(launch_exact(a, static_cast<int>(m), st));
+                timer_.end(st);
+                stats_.kernel_launches += 2;
+                again = false;
+                if (queued) {
+                    B200_CUDA_CHECK(cudaStreamSynchronize(st));
+                    again = !probes_stand();
+                }
+            }
             idle = false;
             continue;
         }
@@ -2320,7 +2336,7 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
         a.fd = static_cast<float*>(w_fd_.ensure(static_cast<size_t>(m) * S * kprime * 4));
         a.fp = static_cast<uint32_t*>(w_fp_.ensure(static_cast<size_t>(m) * S * kprime * 4));
         a.fth = static_cast<float*>(w_fth_.ensure(static_cast<size_t>(m) * S * 4));
-        a.flag = static_cast<uint8_t*>(w_flag_.ensure(static_cast<size_t>(m)));
+        a.flag = static_cast<uint8_t*>(h_flag_.ensure(static_cast<size_t>(m)));   // pinned: kernels write what is not 0
         a.err_rel = filter_err_rel();
         a.cb_bound = cb_norm_bound_;
         a.t2_bound = t2_bound();
@@ -2328,155 +2344,152 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
         // all of its queries on the tensor cores (ivfpq_tc_scan.cu)
         const bool tc = persist && tc_scan_ && tc_cb_ok_ && by_residual_ && d_ == kTcDim && M_ == kTcM && kpt == 1 &&
                         nprobe >= 16 && m * nprobe < (1LL << 30);
-        unsigned int* tc_err = nullptr;
-        timer_.begin(kStageScan, st);
-        if (tc) {
-            const int64_t npairs = m * nprobe;
-            int32_t* keys = static_cast<int32_t*>(w_tc_keys_.ensure(static_cast<size_t>(npairs) * 4));
-            int32_t* vals = static_cast<int32_t*>(w_tc_vals_.ensure(static_cast<size_t>(npairs) * 4));
-            int32_t* keys2 = static_cast<int32_t*>(w_tc_keys2_.ensure(static_cast<size_t>(npairs) * 4));
-            int32_t* vals2 = static_cast<int32_t*>(w_tc_vals2_.ensure(static_cast<size_t>(npairs) * 4));
-            int32_t* first = static_cast<int32_t*>(w_tc_first_.ensure(static_cast<size_t>(nlist_) * 4));
-            int32_t* last = static_cast<int32_t*>(w_tc_last_.ensure(static_cast<size_t>(nlist_) * 4));
-            B200_CUDA_CHECK(launch_tc_keys(cI, npairs, nlist_, keys, vals, st));
-            int end_bit = 1;
-            while ((1 << end_bit) <= nlist_) ++end_bit;
-            size_t sort_bytes = 0;
-            B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys, keys2, vals, vals2,
-                                                            static_cast<int>(npairs), 0, end_bit, st));
-            void* sort_tmp = w_tc_sort_.ensure(sort_bytes);
-            B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, keys, keys2, vals, vals2,
-                                                            static_cast<int>(npairs), 0, end_bit, st));
-            B200_CUDA_CHECK(launch_tc_bounds(keys2, npairs, nlist_, first, last, st));
-            // lists with the most probing queries are handed out first, so that no long list is
-            // left for the end of the launch
-            int32_t* okeys = static_cast<int32_t*>(w_tc_okeys_.ensure(static_cast<size_t>(nlist_) * 16));
-            int32_t* ovals = okeys + nlist_;
-            int32_t* okeys2 = ovals + nlist_;
-            int32_t* order = okeys2 + nlist_;
-            B200_CUDA_CHECK(launch_tc_order_keys(first, last, nlist_, okeys, ovals, st));
-            size_t osort_bytes = 0;
-            B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, osort_bytes, okeys, okeys2, ovals, order, nlist_, 0, 31, st));
-            void* osort_tmp = w_tc_osort_.ensure(osort_bytes);
-            B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(osort_tmp, osort_bytes, okeys, okeys2, ovals, order, nlist_, 0, 31, st));
-            float* tau = static_cast<float*>(w_tc_tau_.ensure(static_cast<size_t>(m) * 4));
-            TcScanArgs t{};
-            t.cb16 = cb16_.as<uint16_t>();
-            t.cbnorm = cbnorm_.as<float>();
-            t.xq = xp;
-            t.centroids = coarse_->rows_f32();
-            t.cD = cD;
-            t.nprobe = nprobe;
-            t.nlist = nlist_;
-            t.nq = m;
-            t.sorted_pair = vals2;
-            t.first = first;
-            t.last = last;
-            t.order = order;
-            t.offsets = offsets_.as<int64_t>();
-            t.lens = lens_.as<int64_t>();
-            t.codes = codes_.as<uint8_t>();
-            t.tau = tau;
-            t.cap = 256;
-            t.cb_bound = a.cb_bound;
-            t.cand_d = static_cast<float*>(w_tc_cd_.ensure(static_cast<size_t>(m) * t.cap * 4));
-            t.cand_p = static_cast<uint32_t*>(w_tc_cp_.ensure(static_cast<size_t>(m) * t.cap * 4));
-            t.cand_n = static_cast<unsigned int*>(w_tc_cn_.ensure(static_cast<size_t>(m) * 4));
-            t.stage_cap = kTcStageCap;
-            t.stage = static_cast<uint4*>(w_tc_stage_.ensure(static_cast<size_t>(num_sms_) * kTcStageCap * 16));
-            t.stage_n = static_cast<unsigned int*>(w_tc_stage_n_.ensure(static_cast<size_t>(num_sms_) * 4));
-            t.work = w_work_.as<unsigned int>();
-            t.scanned = a.scanned;
-            if (!w_tc_err_.get()) {
-                w_tc_err_.ensure(4);
-                B200_CUDA_CHECK(cudaMemsetAsync(w_tc_err_.get(), 0, 4, st));
-            }
-            t.err = tc_err = w_tc_err_.as<unsigned int>();
-#ifdef B200IDX_DEV_PROF
-            const char* pe = std::getenv("B200IDX_PROF");
-            const bool tc_prof = pe && std::strcmp(pe, "1") == 0;
-#else
-            const bool tc_prof = false;
-#endif
-            if (tc_prof) {
-                w_tc_prof_.ensure(64 + static_cast<size_t>(m) * 4);
-                B200_CUDA_CHECK(cudaMemsetAsync(w_tc_prof_.get(), 0, 64, st));
-                t.prof = w_tc_prof_.as<unsigned long long>();
-            }
-            // threshold: one warp per query over the codes of its nearest list
-            B200_CUDA_CHECK(launch_tc_head_tau(t, cI, a.err_rel, a.t2_bound, tau, st));
-            B200_CUDA_CHECK(launch_tc_scan(t, num_sms_, st));
-            B200_CUDA_CHECK(launch_tc_select(t, a.fd, a.fp, a.fth, st));
-            if (tc_prof) {   // development aid: phase cycles of thread 0 (sum over CTAs), candidates per query
-                unsigned long long hp[8];
-                std::vector<unsigned int> cn(static_cast<size_t>(m));
-                B200_CUDA_CHECK(cudaMemcpyAsync(hp, t.prof, 64, cudaMemcpyDeviceToHost, st));
-                B200_CUDA_CHECK(cudaMemcpyAsync(cn.data(), t.cand_n, cn.size() * 4, cudaMemcpyDeviceToHost, st));
-                B200_CUDA_CHECK(cudaStreamSynchronize(st));
-                unsigned long long tot = 0, mx = 0;
-                for (unsigned int c : cn) { tot += c; mx = std::max<unsigned long long>(mx, c); }
-                std::fprintf(stderr, "[tc scan] per-CTA kcycles: ctx_wait %.0f decode %.0f barrier %.0f issue %.0f mma_wait %.0f "
-                             "epilogue %.0f release %.0f; tiles/CTA %.0f; candidates/query avg %.1f max %llu\n",
-                             hp[0] / 1e3 / num_sms_, hp[1] / 1e3 / num_sms_, hp[2] / 1e3 / num_sms_, hp[3] / 1e3 / num_sms_,
-                             hp[4] / 1e3 / num_sms_, hp[5] / 1e3 / num_sms_, hp[6] / 1e3 / num_sms_,
-                             static_cast<double>(hp[7]) / num_sms_, static_cast<double>(tot) / m, mx);
-            }
-            a.tc_rel = kTcErrRel;
-            a.tc_abs = kTcErrAbs;
-            stats_.kernel_launches += 8;
-        } else if (persist) {
-            a.work = w_work_.as<unsigned int>();
-#ifdef B200IDX_DEV_PROF
-            a.prof = static_cast<unsigned long long*>(w_tc_prof_.ensure(128));
-            B200_CUDA_CHECK(cudaMemsetAsync(a.prof, 0, 128, st));
-#endif
-            B200_CUDA_CHECK(launch_persist(a, kpt, num_sms_, st));
-#ifdef B200IDX_DEV_PROF
-            {
-                unsigned long long hp[16];
-                B200_CUDA_CHECK(cudaMemcpyAsync(hp, a.prof, 128, cudaMemcpyDeviceToHost, st));
-                B200_CUDA_CHECK(cudaStreamSynchronize(st));
-                const double nq_s = hp[9] ? static_cast<double>(hp[9]) : 1.0;
-                std::fprintf(stderr, "[persist scan] cycles per query of a slot -- warp 1: build %.0f wait %.0f scan %.0f wait %.0f | "
-                             "warp 0: build %.0f wait %.0f scan %.0f wait %.0f merge %.0f\n", hp[0] / nq_s, hp[1] / nq_s,
-                             hp[2] / nq_s, hp[3] / nq_s, hp[4] / nq_s, hp[5] / nq_s, hp[6] / nq_s, hp[7] / nq_s, hp[8] / nq_s);
-            }
-#endif
-        } else {
-            B200_CUDA_CHECK(launch_fast(a, kpt, st));
-        }
-        timer_.end(st);
-        timer_.begin(kStageMerge, st);
-        const int P = pow2_ceil_int(std::max(S * kprime, 32));
-        const size_t rsmem = static_cast<size_t>(P) * 12;
-        if (S * kprime == 32 && k <= 32 && nprobe <= kRefMaxProbe) {
-            ivfpq_refine_warp_kernel<<<blocks_for(m, kRefWarpsPerBlock), kRefWarpsPerBlock * 32, 0, st>>>(a);
-        } else {
-            B200_CUDA_CHECK(set_smem(ivfpq_refine_kernel, rsmem));
-            ivfpq_refine_kernel<<<static_cast<unsigned>(m), kScanThreads, rsmem, st>>>(a, P);
-        }
-        B200_CUDA_CHECK(cudaGetLastError());
-        timer_.end(st);
-        stats_.kernel_launches += 3;
-        // flags of the page and, behind them, the counter of visited codes: one copy-back and one
-        // synchronisation per page
-        const size_t cnt_off = (static_cast<size_t>(m) + 7) & ~size_t(7);
-        uint8_t* hf = static_cast<uint8_t*>(h_flag_.ensure(cnt_off + 8));
-        B200_CUDA_CHECK(cudaMemcpyAsync(hf, a.flag, static_cast<size_t>(m), cudaMemcpyDeviceToHost, st));
-        B200_CUDA_CHECK(cudaMemcpyAsync(hf + cnt_off, w_tmp_.get(), 8, cudaMemcpyDeviceToHost, st));
-        scanned_src = reinterpret_cast<const unsigned long long*>(hf + cnt_off);
-        idle = false;
+        uint8_t* hf = a.flag;
         unsigned int tc_err_host = 0;
-        if (tc_err) B200_CUDA_CHECK(cudaMemcpyAsync(&tc_err_host, tc_err, 4, cudaMemcpyDeviceToHost, st));
-        B200_CUDA_CHECK(cudaStreamSynchronize(st));
-        idle = true;
-        scanned = *scanned_src;
-        if (tc_err_host) cudaMemsetAsync(tc_err, 0, 4, st);
-        if (tc_err_host & 2u)                       // a staging area overflowed: candidates were lost,
-            std::memset(hf, 1, static_cast<size_t>(m));   // every query of the page takes the exact path
-        if (tc_err_host & 1u) {
-            throw std::runtime_error("IVFPQ tensor-core scan reported error word " + std::to_string(tc_err_host) +
-                                     " (bounded wait ran out)");
+        for (;;) {
+            std::memset(hf, 0, static_cast<size_t>(m));
+            unsigned int* tc_err = nullptr;
+            timer_.begin(kStageScan, st);
+            if (tc) {
+                const int64_t npairs = m * nprobe;
+                int32_t* keys = static_cast<int32_t*>(w_tc_keys_.ensure(static_cast<size_t>(npairs) * 4));
+                int32_t* vals = static_cast<int32_t*>(w_tc_vals_.ensure(static_cast<size_t>(npairs) * 4));
+                int32_t* keys2 = static_cast<int32_t*>(w_tc_keys2_.ensure(static_cast<size_t>(npairs) * 4));
+                int32_t* vals2 = static_cast<int32_t*>(w_tc_vals2_.ensure(static_cast<size_t>(npairs) * 4));
+                int32_t* first = static_cast<int32_t*>(w_tc_first_.ensure(static_cast<size_t>(nlist_) * 4));
+                int32_t* last = static_cast<int32_t*>(w_tc_last_.ensure(static_cast<size_t>(nlist_) * 4));
+                B200_CUDA_CHECK(launch_tc_keys(cI, npairs, nlist_, keys, vals, st));
+                int end_bit = 1;
+                while ((1 << end_bit) <= nlist_) ++end_bit;
+                size_t sort_bytes = 0;
+                B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys, keys2, vals, vals2,
+                                                                static_cast<int>(npairs), 0, end_bit, st));
+                void* sort_tmp = w_tc_sort_.ensure(sort_bytes);
+                B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, keys, keys2, vals, vals2,
+                                                                static_cast<int>(npairs), 0, end_bit, st));
+                B200_CUDA_CHECK(launch_tc_bounds(keys2, npairs, nlist_, first, last, st));
+                // lists with the most probing queries are handed out first, so that no long list is
+                // left for the end of the launch
+                int32_t* okeys = static_cast<int32_t*>(w_tc_okeys_.ensure(static_cast<size_t>(nlist_) * 16));
+                int32_t* ovals = okeys + nlist_;
+                int32_t* okeys2 = ovals + nlist_;
+                int32_t* order = okeys2 + nlist_;
+                B200_CUDA_CHECK(launch_tc_order_keys(first, last, nlist_, okeys, ovals, st));
+                size_t osort_bytes = 0;
+                B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, osort_bytes, okeys, okeys2, ovals, order, nlist_, 0, 31, st));
+                void* osort_tmp = w_tc_osort_.ensure(osort_bytes);
+                B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(osort_tmp, osort_bytes, okeys, okeys2, ovals, order, nlist_, 0, 31, st));
+                float* tau = static_cast<float*>(w_tc_tau_.ensure(static_cast<size_t>(m) * 4));
+                TcScanArgs t{};
+                t.cb16 = cb16_.as<uint16_t>();
+                t.cbnorm = cbnorm_.as<float>();
+                t.xq = xp;
+                t.centroids = coarse_->rows_f32();
+                t.cD = cD;
+                t.nprobe = nprobe;
+                t.nlist = nlist_;
+                t.nq = m;
+                t.sorted_pair = vals2;
+                t.first = first;
+                t.last = last;
+                t.order = order;
+                t.offsets = offsets_.as<int64_t>();
+                t.lens = lens_.as<int64_t>();
+                t.codes = codes_.as<uint8_t>();
+                t.tau = tau;
+                t.cap = 256;
+                t.cb_bound = a.cb_bound;
+                t.cand_d = static_cast<float*>(w_tc_cd_.ensure(static_cast<size_t>(m) * t.cap * 4));
+                t.cand_p = static_cast<uint32_t*>(w_tc_cp_.ensure(static_cast<size_t>(m) * t.cap * 4));
+                t.cand_n = static_cast<unsigned int*>(w_tc_cn_.ensure(static_cast<size_t>(m) * 4));
+                t.stage_cap = kTcStageCap;
+                t.stage = static_cast<uint4*>(w_tc_stage_.ensure(static_cast<size_t>(num_sms_) * kTcStageCap * 16));
+                t.stage_n = static_cast<unsigned int*>(w_tc_stage_n_.ensure(static_cast<size_t>(num_sms_) * 4));
+                t.work = w_work_.as<unsigned int>();
+                t.scanned = a.scanned;
+                if (!w_tc_err_.get()) {
+                    w_tc_err_.ensure(4);
+                    B200_CUDA_CHECK(cudaMemsetAsync(w_tc_err_.get(), 0, 4, st));
+                }
+                t.err = tc_err = w_tc_err_.as<unsigned int>();
+#ifdef B200IDX_DEV_PROF
+                const char* pe = std::getenv("B200IDX_PROF");
+                const bool tc_prof = pe && std::strcmp(pe, "1") == 0;
+#else
+                const bool tc_prof = false;
+#endif
+                if (tc_prof) {
+                    w_tc_prof_.ensure(64 + static_cast<size_t>(m) * 4);
+                    B200_CUDA_CHECK(cudaMemsetAsync(w_tc_prof_.get(), 0, 64, st));
+                    t.prof = w_tc_prof_.as<unsigned long long>();
+                }
+                // threshold: one warp per query over the codes of its nearest list
+                B200_CUDA_CHECK(launch_tc_head_tau(t, cI, a.err_rel, a.t2_bound, tau, st));
+                B200_CUDA_CHECK(launch_tc_scan(t, num_sms_, st));
+                B200_CUDA_CHECK(launch_tc_select(t, a.fd, a.fp, a.fth, st));
+                if (tc_prof) {   // development aid: phase cycles of thread 0 (sum over CTAs), candidates per query
+                    unsigned long long hp[8];
+                    std::vector<unsigned int> cn(static_cast<size_t>(m));
+                    B200_CUDA_CHECK(cudaMemcpyAsync(hp, t.prof, 64, cudaMemcpyDeviceToHost, st));
+                    B200_CUDA_CHECK(cudaMemcpyAsync(cn.data(), t.cand_n, cn.size() * 4, cudaMemcpyDeviceToHost, st));
+                    B200_CUDA_CHECK(cudaStreamSynchronize(st));
+                    unsigned long long tot = 0, mx = 0;
+                    for (unsigned int c : cn) { tot += c; mx = std::max<unsigned long long>(mx, c); }
+                    std::fprintf(stderr, "[tc scan] per-CTA kcycles: ctx_wait %.0f decode %.0f barrier %.0f issue %.0f mma_wait %.0f "
+                                 "epilogue %.0f release %.0f; tiles/CTA %.0f; candidates/query avg %.1f max %llu\n",
+                                 hp[0] / 1e3 / num_sms_, hp[1] / 1e3 / num_sms_, hp[2] / 1e3 / num_sms_, hp[3] / 1e3 / num_sms_,
+                                 hp[4] / 1e3 / num_sms_, hp[5] / 1e3 / num_sms_, hp[6] / 1e3 / num_sms_,
+                                 static_cast<double>(hp[7]) / num_sms_, static_cast<double>(tot) / m, mx);
+                }
+                a.tc_rel = kTcErrRel;
+                a.tc_abs = kTcErrAbs;
+                stats_.kernel_launches += 8;
+            } else if (persist) {
+                a.work = w_work_.as<unsigned int>();
+#ifdef B200IDX_DEV_PROF
+                a.prof = static_cast<unsigned long long*>(w_tc_prof_.ensure(128));
+                B200_CUDA_CHECK(cudaMemsetAsync(a.prof, 0, 128, st));
+#endif
+                B200_CUDA_CHECK(launch_persist(a, kpt, num_sms_, st));
+#ifdef B200IDX_DEV_PROF
+                {
+                    unsigned long long hp[16];
+                    B200_CUDA_CHECK(cudaMemcpyAsync(hp, a.prof, 128, cudaMemcpyDeviceToHost, st));
+                    B200_CUDA_CHECK(cudaStreamSynchronize(st));
+                    const double nq_s = hp[9] ? static_cast<double>(hp[9]) : 1.0;
+                    std::fprintf(stderr, "[persist scan] cycles per query of a slot -- warp 1: build %.0f wait %.0f scan %.0f wait %.0f | "
+                                 "warp 0: build %.0f wait %.0f scan %.0f wait %.0f merge %.0f\n", hp[0] / nq_s, hp[1] / nq_s,
+                                 hp[2] / nq_s, hp[3] / nq_s, hp[4] / nq_s, hp[5] / nq_s, hp[6] / nq_s, hp[7] / nq_s, hp[8] / nq_s);
+                }
+#endif
+            } else {
+                B200_CUDA_CHECK(launch_fast(a, kpt, st));
+            }
+            timer_.end(st);
+            timer_.begin(kStageMerge, st);
+            const int P = pow2_ceil_int(std::max(S * kprime, 32));
+            const size_t rsmem = static_cast<size_t>(P) * 12;
+            if (S * kprime == 32 && k <= 32 && nprobe <= kRefMaxProbe) {
+                ivfpq_refine_warp_kernel<<<blocks_for(m, kRefWarpsPerBlock), kRefWarpsPerBlock * 32, 0, st>>>(a);
+            } else {
+                B200_CUDA_CHECK(set_smem(ivfpq_refine_kernel, rsmem));
+                ivfpq_refine_kernel<<<static_cast<unsigned>(m), kScanThreads, rsmem, st>>>(a, P);
+            }
+            B200_CUDA_CHECK(cudaGetLastError());
+            timer_.end(st);
+            stats_.kernel_launches += 3;
+            idle = false;
+            if (tc_err) B200_CUDA_CHECK(cudaMemcpyAsync(&tc_err_host, tc_err, 4, cudaMemcpyDeviceToHost, st));
+            B200_CUDA_CHECK(cudaStreamSynchronize(st));
+            idle = true;
+            if (tc_err_host) cudaMemsetAsync(tc_err, 0, 4, st);
+            if (tc_err_host & 2u)                       // a staging area overflowed: candidates were lost,
+                std::memset(hf, 1, static_cast<size_t>(m));   // every query of the page takes the exact path
+            if (tc_err_host & 1u) {
+                throw std::runtime_error("IVFPQ tensor-core scan reported error word " + std::to_string(tc_err_host) +
+                                         " (bounded wait ran out)");
+            }
+            if (probes_stand()) break;
         }
         std::vector<int32_t> bad;
         for (int64_t i = 0; i < m; ++i)
@@ -2492,7 +2505,6 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
             timer_.begin(kStageScan, st);
             B200_CUDA_CHECK(launch_collect(a, static_cast<int>(bad.size()), cpos, ccount, st));
             timer_.end(st);
-            B200_CUDA_CHECK(cudaMemcpyAsync(hf, a.flag, static_cast<size_t>(m), cudaMemcpyDeviceToHost, st));
             B200_CUDA_CHECK(cudaStreamSynchronize(st));
             stats_.kernel_launches += 2;
             std::vector<int32_t> still;
@@ -2510,12 +2522,8 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
             stats_.kernel_launches += 1;
         }
     }
-    if (!idle) {   // (the exact-only path queues its kernels without reading anything back)
-        B200_CUDA_CHECK(cudaMemcpyAsync(&scanned, w_tmp_.get(), 8, cudaMemcpyDeviceToHost, st));
-        B200_CUDA_CHECK(cudaStreamSynchronize(st));
-    }
+    if (!idle) B200_CUDA_CHECK(cudaStreamSynchronize(st));
     timer_.collect(stats_);
-    stats_.scan_codes = scanned;
     stats_.kernel_launches += coarse_->stats().kernel_launches;
     stats_.gemm_launches += coarse_->stats().gemm_launches;
     coarse_->stats().kernel_launches = 0;
@@ -2527,13 +2535,26 @@ void IvfpqIndex::search_host(int64_t nq, const float* xq, int k, float* D, int64
     DeviceGuard g(device_);
     cudaStream_t st = stream();
     float* dq = static_cast<float*>(w_q_.ensure(static_cast<size_t>(nq) * d_ * 4));
-    float* dD = static_cast<float*>(w_D_.ensure(static_cast<size_t>(nq) * k * 4));
-    int64_t* dI = static_cast<int64_t*>(w_I_.ensure(static_cast<size_t>(nq) * k * 8));
-    B200_CUDA_CHECK(cudaMemcpyAsync(dq, xq, static_cast<size_t>(nq) * d_ * 4, cudaMemcpyHostToDevice, st));
-    search_device(nq, dq, k, dD, dI);
-    B200_CUDA_CHECK(cudaMemcpyAsync(D, dD, static_cast<size_t>(nq) * k * 4, cudaMemcpyDeviceToHost, st));
-    B200_CUDA_CHECK(cudaMemcpyAsync(I, dI, static_cast<size_t>(nq) * k * 8, cudaMemcpyDeviceToHost, st));
-    B200_CUDA_CHECK(cudaStreamSynchronize(st));
+    HostResults out(h_I_, h_D_, w_I_, w_D_, nq * k);
+    upload_small(dq, xq, static_cast<size_t>(nq) * d_ * 4, h_q_, st);
+    search_device(nq, dq, k, out.D, out.I);
+    out.deliver(D, I, st);
+}
+
+// The counter of visited codes lives on the device and is read when somebody asks.
+SearchStats& IvfpqIndex::stats() {
+    if (!scanned_known_ && w_tmp_.get()) {
+        DeviceGuard g(device_);
+        unsigned long long v = 0;   // (no exception leaves here: the C entry that asks is not guarded)
+        if (cudaMemcpyAsync(&v, w_tmp_.get(), 8, cudaMemcpyDeviceToHost, stream()) == cudaSuccess &&
+            cudaStreamSynchronize(stream()) == cudaSuccess) {
+            stats_.scan_codes = v;
+            scanned_known_ = true;
+        } else {
+            cudaGetLastError();
+        }
+    }
+    return stats_;
 }
 
 }  // namespace b200

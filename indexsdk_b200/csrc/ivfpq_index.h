@@ -33,7 +33,7 @@ public:
     int nprobe() const { return nprobe_; }
     void set_nprobe(int p) { nprobe_ = p; }
     bool is_trained() const { return has_centroids_ && has_codebooks_; }
-    SearchStats& stats() { return stats_; }
+    SearchStats& stats();
     SearchStats& coarse_stats() { return coarse_->stats(); }
     void set_timing(bool on) {
         timer_.enable(on);
@@ -109,6 +109,8 @@ private:
         w_tc_fd0_, w_tc_fp0_, w_tc_fth0_, w_tc_tau_, w_tc_cd_, w_tc_cp_, w_tc_cn_, w_tc_sort_, w_tc_err_, w_tc_prof_, w_tc_stage_, w_tc_stage_n_, w_tc_okeys_, w_tc_osort_;
     PinnedBuffer h_flag_;
     SearchStats stats_;
+    bool scanned_known_ = true;   // stats_.scan_codes holds the device's counter
+    PinnedBuffer h_q_, h_D_, h_I_;
     StageTimer timer_;
 };
 

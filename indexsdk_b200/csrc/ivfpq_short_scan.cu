@@ -521,8 +521,10 @@ short_select_kernel(const ShortScanArgs a) {
     __shared__ uint32_t hist[256], s_warp[32], s_out[2], s_fill, s_eq;
     const int64_t q = blockIdx.x;
     const uint32_t n = a.count[q];
-    if (threadIdx.x == 0) a.flag[q] = n > a.cap ? 1 : 0;
-    if (n > a.cap) return;
+    if (n > a.cap) {
+        if (threadIdx.x == 0) a.flag[q] = 1;
+        return;
+    }
     uint2* row = a.cand + q * a.cap;
     if (a.by_residual) {
         for (uint32_t i = threadIdx.x; i < n; i += kSelThreadsShort) {

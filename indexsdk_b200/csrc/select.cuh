@@ -64,17 +64,21 @@ struct EmitArgs {
     int ldk;
     const int32_t* qmap;     // optional: output row = qmap[q] (fallback re-runs scatter into place)
     int q_mod;               // > 0: row q uses the query norm of row q % q_mod (multi-index search)
+    const int* err;          // device error word of the passes before, and where the host reads it (pinned, zeroed by
+    int* err_host;           // the host beforehand); nullptr: the caller reads the word itself
     const MemberView* members;   // with q_mod: row q's labels are those of member q / q_mod (device array, or nullptr)
 };
 // Per query: the k smallest of cand[q][0..min(counts[q],cap)) in ascending order as results (FLT_MAX / -1
 // where there are fewer).  counts == nullptr means every row holds n_fixed candidates.  overflow[q] is
 // set to 1 when counts[q] > cap (the row's result is then not trustworthy and the caller re-runs it
-// without a threshold); *any_overflow is set to 1 when that happens to any row.
+// without a threshold), and so is *any_overflow; neither is written otherwise.  D, I, overflow and
+// any_overflow may lie in pinned host memory: stores there cost no copy and no wait of their own.
 cudaError_t launch_select_emit(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap,
                                uint8_t* overflow, uint32_t* any_overflow, const EmitArgs& e, cudaStream_t stream);
 // fp32 indexes: pruning, exact distances, selection and results of short candidate lists in one launch.
-// status[q] = 0 done, 1 row overflowed, 2 list too long for it (prune, refine and select it instead; the row
-// is unchanged); *any_status is set to 1 when any row is left.  k <= kFinishMaxK.  few: lists of little
+// status[q], written when it is not 0: 1 row overflowed, 2 list too long for it (prune, refine and select it
+// instead; the candidates are unchanged, the results are padding); *any_status is set to 1 when any row is
+// left.  k <= kFinishMaxK.  few: lists of little
 // more than k candidates are expected (a threshold over the whole base), no need to prune them first.
 constexpr int kFinishMaxK = 256;
 cudaError_t launch_finish_f32(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int d, const float* eps,
