@@ -19,8 +19,12 @@ struct RankScratch {
 // over the spanned range: two or three passes, almost no collisions).  After `passes` passes the upper
 // edge of the bin is returned (a bound from above, 2^-20 of the range wide after two) unless the rank is
 // settled before; passes = 4 always settles it.  Every thread of the block must call this.
+struct RankResult {
+    uint32_t lo, hi;   // the r-th smallest key lies in [lo, hi] (both 0xFFFFFFFF: fewer than r keys)
+    uint32_t left;     // its rank among the keys in there
+};
 template <int NT, typename Visit>
-__device__ __forceinline__ uint32_t block_kth32(Visit visit, uint32_t r, RankScratch& s, int passes) {
+__device__ __forceinline__ RankResult block_rank32(Visit visit, uint32_t r, RankScratch& s, int passes) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     constexpr int kPer = kRankBins / NT;
     if (threadIdx.x == 0) {
@@ -47,7 +51,7 @@ __device__ __forceinline__ uint32_t block_kth32(Visit visit, uint32_t r, RankScr
     }
     __syncthreads();
     uint32_t lo = s.lo, hi = s.hi;
-    if (s.n < r) return 0xFFFFFFFFu;
+    if (s.n < r) return RankResult{0xFFFFFFFFu, 0xFFFFFFFFu, 0u};
     for (int pass = 0; pass < passes && lo != hi; ++pass) {
         const int shift = max(0, 22 - __clz(hi - lo));
         for (int b = threadIdx.x; b < kRankBins; b += NT) s.hist[b] = 0u;
@@ -89,7 +93,11 @@ __device__ __forceinline__ uint32_t block_kth32(Visit visit, uint32_t r, RankScr
         r -= s.below;
     }
     __syncthreads();   // the scratch may be reused
-    return hi;
+    return RankResult{lo, hi, r};
+}
+template <int NT, typename Visit>
+__device__ __forceinline__ uint32_t block_kth32(Visit visit, uint32_t r, RankScratch& s, int passes) {
+    return block_rank32<NT>(visit, r, s, passes).hi;
 }
 
 }  // namespace b200
