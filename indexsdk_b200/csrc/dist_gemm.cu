@@ -553,7 +553,7 @@ struct RowEpilogue {
 };
 
 __device__ __forceinline__ int tile_of(const GemmArgs& a, int sel) {
-    if (a.tile_first >= 0) return a.tile_first + sel;   // a contiguous stretch of tiles (whole base: first = 0)
+    if (a.tile_first >= 0) return a.tile_first + sel * a.tile_step;   // a stretch of tiles (whole base: first = 0)
     return static_cast<int>(static_cast<int64_t>(sel) * a.n_tiles_total / a.n_tiles_sel);
 }
 
@@ -1145,6 +1145,7 @@ cudaError_t launch_one(const GemmLaunch& L, GemmArgs a, const CUtensorMap* mapA,
     const int n_qb = (a.nq + kTileQ - 1) / kTileQ;
     const int64_t total = static_cast<int64_t>(n_qb) * a.n_tiles_sel;
     if (total <= 0) return cudaSuccess;
+    if (a.tile_step < 1) a.tile_step = 1;
     if (L.simt) {
         const int grid = static_cast<int>(total < 4LL * L.num_sms ? total : 4LL * L.num_sms);
         dist_gemm_simt_kernel<KIND, MODE, BURST><<<grid, kTileQ, 0, stream>>>(a);

@@ -63,8 +63,9 @@ struct GemmArgs {
     int64_t N;
     int n_tiles_total;    // ceil(N / kTileB)
     int n_tiles_sel;      // tiles visited by this pass
-    int tile_first;       // >= 0: tiles tile_first .. tile_first + n_tiles_sel - 1;
+    int tile_first;       // >= 0: tiles tile_first, tile_first + tile_step, ...: n_tiles_sel of them;
                           // -1: n_tiles_sel tiles spread evenly, tile(i) = i * n_tiles_total / n_tiles_sel
+    int tile_step;        // 0 and 1: consecutive tiles
     int metric;           // kMetricIP / kMetricL2 / kMetricCos (i8 only)
     const void* bnorm;    // float* (f16/bf16 kinds) or int32_t* (i8): squared norm per base row, L2 and cosine
     const int32_t* qnorm_i32;   // kMetricCos: squared norm per query

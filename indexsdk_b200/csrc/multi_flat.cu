@@ -190,14 +190,20 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
     const size_t nm = cur_.size();
     const int n_qb = (nq + kTileQ - 1) / kTileQ;
     uint32_t cap = cap_;
-    int burst = 32;
+    int burst = 32, step = 1;
     if (with_tau) {
-        for (size_t i = 0; i < nm; ++i)
-            if ((seg_start_[i + 1] - seg_start_[i]) / 32 < 8LL * k) burst = 8;
+        int64_t least = cap_;
+        for (size_t i = 0; i < nm; ++i) least = std::min(least, seg_start_[i + 1] - seg_start_[i]);
+        // The minima of every fourth tile are enough where each member still has 8 k bursts of 8 in them:
+        // four times the candidates (k of every 4 k rows pass), but the first pass reads a quarter of the
+        // rows, and with few queries it is bound by that (32 members of 20 000 x 128, 64 queries, k = 10:
+        // 38 -> 14 us, the end 26 -> 34).
+        if ((least / kTileB) / 4 * (kTileB / 8) >= 8LL * k) step = 4;
+        if (least / kTileB / step * (kTileB / 32) < 8LL * k) burst = 8;
         // Room for 9 k keys, and for the slots the epilogue's threads reserve in blocks of 8 and leave
         // unused: four threads per row in each CTA that walks the member, an open and a reserved block each.
         const double ctas = static_cast<double>(cap_ / kTileB) * num_sms_ / (static_cast<double>(n_qb) * (total_rows_ / kTileB));
-        const uint64_t want = 10ull * k + 64ull * (static_cast<uint64_t>(std::min<double>(ctas, cap_ / kTileB)) + 2);
+        const uint64_t want = (step > 1 ? 12ull : 10ull) * k + 64ull * (static_cast<uint64_t>(std::min<double>(ctas, cap_ / kTileB)) + 2);
         cap = 512;
         while (cap < want) cap <<= 1;
     }
@@ -250,7 +256,10 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
             a.mins_stride = mins_stride;
             L.mode = kModeBurstMin;
             L.burst = burst;
-            B200_CUDA_CHECK(launch_dist_gemm(L, a, &map_a, &map_b_, st));
+            GemmArgs sample = a;
+            sample.tile_step = step;
+            sample.n_tiles_sel = (a.n_tiles_sel + step - 1) / step;
+            B200_CUDA_CHECK(launch_dist_gemm(L, sample, &map_a, &map_b_, st));
             TauFold fold;
             fold.counts = counts;
             fold.q_mod = nq;

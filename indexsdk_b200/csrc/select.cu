@@ -115,7 +115,11 @@ kth_threshold_kernel(const uint32_t* mins, int stride, int n, int k, const float
     }
     const uint32_t* keys = staged ? kth_keys : row;
     uint32_t kth = block_kth32<kSelThreads>(
-        [&](auto&& f) { for (int i = threadIdx.x; i < n; i += kSelThreads) f(keys[i]); }, static_cast<uint32_t>(k), rank, 2);
+        [&](auto&& f) {
+            for (int i = threadIdx.x; i < n; i += kSelThreads)
+                if (keys[i] != 0xFFFFFFFFu) f(keys[i]);   // bursts that were not visited do not widen the range
+        },
+        static_cast<uint32_t>(k), rank, 2);
     if (threadIdx.x == 0) {
         if (eps) {
             float f = ord_to_float(kth);
@@ -254,15 +258,21 @@ kth_threshold_warp_kernel(const uint32_t* mins, int stride, int n, int nq, int k
     }
     uint32_t v[NPL];
     const uint32_t* row = mins + static_cast<int64_t>(q) * stride;
-    uint32_t all_and = 0xFFFFFFFFu, all_or = 0u;
+    uint32_t all_and = 0xFFFFFFFFu, all_or = 0u, real = 0u;
 #pragma unroll
     for (int j = 0; j < NPL; ++j) {
         const int i = j * 32 + lane;
         v[j] = i < n ? row[i] : 0xFFFFFFFFu;
-        if (i < n) {
+        if (v[j] != 0xFFFFFFFFu) {   // (bursts that were not visited do not widen the range)
             all_and &= v[j];
             all_or |= v[j];
+            ++real;
         }
+    }
+    real = __reduce_add_sync(0xffffffffu, real);
+    if (real < static_cast<uint32_t>(k)) {
+        if (lane == 0) store_tau(q, tau_all, tau, fold);
+        return;
     }
     all_and = __reduce_and_sync(0xffffffffu, all_and);
     all_or = __reduce_or_sync(0xffffffffu, all_or);
