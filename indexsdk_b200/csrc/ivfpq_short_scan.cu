@@ -28,6 +28,10 @@
 
 #include <algorithm>
 
+#include "block_rank.cuh"
+#include "common.cuh"
+#include "ivfpq_exact.cuh"
+
 namespace b200 {
 namespace {
 
@@ -35,7 +39,8 @@ constexpr int kKsub = 256;
 constexpr int kBoundThreads = 1024;
 constexpr int kBins = 4096;
 constexpr int kScanThreadsShort = 1024;
-constexpr int kSelThreadsShort = 512;
+constexpr int kWideThreads = 384;
+constexpr int kSelThreadsShort = 256;
 constexpr int kSortMax = 2048;           // pairs sorted in shared memory
 constexpr float kPadDist = 3.402823466e+38f;
 constexpr int64_t kNoLabel = 0x7fffffffffffffffll;
@@ -85,6 +90,9 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* warp_t
 
 // ---- 1. table and bound ----
 template <int M>
+__host__ __device__ constexpr bool wide() { return M % 16 == 0; }   // rotated codes, 16 columns per table row
+
+template <int M>
 __global__ void __launch_bounds__(kBoundThreads)
 short_bound_kernel(const ShortScanArgs a) {
     extern __shared__ __align__(16) float bound_sm[];
@@ -127,8 +135,9 @@ short_bound_kernel(const ShortScanArgs a) {
     }
     __syncthreads();
     for (int i = tid; i < M * kKsub; i += kBoundThreads) {
-        const int m = i / kKsub;
-        const float* cw = a.codebooks + static_cast<int64_t>(i) * a.dsub;
+        // entry i of the table: sub-quantizer m, its codeword (rotated codes: [M / 16][256][16])
+        const int m = wide<M>() ? (i >> 12) * 16 + (i & 15) : i / kKsub;
+        const float* cw = (wide<M>() ? a.cbT : a.codebooks) + static_cast<int64_t>(i) * a.dsub;
         float e = 0.f;
         auto term = [&](int t, float c) {
             const float v = qs[m * a.dsub + t];
@@ -170,40 +179,80 @@ short_bound_kernel(const ShortScanArgs a) {
     {
         int p = 0;
         uint32_t lo = kInfBits, hi = 0u;
-        for (uint32_t i0 = tid; i0 < n1; i0 += 4 * kBoundThreads) {
-            uint32_t w[4][M / 4];
-            float t[4];
+        if constexpr (!wide<M>()) {
+            for (uint32_t i0 = tid; i0 < n1; i0 += 4 * kBoundThreads) {
+                uint32_t w[4][M / 4];
+                float t[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {   // four vectors' loads in flight
-                const uint32_t i = i0 + j * kBoundThreads;
-                t[j] = 0.f;
+                for (int j = 0; j < 4; ++j) {   // four vectors' loads in flight
+                    const uint32_t i = i0 + j * kBoundThreads;
+                    t[j] = 0.f;
 #pragma unroll
-                for (int g = 0; g < M / 4; ++g) w[j][g] = 0u;
-                if (i < n1) {
-                    while (pre[p + 1] <= i) ++p;
-                    const uint32_t pos = beg[p] + (i - pre[p]);
-                    if (a.by_residual) t[j] = base[p] + __ldg(a.t2 + pos);
-                    if (M == 4) {
-                        w[j][0] = __ldg(reinterpret_cast<const uint32_t*>(a.codes) + pos);
-                    } else {
-                        const uint2 c = __ldg(reinterpret_cast<const uint2*>(a.codes) + pos);
-                        w[j][0] = c.x;
-                        w[j][M / 4 - 1] = c.y;
+                    for (int g = 0; g < M / 4; ++g) w[j][g] = 0u;
+                    if (i < n1) {
+                        while (pre[p + 1] <= i) ++p;
+                        const uint32_t pos = beg[p] + (i - pre[p]);
+                        if (a.by_residual) t[j] = base[p] + __ldg(a.t2 + pos);
+                        if (M == 4) {
+                            w[j][0] = __ldg(reinterpret_cast<const uint32_t*>(a.codes) + pos);
+                        } else {
+                            const uint2 c = __ldg(reinterpret_cast<const uint2*>(a.codes) + pos);
+                            w[j][0] = c.x;
+                            w[j][M / 4 - 1] = c.y;
+                        }
                     }
                 }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t i = i0 + j * kBoundThreads;
+                    if (i >= n1) break;
+                    float acc = t[j];
+#pragma unroll
+                    for (int m = 0; m < M; ++m) acc = acc + tab[m * kKsub + ((w[j][m >> 2] >> (8 * (m & 3))) & 255u)];
+                    // (NaN becomes 0: a query that holds one collects nothing in the scan)
+                    const uint32_t b = __float_as_uint(fmaxf(acc, 0.f));
+                    dist[i] = b;
+                    lo = min(lo, b);
+                    hi = max(hi, b);
+                }
             }
+        } else {
+            constexpr int U = M <= 16 ? 4 : (M <= 32 ? 2 : 1);   // vectors whose codes are in flight
+            for (uint32_t i0 = tid; i0 < n1; i0 += U * kBoundThreads) {
+                uint4 c[U][M / 16 > 0 ? M / 16 : 1];
+                float acc[U];
+                uint32_t pos[U];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t i = i0 + j * kBoundThreads;
-                if (i >= n1) break;
-                float acc = t[j];
+                for (int j = 0; j < U; ++j) {
+                    const uint32_t i = i0 + j * kBoundThreads;
+                    acc[j] = 0.f;
+                    pos[j] = 0u;
+                    if (i < n1) {
+                        while (pre[p + 1] <= i) ++p;
+                        pos[j] = beg[p] + (i - pre[p]);
+                        if (a.by_residual) acc[j] = base[p] + __ldg(a.t2 + pos[j]);
+                    }
 #pragma unroll
-                for (int m = 0; m < M; ++m) acc = acc + tab[m * kKsub + ((w[j][m >> 2] >> (8 * (m & 3))) & 255u)];
-                // (NaN becomes 0: a query that holds one collects nothing in the scan)
-                const uint32_t b = __float_as_uint(fmaxf(acc, 0.f));
-                dist[i] = b;
-                lo = min(lo, b);
-                hi = max(hi, b);
+                    for (int g = 0; g < M / 16; ++g)
+                        c[j][g] = i < n1 ? __ldg(reinterpret_cast<const uint4*>(a.codes + static_cast<size_t>(pos[j]) * M) + g)
+                                         : make_uint4(0u, 0u, 0u, 0u);
+                }
+#pragma unroll
+                for (int j = 0; j < U; ++j) {
+                    const uint32_t i = i0 + j * kBoundThreads;
+                    if (i >= n1) break;
+#pragma unroll
+                    for (int g = 0; g < M / 16; ++g) {
+                        const uint32_t w[4] = {c[j][g].x, c[j][g].y, c[j][g].z, c[j][g].w};
+#pragma unroll
+                        for (int e = 0; e < 16; ++e)
+                            acc[j] += tab[(g * kKsub + ((w[e >> 2] >> (8 * (e & 3))) & 255u)) * 16 + ((e + pos[j]) & 15u)];
+                    }
+                    const uint32_t b = __float_as_uint(fmaxf(acc[j], 0.f));
+                    dist[i] = b;
+                    lo = min(lo, b);
+                    hi = max(hi, b);
+                }
             }
         }
         lo = __reduce_min_sync(0xffffffffu, lo);
@@ -284,7 +333,7 @@ short_bound_kernel(const ShortScanArgs a) {
         tb = min(kInfBits, lo_b + ((1u << shift) - 1u));   // (both below 2^31)
         // Thousands of vectors with one distance (equal codes): the ones with the smallest labels count, so
         // the r-th smallest label among those seen here bounds theirs.
-        if (!a.by_residual && shift == 0 && in > 1024u) {
+        if (!wide<M>() && !a.by_residual && shift == 0 && in > 1024u) {
             if (tid == 0) {
                 s_llo = ~0ull;
                 s_lhi = 0ull;
@@ -336,11 +385,16 @@ short_bound_kernel(const ShortScanArgs a) {
     }
     if (tid == 0) {
         float thr = __uint_as_float(tb);
+        // scanned distances of raw short codes are the canonical ones; the others are off by eps at most
+        float eps = 0.f;
         if (a.by_residual && tb != kInfBits) {
             const float coarse_max = a.cD[q * a.nprobe + a.nprobe - 1];
-            const float eps = a.err_rel * (fabsf(coarse_max) + a.t2_bound + 2.f * sqrtf(s_qn2) * a.cb_bound + thr);
-            thr = thr + 2.f * eps;
+            eps = a.err_rel * (fabsf(coarse_max) + a.t2_bound + 2.f * sqrtf(s_qn2) * a.cb_bound + thr);
+        } else if (wide<M>() && tb != kInfBits) {
+            eps = a.err_rel * thr;
         }
+        thr = thr + 2.f * eps;
+        a.eps[q] = eps;
         a.thr[q] = thr;
         a.label_max[q] = label_max;
     }
@@ -457,33 +511,128 @@ short_scan_kernel(const ShortScanArgs a, int S) {
                     if (lane == 0) slot = atomicAdd(a.count + q, static_cast<uint32_t>(__popc(bal)));
                     slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(bal & ((1u << lane) - 1u));
                     if (pass && slot < a.cap) {
-                        a.cand[q * a.cap + slot] = make_uint2(pos, RESID ? static_cast<uint32_t>(l) : __float_as_uint(acc[j][e]));
+                        a.cand[q * a.cap + slot] = make_uint2(pos, __float_as_uint(acc[j][e]));
+                        if (RESID) a.probe[q * a.cap + slot] = static_cast<uint16_t>(l);
                     }
                 }
         }
     }
 }
 
-// ---- 3. exact order ----
-// Canonical distance of a residual-encoded vector: sum over ascending m of |(q - c)_m - cb[m][code_m]|^2.
-__device__ __forceinline__ float canonical_residual(const ShortScanArgs& a, int64_t q, uint32_t pos, int64_t list) {
-    const uint8_t* code = a.codes + static_cast<size_t>(pos) * a.M;
-    const float* qv = a.xq + q * a.d;
-    const float* cen = a.centroids + list * a.d;
-    float acc = 0.f;
-    for (int m = 0; m < a.M; ++m) {
-        const float* cw = a.codebooks + (static_cast<int64_t>(m) * kKsub + code[m]) * a.dsub;
-        float e = 0.f;
-        for (int t = 0; t < a.dsub; ++t) {
-            const float r = __ldg(qv + m * a.dsub + t) - __ldg(cen + m * a.dsub + t);
-            const float df = r - __ldg(cw + t);
-            e = fmaf(df, df, e);
+// ---- 2'. scan of wide codes ----
+// The table of the wide-code filter (see ivfpq_index.cu): rows of 32 columns, the 16 sub-quantizers of a
+// group twice, lane l at sub-quantizer (s + l) mod 16 in step s, so that 32 lanes read 32 banks.  A lane
+// holds one vector; the codes of the next 32 vectors are on their way while 32 are looked up.
+template <int MT, bool RESID>
+__global__ void __launch_bounds__(kWideThreads, MT <= 3 ? 2 : 1)
+wide_scan_kernel(const ShortScanArgs a, int S) {
+    constexpr uint32_t U = 128;    // vectors of a unit
+    extern __shared__ __align__(16) float wide_sm[];
+    float* lut = wide_sm;                                                   // [MT][256][32]
+    uint32_t* upre = reinterpret_cast<uint32_t*>(lut + MT * kKsub * 32);    // [nprobe + 1] units before the probe
+    uint32_t* beg = upre + a.nprobe + 1;
+    uint32_t* len = beg + a.nprobe;
+    float* base = reinterpret_cast<float*>(len + a.nprobe);
+    __shared__ uint32_t s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lut_base = static_cast<uint32_t>(__cvta_generic_to_shared(lut));
+    uint32_t col[16];
+#pragma unroll
+    for (int s = 0; s < 16; ++s) col[s] = lut_base + 4u * (((s + lane) & 15) + (lane & 16));
+    const int64_t items = a.nq * S;
+    const int64_t it0 = items * blockIdx.x / gridDim.x, it1 = items * (blockIdx.x + 1) / gridDim.x;
+    int64_t cur_q = -1;
+    uint32_t units = 0;
+    float thr = 0.f;
+    const uint4* codes4 = reinterpret_cast<const uint4*>(a.codes);
+    for (int64_t it = it0; it < it1; ++it) {
+        const int64_t q = it / S;
+        const uint32_t split = static_cast<uint32_t>(it - q * S);
+        if (q != cur_q) {
+            __syncthreads();   // the previous query's table and probes are still read
+            cur_q = q;
+            const float4* src = reinterpret_cast<const float4*>(a.lut + q * (MT * 16 * kKsub));
+            for (int i = threadIdx.x; i < MT * kKsub * 4; i += kWideThreads) {
+                const float4 v = __ldg(src + i);
+                float4* row = reinterpret_cast<float4*>(lut) + (i >> 2) * 8 + (i & 3);
+                row[0] = v;
+                row[4] = v;
+            }
+            units = 0;
+            for (int p0 = 0; p0 < a.nprobe; p0 += kWideThreads) {
+                const int p = p0 + threadIdx.x;
+                Probe pr{0u, 0u, 0.f};
+                if (p < a.nprobe) pr = load_probe(a, q, p);
+                uint32_t sum;
+                const uint32_t ex = block_exclusive((pr.len + U - 1) / U, s_warp, &sum);
+                if (p < a.nprobe) {
+                    upre[p] = units + ex;
+                    beg[p] = pr.begin;
+                    len[p] = pr.len;
+                    base[p] = pr.base;
+                }
+                units += sum;
+            }
+            thr = a.thr[q];
+            __syncthreads();
         }
-        acc = acc + e;
+        const uint32_t u0 = static_cast<uint32_t>(static_cast<uint64_t>(units) * split / S);
+        const uint32_t u1 = static_cast<uint32_t>(static_cast<uint64_t>(units) * (split + 1) / S);
+        for (uint32_t u = u0 + warp; u < u1; u += kWideThreads / 32) {
+            int l = 0, h = a.nprobe;   // last probe with upre[p] <= u: the one that holds unit u
+            while (h - l > 1) {
+                const int mid = (l + h) >> 1;
+                if (upre[mid] <= u) l = mid;
+                else h = mid;
+            }
+            const uint32_t first = (u - upre[l]) * U, n = len[l], pos0 = beg[l];
+            const float bias = RESID ? base[l] : 0.f;
+            const uint32_t last = min(first + U, n);
+            uint4 c[MT], d[MT];
+            float t = 0.f, tn = 0.f;
+            // (lists are stored padded to 32 vectors: the loads stay inside the list)
+            auto fetch = [&](uint32_t i, uint4 (&dst)[MT], float& t2) {
+                const size_t v = pos0 + i + lane;
+#pragma unroll
+                for (int g = 0; g < MT; ++g) dst[g] = __ldg(codes4 + v * MT + g);
+                if (RESID) t2 = __ldg(a.t2 + v);
+            };
+            auto process = [&](uint32_t i, const uint4 (&cc)[MT], float t2) {
+                float acc = RESID ? bias + t2 : 0.f;
+#pragma unroll
+                for (int g = 0; g < MT; ++g) {
+                    const uint32_t w[4] = {cc[g].x, cc[g].y, cc[g].z, cc[g].w};
+#pragma unroll
+                    for (int s = 0; s < 16; ++s) {
+                        const uint32_t addr = __byte_perm(w[s >> 2], 0u, 0x4440u + (s & 3)) * 128u + col[s];
+                        float val;
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(val) : "r"(addr + static_cast<uint32_t>(g) * (kKsub * 32 * 4)));
+                        acc = acc + val;
+                    }
+                }
+                const bool pass = i + lane < n && acc <= thr;
+                const unsigned bal = __ballot_sync(0xffffffffu, pass);
+                if (!bal) return;
+                uint32_t slot = 0;
+                if (lane == 0) slot = atomicAdd(a.count + q, static_cast<uint32_t>(__popc(bal)));
+                slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(bal & ((1u << lane) - 1u));
+                if (pass && slot < a.cap) {
+                    a.cand[q * a.cap + slot] = make_uint2(pos0 + i + lane, __float_as_uint(acc));
+                    if (RESID) a.probe[q * a.cap + slot] = static_cast<uint16_t>(l);
+                }
+            };
+            fetch(first, c, t);
+            for (uint32_t i = first; i < last; i += 64) {
+                if (i + 32 < last) fetch(i + 32, d, tn);
+                process(i, c, t);
+                if (i + 64 < last) fetch(i + 64, c, t);
+                if (i + 32 < last) process(i + 32, d, tn);
+            }
+        }
     }
-    return acc;
 }
 
+// ---- 3. exact order ----
 // Rank search over unsigned keys of `bits` bits, eight at a time; key(i, &v) says whether entry i takes
 // part.  Returns the r-th smallest (1-based); *left = rank among the entries equal to it.
 template <typename KeyT, typename F>
@@ -514,7 +663,7 @@ __device__ KeyT block_kth(F key, uint32_t n, uint32_t r, uint32_t* hist, uint32_
     return prefix;
 }
 
-__global__ void __launch_bounds__(kSelThreadsShort)
+__global__ void __launch_bounds__(kSelThreadsShort, 3)
 short_select_kernel(const ShortScanArgs a) {
     __shared__ __align__(16) int64_t sl[kSortMax];
     __shared__ float sd[kSortMax];
@@ -526,16 +675,58 @@ short_select_kernel(const ShortScanArgs a) {
         return;
     }
     uint2* row = a.cand + q * a.cap;
-    if (a.by_residual) {
+    const uint32_t k = static_cast<uint32_t>(a.k);
+    if (a.by_residual || a.rotated) {
+        // Scanned distances are off by eps at most: k of them lie at or below their k-th smallest, so whatever
+        // exceeds that by more than 2 eps is out (marked 0xFFFFFFFF); the others get their canonical distance.
+        __shared__ RankScratch rank;
+        const uint32_t kth_scan = block_kth32<kSelThreadsShort>(
+            [&](auto&& f) { for (uint32_t i = threadIdx.x; i < n; i += kSelThreadsShort) f(float_to_ord(__uint_as_float(row[i].y))); },
+            k, rank, 2);
+        float lim = __uint_as_float(kInfBits);   // fewer than k: all of them
+        if (kth_scan != 0xFFFFFFFFu) {
+            lim = ord_to_float(kth_scan) + 2.f * a.eps[q];
+            lim = lim + fabsf(lim) * 9.5367431640625e-07f;   // the rounding of the sum
+            if (!(lim <= __uint_as_float(kInfBits))) lim = __uint_as_float(kInfBits);
+        }
+        // survivors first, so that full warps work on them (sl doubles as their list)
+        uint32_t* live = reinterpret_cast<uint32_t*>(sl);
+        if (threadIdx.x == 0) s_fill = 0u;
+        __syncthreads();
         for (uint32_t i = threadIdx.x; i < n; i += kSelThreadsShort) {
-            const uint2 c = row[i];
-            const int64_t list = a.cI[q * a.nprobe + c.y];
-            row[i].y = __float_as_uint(canonical_residual(a, q, c.x, list));
+            if (__uint_as_float(row[i].y) <= lim) {
+                const uint32_t slot = atomicAdd(&s_fill, 1u);
+                if (slot < 2u * kSortMax) live[slot] = i;
+            }
         }
         __syncthreads();
+        const uint32_t nl = s_fill;
+        const bool listed = nl <= 2u * kSortMax;
+        auto refine = [&](uint32_t i) {
+            const uint2 c = row[i];
+            const int64_t list = a.by_residual ? a.cI[q * a.nprobe + a.probe[q * a.cap + i]] : 0;
+            return __float_as_uint(exact_distance(a, q, c.x, list));
+        };
+        if (listed) {
+            uint32_t* val = reinterpret_cast<uint32_t*>(sd);   // [kSortMax]: results wait there until the others are marked
+            for (uint32_t j0 = 0; j0 < nl; j0 += kSortMax) {
+                const uint32_t j1 = min(nl, j0 + kSortMax);
+                for (uint32_t j = j0 + threadIdx.x; j < j1; j += kSelThreadsShort) val[j - j0] = refine(live[j]);
+                __syncthreads();
+                if (j0 == 0)
+                    for (uint32_t i = threadIdx.x; i < n; i += kSelThreadsShort)
+                        if (!(__uint_as_float(row[i].y) <= lim)) row[i].y = 0xFFFFFFFFu;
+                __syncthreads();
+                for (uint32_t j = j0 + threadIdx.x; j < j1; j += kSelThreadsShort) row[live[j]].y = val[j - j0];
+                __syncthreads();
+            }
+        } else {
+            for (uint32_t i = threadIdx.x; i < n; i += kSelThreadsShort)
+                row[i].y = __uint_as_float(row[i].y) <= lim ? refine(i) : 0xFFFFFFFFu;
+            __syncthreads();
+        }
     }
-    const uint32_t k = static_cast<uint32_t>(a.k);
-    auto dist_key = [&](uint32_t i, uint32_t& v) { v = row[i].y; return true; };
+    auto dist_key = [&](uint32_t i, uint32_t& v) { v = row[i].y; return v != 0xFFFFFFFFu; };
     // Distances are >= 0: their bits order like the values.  All candidates when they fit the sort, else
     // those below the k-th distance and as many of the ties with it as there is room for -- the ones with
     // the smallest labels when there are more.
@@ -570,7 +761,7 @@ short_select_kernel(const ShortScanArgs a) {
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < n; i += kSelThreadsShort) {
         const uint2 c = row[i];
-        if (c.y > kth) continue;
+        if (c.y > kth || c.y == 0xFFFFFFFFu) continue;
         const int64_t label = a.ids[c.x];
         if (c.y == kth) {
             const uint64_t u = static_cast<uint64_t>(label) ^ (1ull << 63);
@@ -633,12 +824,38 @@ cudaError_t launch_m(const ShortScanArgs& a, int num_sms, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+template <int M>
+cudaError_t launch_wide(const ShortScanArgs& a, int num_sms, cudaStream_t st) {
+    constexpr int MT = M / 16;
+    const size_t bound_smem = static_cast<size_t>(M * kKsub + kBins + 3 * kShortMaxProbe + 1 + a.d + a.n1_max) * 4;
+    cudaError_t e = cudaFuncSetAttribute(short_bound_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bound_smem));
+    if (e != cudaSuccess) return e;
+    short_bound_kernel<M><<<static_cast<unsigned>(a.nq), kBoundThreads, bound_smem, st>>>(a);
+    const size_t smem = static_cast<size_t>(MT * kKsub * 32 + 4 * a.nprobe + 1) * 4;
+    auto kern = a.by_residual ? wide_scan_kernel<MT, true> : wide_scan_kernel<MT, false>;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWideThreads, smem);
+    if (e != cudaSuccess) return e;
+    const int64_t blocks = static_cast<int64_t>(num_sms) * std::max(1, per_sm);
+    // shares as in launch_m
+    const int S = static_cast<int>(std::max<int64_t>(1, (4LL * blocks + a.nq - 1) / a.nq));
+    kern<<<static_cast<unsigned>(std::min<int64_t>(blocks, a.nq * S)), kWideThreads, smem, st>>>(a, S);
+    short_select_kernel<<<static_cast<unsigned>(a.nq), kSelThreadsShort, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_short_scan(const ShortScanArgs& a, int num_sms, cudaStream_t st) {
     switch (a.M) {
         case 4: return launch_m<4>(a, num_sms, st);
         case 8: return launch_m<8>(a, num_sms, st);
+        case 16: return launch_wide<16>(a, num_sms, st);
+        case 32: return launch_wide<32>(a, num_sms, st);
+        case 48: return launch_wide<48>(a, num_sms, st);
+        case 64: return launch_wide<64>(a, num_sms, st);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -1,4 +1,4 @@
-// IVFPQ scan for short codes (M = 4 or 8 bytes), see ivfpq_short_scan.cu.
+// IVFPQ scan with a bound, for short codes (M = 4 or 8 bytes) and for large k, see ivfpq_short_scan.cu.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -6,7 +6,7 @@
 namespace b200 {
 
 constexpr int kShortMaxProbe = 1024;     // probes whose metadata a block stages in shared memory
-constexpr uint32_t kShortMaxBound = 32768;   // vectors the bound is taken from
+constexpr uint32_t kShortMaxBound = 16384;   // vectors the bound is taken from (wide codes: half as many)
 constexpr uint32_t kShortMaxCap = 32768; // candidates a query may collect; more take the exact scan
 
 struct ShortScanArgs {
@@ -16,20 +16,24 @@ struct ShortScanArgs {
     int64_t nq;
     const int64_t* offsets;  // [nlist + 1] first position of every list (multiples of 32)
     const int64_t* lens;     // [nlist]
-    const uint8_t* codes;    // [positions][M], not rotated
+    const uint8_t* codes;    // [positions][M]
+    int rotated;             // M = 16, 32, 48, 64: bytes of a 16-byte group rotated by the position
     const int64_t* ids;
     const float* t2;         // residual encoding: the per-vector term
     int by_residual;
     const float* xq;         // [nq][d]
     const float* centroids;  // [nlist][d]
     const float* codebooks;  // [M][256][dsub]
+    const float* cbT;        // rotated codes: regrouped [M / 16][256][16][dsub]
     float err_rel, t2_bound, cb_bound;   // filter error bound of residual encoding (see IvfpqIndex::search_stages)
     // scratch
-    float* lut;              // [nq][M][256]
+    float* lut;              // [nq][M][256], rotated codes [nq][M / 16][256][16]
+    float* eps;              // [nq] error of a scanned distance that matters
     float* thr;              // [nq] collect below ...
     uint64_t* label_max;     // [nq] ... and at it the labels up to this one (sign bit flipped; raw encoding)
     uint32_t* count;         // [nq]
-    uint2* cand;             // [nq][cap] (position, distance bits | probe)
+    uint2* cand;             // [nq][cap] (position, distance bits)
+    uint16_t* probe;         // [nq][cap] which probe (residual encoding)
     uint32_t cap;
     uint32_t n1_max;         // most vectors a query's bound is taken from (shared memory of that kernel)
     // results
@@ -49,6 +53,23 @@ inline bool use_short_scan(int M, bool residual, double visited, int nprobe, int
     if ((M != 4 && M != 8) || nprobe > kShortMaxProbe || k > 1024) return false;
     if (residual && nprobe > 1) return true;
     return visited * M >= (residual || k > 64 ? 4096.0 : 32768.0);
+}
+// Wide codes (M = 16, 32, 48, 64): sorted lists in registers are a good filter while they are short (k' = 32 or
+// 64, k <= 48) and the batch is large; otherwise the insertions, or the one block per query and split, cost
+// more than the bound does.  nq queries, us before / this way (1 M vectors, residual codes):
+//   k = 100, 3 900 vectors visited, 512 queries: M = 16 230 / 168, M = 64 424 / 246; k = 300: 1 149 / 199, 1 661 / 280
+//   k = 100, 31 000, 2 048 queries: M = 16 861 / 650, M = 32 1 471 / 894, M = 48 1 795 / 1 209, M = 64 3 333 / 1 653
+//   k = 10,  3 900, 64 queries: M = 32 108 / 106, M = 64 123 / 112;   512 queries: M = 32 148 / 179, M = 64 220 / 246
+//   k = 10,  31 000, 512 queries: M = 32 427 / 307, M = 48 497 / 414, M = 64 831 / 501
+//   k = 10,  31 000, 2 048 queries: M = 16 375 / 645, M = 32 859 / 886, M = 48 1 036 / 1 202, M = 64 2 020 / 1 646
+// Below about 2 000 vectors a query the bound is not worth its launch.  16-byte codes with k <= 48 stay with the
+// lists: their tables are small, and the persistent kernel takes over from 1 184 queries on.
+inline bool use_bounded_scan(int M, double visited, int nprobe, int k, int64_t nq) {
+    if (M % 16 != 0 || M > 64 || k > 1024 || nprobe > kShortMaxProbe || visited < 2048.0) return false;
+    if (k > 48) return true;
+    if (M == 16) return false;
+    if (nq <= 64) return true;
+    return visited >= 16384.0 && (nq <= 1024 || M == 64);
 }
 cudaError_t launch_short_scan(const ShortScanArgs& a, int num_sms, cudaStream_t st);
 
