@@ -1,6 +1,7 @@
-// IVFPQ scan for short codes: M = 4 or 8 bytes a vector.
+// IVFPQ scan with a bound: short codes (M = 4 or 8 bytes a vector), and wide ones (M = 16, 32, 48, 64, whose
+// groups of 16 bytes are stored rotated by the position) where sorted lists are the slower filter.
 //
-// The lookups of such a code are few (4 or 8), so neither the 16-column tables of the wide-code scan
+// The lookups of a short code are few (4 or 8), so neither the 16-column tables of the wide-code scan
 // nor its sorted lists in registers pay: with k = 300 the insertions into a warp's list of 512 pairs
 // are a chain that costs far more than the lookups.  Instead the k-th distance is bounded first and
 // everything under the bound is collected:
@@ -16,14 +17,17 @@
 //        query's candidate row.
 //   3  short_select_kernel: one block per query, exact order by (distance, label).
 // Raw encoding: the table holds the canonical |q_m - cb|^2 and they are added in ascending m, so the
-// scanned distances ARE the canonical ones.  Residual encoding scans |q-c|^2 + t2 - 2 q.cb, widens the
-// bound by twice its error and computes the canonical distance of the collected vectors.
+// scanned distances ARE the canonical ones.  Residual encoding scans |q-c|^2 + t2 - 2 q.cb, and wide codes add
+// in the order of their rotation: there the bound is widened by twice the error, and the collected vectors
+// within twice the error of the k-th get their canonical distance.
+// Wide codes: wide_scan_kernel takes the place of short_scan_kernel, with the table rows of the wide-code filter
+// (ivfpq_index.cu); what they measured stands at use_bounded_scan.
 // A query with more than `cap` vectors under its bound (tens of thousands of equal codes) is flagged
 // and scanned exactly by the caller.
 // What bounds it (64 queries, 10 M vectors, M = 4, 64 of 1024 lists, k = 300; the exact scan this
-// replaces took 2.14 ms): the bound takes 63 us (64 blocks, one after the
-// other step inside), the scan 65 (issue slots: about 40 instructions a vector, and two table fills per block),
-// the order 15; the whole call 2.80 -> 0.25 ms.
+// replaces took 2.14 ms): the bound takes 41 us (64 blocks, one step
+// after the other inside), the scan 65 (issue slots: about 40 instructions a vector, and two table fills per
+// block), the order 20; the whole call 2.77 -> 0.23 ms.
 #include "ivfpq_short_scan.cuh"
 
 #include <algorithm>
@@ -36,7 +40,6 @@ namespace b200 {
 namespace {
 
 constexpr int kKsub = 256;
-constexpr int kBoundThreads = 1024;
 constexpr int kBins = 4096;
 constexpr int kScanThreadsShort = 1024;
 constexpr int kWideThreads = 384;
@@ -91,10 +94,15 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* warp_t
 // ---- 1. table and bound ----
 template <int M>
 __host__ __device__ constexpr bool wide() { return M % 16 == 0; }   // rotated codes, 16 columns per table row
+// Threads of the bound's block: wide codes need 44 registers and up to 110 KB, so two blocks of 512 share an SM
+// where one of 1 024 would have it alone (1 000 queries, M = 48: 121 -> 103 us).
+template <int M>
+__host__ __device__ constexpr int bound_threads() { return wide<M>() ? 512 : 1024; }
 
 template <int M>
-__global__ void __launch_bounds__(kBoundThreads)
+__global__ void __launch_bounds__(bound_threads<M>())
 short_bound_kernel(const ShortScanArgs a) {
+    constexpr int kBoundThreads = bound_threads<M>();
     extern __shared__ __align__(16) float bound_sm[];
     float* tab = bound_sm;                                                  // [M][256]
     uint32_t* hist = reinterpret_cast<uint32_t*>(tab + M * kKsub);          // [kBins]
@@ -810,7 +818,7 @@ cudaError_t launch_m(const ShortScanArgs& a, int num_sms, cudaStream_t st) {
     const size_t bound_smem = static_cast<size_t>(M * kKsub + kBins + 3 * kShortMaxProbe + 1 + a.d + a.n1_max) * 4;
     cudaError_t e = cudaFuncSetAttribute(short_bound_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bound_smem));
     if (e != cudaSuccess) return e;
-    short_bound_kernel<M><<<static_cast<unsigned>(a.nq), kBoundThreads, bound_smem, st>>>(a);
+    short_bound_kernel<M><<<static_cast<unsigned>(a.nq), bound_threads<M>(), bound_smem, st>>>(a);
     // About eight shares per block: the blocks' loads differ by one share at most, and a block
     // changes queries (128 KB of table to fill) as seldom as the batch allows.
     const int S = static_cast<int>(std::max<int64_t>(1, (8LL * num_sms + a.nq - 1) / a.nq));
@@ -830,7 +838,7 @@ cudaError_t launch_wide(const ShortScanArgs& a, int num_sms, cudaStream_t st) {
     const size_t bound_smem = static_cast<size_t>(M * kKsub + kBins + 3 * kShortMaxProbe + 1 + a.d + a.n1_max) * 4;
     cudaError_t e = cudaFuncSetAttribute(short_bound_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bound_smem));
     if (e != cudaSuccess) return e;
-    short_bound_kernel<M><<<static_cast<unsigned>(a.nq), kBoundThreads, bound_smem, st>>>(a);
+    short_bound_kernel<M><<<static_cast<unsigned>(a.nq), bound_threads<M>(), bound_smem, st>>>(a);
     const size_t smem = static_cast<size_t>(MT * kKsub * 32 + 4 * a.nprobe + 1) * 4;
     auto kern = a.by_residual ? wide_scan_kernel<MT, true> : wide_scan_kernel<MT, false>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
