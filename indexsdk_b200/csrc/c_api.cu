@@ -113,7 +113,7 @@ struct MultiScratch {
     std::mutex mu;           // held for a whole multi-index search that uses this device
     DeviceBuffer q, D, I, allD, allI, mD, mI, gD, gI;
     PinnedBuffer hq, hD, hI;
-    std::unique_ptr<FlatGroup> group;   // concatenated copy of the small Flat indexes searched together last
+    std::unique_ptr<FlatGroup> group;   // tables of the small Flat indexes searched together last
 };
 MultiScratch& multi_scratch(int device) {
     static std::mutex table_mu;
@@ -320,7 +320,7 @@ int b200idx_search_multi(b200idx_t* const* hs, int nh, int64_t n, const void* x,
                     cudaStream_t st = static_cast<cudaStream_t>(b200idx_stream(hs[members[0]]));
                     upload_small(dq, x, static_cast<size_t>(n) * row, sc.hq, st);
                     // Small exact indexes of one device are searched in ONE pass over their
-                    // concatenated bases (segmented search): launches do not grow with their number.
+                    // bases (segmented search): launches do not grow with their number.
                     std::vector<FlatIndex*> fm;
                     bool groupable = members.size() >= 2 && hs[members[0]]->kind != 2;
                     for (size_t j = 0; groupable && j < members.size(); ++j) {

@@ -84,12 +84,12 @@ struct GemmArgs {
     // lets the row take part (nullptr: every row does)
     const uint32_t* qmask;
     int64_t qmask_stride;
-    // optional segmented base: the concatenated bases of several indexes that are searched with the
+    // optional segmented base: several indexes in one common space of positions that are searched with the
     // same queries in ONE pass (multi-index search).  A tile belongs to exactly one index (segments
     // start on tile boundaries); per tile:
     //   seg_index: which index; the candidates of (index i, query q) go to row
     //              (i - seg_first) * nq + q of cand / tau (direct mode only)
-    //   seg_col0 : position of the index's first base row in the concatenated base (the slot of a
+    //   seg_col0 : position of the index's first base row (the slot of a
     //              candidate is its position minus this; burst minima count their slots from it too)
     //   seg_end  : position one past the index's last real base row
     // With thresholds (direct = 0) tau, counts, cand and mins are per candidate row.  Folded operands

@@ -81,6 +81,7 @@ int FlatIndex::gemm_kind() const {
 
 void FlatIndex::reserve(int64_t n) {
     if (n <= cap_rows_) return;
+    generation_ = next_generation();   // the rows move: tables that point at them are out of date even if the add fails
     int64_t want = std::max<int64_t>(n, cap_rows_ + cap_rows_ / 2);
     want = round_up(want, kTileB);
     const size_t row_op = static_cast<size_t>(op_cols()) * op_elem_bytes();

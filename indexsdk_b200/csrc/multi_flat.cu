@@ -11,7 +11,7 @@ namespace {
 
 constexpr int64_t kMaxMemberRows = 65536;                 // larger members use the thresholded pipeline of their own
 constexpr size_t kGroupCandBytes = size_t(2) << 30;       // candidate scratch per pass
-constexpr size_t kGroupBaseBytes = size_t(8) << 30;       // concatenated copy
+constexpr size_t kGroupBaseBytes = size_t(8) << 30;       // operand, norms and exact rows of all members
 inline int64_t pad_tile(int64_t n) { return (n + kTileB - 1) / kTileB * kTileB; }
 inline size_t op_elem(int dtype) { return dtype == kI8 ? 1 : 2; }
 

@@ -969,7 +969,7 @@ __device__ __forceinline__ int warp_sum_i(int v) {
 }
 
 // Query operand rows of d + kFoldCols bf16: the query, three ones (they pick up the base row's
-// folded norm), three zeros (the threshold terms, written by fold_tau_kernel once the threshold is
+// folded norm), three zeros (the threshold terms, written by store_tau once the threshold is
 // known) and zero padding.
 __global__ void prep_queries_f32_kernel(const float* xq, int nq, int d, int metric, float ymax,
                                         __nv_bfloat16* qb, float* qnorm, float* eps) {
