@@ -49,6 +49,7 @@
 #include "ivfpq_tc_scan.cuh"
 #include "kmeans.h"
 #include "ptx_sm100.cuh"
+#include "smem_limit.h"
 #include "select.cuh"
 
 namespace b200 {
@@ -1573,13 +1574,6 @@ ivfpq_collect_refine_kernel(const ScanArgs a, const uint32_t* cpos, const uint32
     if (threadIdx.x == 0) a.flag[q] = 0;
 }
 
-template <typename Kern>
-cudaError_t set_smem(Kern kern, size_t smem) {
-    if (smem > 48 * 1024)
-        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    return cudaSuccess;
-}
-
 constexpr int fast_scan_threads(int mt) { return mt >= 2 ? 256 : 128; }
 
 template <int MT>
@@ -1591,7 +1585,7 @@ cudaError_t launch_fast_mt(const ScanArgs& a, int kpt, cudaStream_t st) {
 #define B200_FAST_CASE(KP)                                           \
     case KP: {                                                       \
         auto kern = ivfpq_fast_scan_kernel<MT, KP, NT>;              \
-        cudaError_t e = set_smem(kern, smem);                        \
+        cudaError_t e = allow_max_smem(kern);                        \
         if (e != cudaSuccess) return e;                              \
         kern<<<grid, NT, smem, st>>>(a);                             \
         return cudaGetLastError();                                   \
@@ -1646,7 +1640,7 @@ cudaError_t launch_exact(const ScanArgs& a, int nq_launch, cudaStream_t st) {
 #define B200_EXACT_CASE(KP)                                          \
     case KP: {                                                       \
         auto kern = ivfpq_exact_scan_kernel<KP>;                     \
-        cudaError_t e = set_smem(kern, smem);                        \
+        cudaError_t e = allow_max_smem(kern);                        \
         if (e != cudaSuccess) return e;                              \
         kern<<<nq_launch, kScanThreads, smem, st>>>(a);              \
         return cudaGetLastError();                                   \
@@ -1670,7 +1664,7 @@ cudaError_t launch_collect(const ScanArgs& a, int nslots, uint32_t* cpos, uint32
 #define B200_COLLECT_CASE(MTV)                                                \
     case MTV: {                                                               \
         auto kern = ivfpq_collect_kernel<MTV>;                                \
-        e = set_smem(kern, smem);                                             \
+        e = allow_max_smem(kern);                                             \
         if (e != cudaSuccess) return e;                                       \
         kern<<<nslots, kScanThreads, smem, st>>>(a, cpos, ccount);            \
         break;                                                                \
@@ -2481,7 +2475,7 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
             if (S * kprime == 32 && k <= 32 && nprobe <= kRefMaxProbe) {
                 ivfpq_refine_warp_kernel<<<blocks_for(m, kRefWarpsPerBlock), kRefWarpsPerBlock * 32, 0, st>>>(a);
             } else {
-                B200_CUDA_CHECK(set_smem(ivfpq_refine_kernel, rsmem));
+                B200_CUDA_CHECK(allow_max_smem(ivfpq_refine_kernel));
                 ivfpq_refine_kernel<<<static_cast<unsigned>(m), kScanThreads, rsmem, st>>>(a, P);
             }
             B200_CUDA_CHECK(cudaGetLastError());

@@ -35,6 +35,7 @@
 #include "block_rank.cuh"
 #include "common.cuh"
 #include "ivfpq_exact.cuh"
+#include "smem_limit.h"
 
 namespace b200 {
 namespace {
@@ -816,7 +817,7 @@ short_select_kernel(const ShortScanArgs a) {
 template <int M>
 cudaError_t launch_m(const ShortScanArgs& a, int num_sms, cudaStream_t st) {
     const size_t bound_smem = static_cast<size_t>(M * kKsub + kBins + 3 * kShortMaxProbe + 1 + a.d + a.n1_max) * 4;
-    cudaError_t e = cudaFuncSetAttribute(short_bound_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bound_smem));
+    cudaError_t e = allow_max_smem(short_bound_kernel<M>);
     if (e != cudaSuccess) return e;
     short_bound_kernel<M><<<static_cast<unsigned>(a.nq), bound_threads<M>(), bound_smem, st>>>(a);
     // About eight shares per block: the blocks' loads differ by one share at most, and a block
@@ -825,7 +826,7 @@ cudaError_t launch_m(const ShortScanArgs& a, int num_sms, cudaStream_t st) {
     const int grid = static_cast<int>(std::min<int64_t>(num_sms, a.nq * S));
     const size_t scan_smem = static_cast<size_t>(M * kKsub * replicas<M>() + 4 * kShortMaxProbe + 1) * 4;
     auto kern = a.by_residual ? short_scan_kernel<M, true> : short_scan_kernel<M, false>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(scan_smem));
+    e = allow_max_smem(kern);
     if (e != cudaSuccess) return e;
     kern<<<grid, kScanThreadsShort, scan_smem, st>>>(a, S);
     short_select_kernel<<<static_cast<unsigned>(a.nq), kSelThreadsShort, 0, st>>>(a);
@@ -836,12 +837,12 @@ template <int M>
 cudaError_t launch_wide(const ShortScanArgs& a, int num_sms, cudaStream_t st) {
     constexpr int MT = M / 16;
     const size_t bound_smem = static_cast<size_t>(M * kKsub + kBins + 3 * kShortMaxProbe + 1 + a.d + a.n1_max) * 4;
-    cudaError_t e = cudaFuncSetAttribute(short_bound_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bound_smem));
+    cudaError_t e = allow_max_smem(short_bound_kernel<M>);
     if (e != cudaSuccess) return e;
     short_bound_kernel<M><<<static_cast<unsigned>(a.nq), bound_threads<M>(), bound_smem, st>>>(a);
     const size_t smem = static_cast<size_t>(MT * kKsub * 32 + 4 * a.nprobe + 1) * 4;
     auto kern = a.by_residual ? wide_scan_kernel<MT, true> : wide_scan_kernel<MT, false>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    e = allow_max_smem(kern);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWideThreads, smem);

@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "dist_gemm.cuh"
+#include "smem_limit.h"
 
 namespace b200 {
 namespace {
@@ -1143,7 +1144,7 @@ cudaError_t launch_select_emit(const uint64_t* cand, const uint32_t* counts, uin
     const uint32_t stage = large ? 12288u : 2048u;
     const size_t smem = (static_cast<size_t>(P) + stage) * sizeof(uint64_t);
     auto kern = large ? select_emit_kernel<512> : select_emit_kernel<kSelThreads>;
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t err = allow_max_smem(kern);
     if (err != cudaSuccess) return err;
     kern<<<e.nq, large ? 512 : kSelThreads, smem, stream>>>(cand, counts, n_fixed, cap, P, stage, overflow, any_overflow, e);
     return cudaGetLastError();
@@ -1155,7 +1156,7 @@ cudaError_t launch_finish_f32(const uint64_t* cand, const uint32_t* counts, uint
     if (e.nq <= 0 || e.k <= 0) return cudaSuccess;
     if (few && e.k <= 32 && !e.members && status) {
         const size_t smem = (kFinThreads / 32) * (static_cast<size_t>(d) + 32 * kRefPitch) * sizeof(float);
-        cudaError_t err = cudaFuncSetAttribute(finish_warp_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        cudaError_t err = allow_max_smem(finish_warp_f32_kernel);
         if (err != cudaSuccess) return err;
         finish_warp_f32_kernel<<<(e.nq + kFinThreads / 32 - 1) / (kFinThreads / 32), kFinThreads, smem, stream>>>(
             cand, counts, cap, d, xq, xb, status, e);
@@ -1164,7 +1165,7 @@ cudaError_t launch_finish_f32(const uint64_t* cand, const uint32_t* counts, uint
     const uint32_t stage = cap < kFinStage ? cap : kFinStage;
     const size_t rows = 4 * 32 * kRefPitch * sizeof(float), held = stage * sizeof(uint64_t);
     const size_t smem = kFinKeep * sizeof(uint64_t) + static_cast<size_t>(d) * 4 + (rows > held ? rows : held);
-    cudaError_t err = cudaFuncSetAttribute(finish_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t err = allow_max_smem(finish_f32_kernel);
     if (err != cudaSuccess) return err;
     finish_f32_kernel<<<e.nq, kFinThreads, smem, stream>>>(cand, counts, cap, stage, d, eps, xq, xb, status, any_status, e);
     return cudaGetLastError();
@@ -1196,12 +1197,7 @@ cudaError_t launch_refine_f32(uint64_t* cand, const uint32_t* counts, uint32_t n
     if (gx > want) gx = want;
     if (gx > 64) gx = 64;
     if (gx < 1) gx = 1;
-    const size_t smem = (static_cast<size_t>(d) + 4 * 32 * kRefPitch) * sizeof(float);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(refine_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
+    const size_t smem = (static_cast<size_t>(d) + 4 * 32 * kRefPitch) * sizeof(float);   // (34 KB at d = 4096)
     for (int q0 = 0; q0 < nq; q0 += 65535) {
         const int nqq = nq - q0 < 65535 ? nq - q0 : 65535;
         refine_f32_kernel<<<dim3(gx, nqq), 128, smem, stream>>>(cand + static_cast<int64_t>(q0) * cap,

@@ -6,6 +6,8 @@ An index here owns one stream and one set of scratch buffers, so the C ABI seria
 a handle; the test runs searches of different sizes from several threads at once (ctypes releases
 the GIL during the call) and compares every result with the single-threaded one.
 """
+import os
+import subprocess
 import threading
 
 import numpy as np
@@ -14,6 +16,7 @@ import pytest
 from indexsdk_b200 import datasets
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _hammer(index, queries, k, expect, errors, rounds):
@@ -64,3 +67,18 @@ def test_concurrent_searches_on_one_ivfpq_index(b200):
     for t in threads:
         t.join()
     assert not errors, errors[:3]
+
+
+@pytest.mark.parametrize("which", ["select", "finish", "bound"])
+def test_two_indexes_share_their_kernels(b200, which):
+    """Calls on different handles run concurrently, also when the same kernels need another amount of
+    shared memory in each: what one thread asks for must not shrink what the other was granted.  (Threads of
+    a C++ program: the window is too short for threads that take turns at the interpreter.)"""
+    src = os.path.join(ROOT, "tests", "cpp", "test_two_indexes.cpp")
+    build = os.path.join(ROOT, "indexsdk_b200", "_build")
+    exe = os.path.join(build, "test_two_indexes")
+    if not os.path.exists(exe) or os.path.getmtime(src) > os.path.getmtime(exe):
+        subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "include"), src, "-o", exe,
+                        "-L", build, "-lb200idx", "-Wl,-rpath," + build, "-lpthread"], check=True)
+    r = subprocess.run([exe, which], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "0 failed" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
