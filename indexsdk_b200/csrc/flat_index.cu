@@ -492,8 +492,8 @@ void FlatIndex::run_tail(const PageTail& t, bool fused) {
 }
 
 // Queues a search of fp32 queries on the stream without waiting for it, where one page holds it; the
-// results are there, or padding, when the stream has got that far.  Once it has, queued_ok() says whether
-// they stand (false: search_device has to do it again).
+// results are there when the stream has got that far.  Once it has, queued_left() names the queries whose
+// candidates outgrew their lists: their results are padding, and search_device has to search for them.
 bool FlatIndex::queue_search(int64_t nq, const float* xq, int k, float* D, int64_t* I, int ldk) {
     if (nq <= 0 || n_ == 0 || dtype_ != kF32) return false;
     const Plan plan = make_plan(k, nq);
@@ -506,12 +506,13 @@ bool FlatIndex::queue_search(int64_t nq, const float* xq, int k, float* D, int64
     return true;
 }
 
-bool FlatIndex::queued_ok() {
+std::vector<int32_t> FlatIndex::queued_left() {
     timer_.collect(stats_);
     throw_on_error(queued_);
+    std::vector<int32_t> left;
     for (int i = 0; i < queued_.nq; ++i)
-        if (queued_.status[i]) return false;
-    return true;
+        if (queued_.status[i]) left.push_back(i);
+    return left;
 }
 
 int64_t FlatIndex::page_rows(uint32_t cap) const {

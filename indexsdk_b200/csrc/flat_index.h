@@ -123,7 +123,7 @@ public:
     // the call synchronises that stream before returning (candidate-overflow check).
     void search_device(int64_t nq, const void* xq, bool q_is_f16, int k, float* D, int64_t* I, int ldk);
     bool queue_search(int64_t nq, const float* xq, int k, float* D, int64_t* I, int ldk);
-    bool queued_ok();
+    std::vector<int32_t> queued_left();
     // Host-pointer search: pinned staging, H2D, search_device, D2H.
     void search_host(int64_t nq, const void* xq, bool q_is_f16, int k, float* D, int64_t* I);
     // mask: nq rows of ceil(ntotal / 8) bytes, bit (i % 8) of byte i / 8 = 1 lets base position i take part

@@ -2138,8 +2138,6 @@ void IvfpqIndex::search_preassigned_device(int64_t nq, const float* xq, int k, c
     search_stages(nq, xq, k, D, I, cD, cI);
 }
 
-// pre_cD / pre_cI: [nq][nprobe] probe distances and list ids computed elsewhere (nullptr: run the
-// coarse stage here).
 // The scan with a bound (ivfpq_short_scan.cu): the queries of a page in groups whose candidate rows fit 1 GB.
 // Returns the queries that need the exact scan (more candidates than a row holds).
 std::vector<int32_t> IvfpqIndex::search_short(const ShortScanArgs& a, int64_t m, cudaStream_t st) {
@@ -2193,15 +2191,48 @@ float IvfpqIndex::t2_bound() const {
     return cb_norm_bound_ * cb_norm_bound_ + 2.f * coarse_->raw_view().max_norm * cb_norm_bound_;
 }
 
+// pre_cD / pre_cI: [nq][nprobe] probe distances and list ids computed elsewhere (nullptr: run the
+// coarse stage here).
 void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int64_t* I, const float* pre_cD,
                                const int64_t* pre_cI) {
     if (nq <= 0) return;
     if (!is_trained()) throw std::invalid_argument("IVFPQ index is not trained (centroids / codebooks missing)");
     if (k > 1024) throw std::invalid_argument("IVFPQ search supports k <= 1024");
     DeviceGuard g(device_);
-    cudaStream_t st = stream();
     stats_.searches += 1;
     stats_.queries += static_cast<uint64_t>(nq);
+    scanned_known_ = false;
+    if (!search_pages(nq, xq, k, D, I, pre_cD, pre_cI, Route{})) B200_CUDA_CHECK(cudaStreamSynchronize(stream()));
+    timer_.collect(stats_);
+    stats_.kernel_launches += coarse_->stats().kernel_launches;
+    stats_.gemm_launches += coarse_->stats().gemm_launches;
+    coarse_->stats().kernel_launches = 0;
+    coarse_->stats().gemm_launches = 0;
+}
+
+// Some queries of a page once more, on another route: they are gathered, searched by themselves, and their
+// results take the place of what the page left for them.  Queued on the stream.
+void IvfpqIndex::search_again(const std::vector<int32_t>& which, const float* xq, int k, float* D, int64_t* I, Route r) {
+    cudaStream_t st = stream();
+    Again& w = again_[r.depth++];
+    const int n = static_cast<int>(which.size());
+    int32_t* idx = static_cast<int32_t*>(w.idx.ensure(static_cast<size_t>(n) * 4));
+    B200_CUDA_CHECK(cudaMemcpyAsync(idx, which.data(), static_cast<size_t>(n) * 4, cudaMemcpyHostToDevice, st));
+    float* x = static_cast<float*>(w.x.ensure(static_cast<size_t>(n) * d_ * 4));
+    B200_CUDA_CHECK(launch_gather_rows(xq, idx, n, d_ * 4, x, st));
+    float* rD = static_cast<float*>(w.D.ensure(static_cast<size_t>(n) * k * 4));
+    int64_t* rI = static_cast<int64_t*>(w.I.ensure(static_cast<size_t>(n) * k * 8));
+    search_pages(n, x, k, rD, rI, nullptr, nullptr, r);
+    B200_CUDA_CHECK(launch_scatter_rows(rD, idx, n, k * 4, D, st));
+    B200_CUDA_CHECK(launch_scatter_rows(rI, idx, n, k * 8, I, st));
+    stats_.kernel_launches += 3;
+}
+
+// The stages, a page of queries at a time.  Queued on the stream, which is waited for where a decision needs
+// results; returns whether it has been left idle.
+bool IvfpqIndex::search_pages(int64_t nq, const float* xq, int k, float* D, int64_t* I, const float* pre_cD,
+                              const int64_t* pre_cI, Route r) {
+    cudaStream_t st = stream();
     const int nprobe = std::max(1, std::min(nprobe_, nlist_));
     // filter width: k' = 32 * KPT >= k + 16
     int kpt = 1;
@@ -2212,15 +2243,15 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
                                                     : use_short_scan(M_, by_residual_, visited, nprobe, k));
     const int kprime = 32 * kpt;
     const int64_t page = 16384;
-    bool idle = true;    // the stream has been synchronised and nothing was queued since
-    scanned_known_ = false;
+    bool idle = true;
     for (int64_t q0 = 0; q0 < nq; q0 += page) {
         const int64_t m = std::min(page, nq - q0);
         const float* xp = xq + q0 * d_;
         const float* cD;
         const int64_t* cI;
         // The probes of the page are queued and scanned without looking at their statuses, which are read
-        // with the scan's; in the rare case that one is not 0 (candidate overflow) the page is done again.
+        // with the scan's; the few queries whose candidates outgrew the coarse search's lists find no probes
+        // then, and are searched again behind the others.
         bool queued = false;
         if (pre_cI) {
             cD = pre_cD + q0 * nprobe;
@@ -2229,17 +2260,22 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
             float* wD = static_cast<float*>(w_cD_.ensure(static_cast<size_t>(m) * nprobe * 4));
             int64_t* wI = static_cast<int64_t*>(w_cI_.ensure(static_cast<size_t>(m) * nprobe * 8));
             timer_.begin(kStageCoarse, st);
-            queued = coarse_->queue_search(m, xp, nprobe, wD, wI, nprobe);
+            queued = r.ahead && coarse_->queue_search(m, xp, nprobe, wD, wI, nprobe);
             if (!queued) coarse_->search_device(m, xp, false, nprobe, wD, wI, nprobe);
             timer_.end(st);
             cD = wD;
             cI = wI;
         }
-        auto probes_stand = [&]() {   // stream idle
-            if (!queued || coarse_->queued_ok()) return true;
-            coarse_->search_device(m, xp, false, nprobe, const_cast<float*>(cD), const_cast<int64_t*>(cI), nprobe);
-            queued = false;
-            return false;
+        float* outD = D + q0 * k;
+        int64_t* outI = I + q0 * k;
+        auto search_left = [&]() {   // stream idle since the page's first scan; the page's scratch is free again
+            if (!queued) return;
+            const std::vector<int32_t> left = coarse_->queued_left();
+            if (left.empty()) return;
+            Route again = r;
+            again.ahead = false;
+            search_again(left, xp, k, outD, outI, again);
+            idle = false;
         };
 
         ScanArgs a{};
@@ -2263,8 +2299,8 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
         a.xq = xp;
         a.centroids = coarse_->rows_f32();
         a.codebooks = codebooks_.as<float>();
-        a.outD = D + q0 * k;
-        a.outI = I + q0 * k;
+        a.outD = outD;
+        a.outI = outI;
         a.scanned = w_tmp_.as<unsigned long long>();
         a.qlist = nullptr;
 
@@ -2296,8 +2332,8 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
             s.outD = a.outD;
             s.outI = a.outI;
             s.scanned = a.scanned;
-            std::vector<int32_t> bad = search_short(s, m, st);
-            if (!probes_stand()) bad = search_short(s, m, st);
+            const std::vector<int32_t> bad = search_short(s, m, st);
+            idle = bad.empty();
             if (!bad.empty()) {
                 stats_.fallback_queries += bad.size();
                 int32_t* ql = static_cast<int32_t*>(w_qlist_.ensure(bad.size() * 4));
@@ -2307,22 +2343,17 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
                 stats_.kernel_launches += 1;
             }
             timer_.end(st);
-            idle = false;
+            search_left();
             continue;
         }
         if (!fast) {
-            for (bool again = true; again;) {
-                timer_.begin(kStageScan, st);
-                B200_CUDA_CHECK(launch_exact(a, static_cast<int>(m), st));
-                timer_.end(st);
-                stats_.kernel_launches += 2;
-                again = false;
-                if (queued) {
-                    B200_CUDA_CHECK(cudaStreamSynchronize(st));
-                    again = !probes_stand();
-                }
-            }
-            idle = false;
+            timer_.begin(kStageScan, st);
+            B200_CUDA_CHECK(launch_exact(a, static_cast<int>(m), st));
+            timer_.end(st);
+            stats_.kernel_launches += 2;
+            if (queued) B200_CUDA_CHECK(cudaStreamSynchronize(st));
+            idle = queued;
+            search_left();
             continue;
         }
         // probe splits: enough CTAs to fill the machine, bounded so that the refine kernel's
@@ -2349,150 +2380,145 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
                         nprobe >= 16 && m * nprobe < (1LL << 30);
         uint8_t* hf = a.flag;
         unsigned int tc_err_host = 0;
-        for (;;) {
-            std::memset(hf, 0, static_cast<size_t>(m));
-            unsigned int* tc_err = nullptr;
-            timer_.begin(kStageScan, st);
-            if (tc) {
-                const int64_t npairs = m * nprobe;
-                int32_t* keys = static_cast<int32_t*>(w_tc_keys_.ensure(static_cast<size_t>(npairs) * 4));
-                int32_t* vals = static_cast<int32_t*>(w_tc_vals_.ensure(static_cast<size_t>(npairs) * 4));
-                int32_t* keys2 = static_cast<int32_t*>(w_tc_keys2_.ensure(static_cast<size_t>(npairs) * 4));
-                int32_t* vals2 = static_cast<int32_t*>(w_tc_vals2_.ensure(static_cast<size_t>(npairs) * 4));
-                int32_t* first = static_cast<int32_t*>(w_tc_first_.ensure(static_cast<size_t>(nlist_) * 4));
-                int32_t* last = static_cast<int32_t*>(w_tc_last_.ensure(static_cast<size_t>(nlist_) * 4));
-                B200_CUDA_CHECK(launch_tc_keys(cI, npairs, nlist_, keys, vals, st));
-                int end_bit = 1;
-                while ((1 << end_bit) <= nlist_) ++end_bit;
-                size_t sort_bytes = 0;
-                B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys, keys2, vals, vals2,
-                                                                static_cast<int>(npairs), 0, end_bit, st));
-                void* sort_tmp = w_tc_sort_.ensure(sort_bytes);
-                B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, keys, keys2, vals, vals2,
-                                                                static_cast<int>(npairs), 0, end_bit, st));
-                B200_CUDA_CHECK(launch_tc_bounds(keys2, npairs, nlist_, first, last, st));
-                // lists with the most probing queries are handed out first, so that no long list is
-                // left for the end of the launch
-                int32_t* okeys = static_cast<int32_t*>(w_tc_okeys_.ensure(static_cast<size_t>(nlist_) * 16));
-                int32_t* ovals = okeys + nlist_;
-                int32_t* okeys2 = ovals + nlist_;
-                int32_t* order = okeys2 + nlist_;
-                B200_CUDA_CHECK(launch_tc_order_keys(first, last, nlist_, okeys, ovals, st));
-                size_t osort_bytes = 0;
-                B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, osort_bytes, okeys, okeys2, ovals, order, nlist_, 0, 31, st));
-                void* osort_tmp = w_tc_osort_.ensure(osort_bytes);
-                B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(osort_tmp, osort_bytes, okeys, okeys2, ovals, order, nlist_, 0, 31, st));
-                float* tau = static_cast<float*>(w_tc_tau_.ensure(static_cast<size_t>(m) * 4));
-                TcScanArgs t{};
-                t.cb16 = cb16_.as<uint16_t>();
-                t.cbnorm = cbnorm_.as<float>();
-                t.xq = xp;
-                t.centroids = coarse_->rows_f32();
-                t.cD = cD;
-                t.nprobe = nprobe;
-                t.nlist = nlist_;
-                t.nq = m;
-                t.sorted_pair = vals2;
-                t.first = first;
-                t.last = last;
-                t.order = order;
-                t.offsets = offsets_.as<int64_t>();
-                t.lens = lens_.as<int64_t>();
-                t.codes = codes_.as<uint8_t>();
-                t.tau = tau;
-                t.cap = 256;
-                t.cb_bound = a.cb_bound;
-                t.cand_d = static_cast<float*>(w_tc_cd_.ensure(static_cast<size_t>(m) * t.cap * 4));
-                t.cand_p = static_cast<uint32_t*>(w_tc_cp_.ensure(static_cast<size_t>(m) * t.cap * 4));
-                t.cand_n = static_cast<unsigned int*>(w_tc_cn_.ensure(static_cast<size_t>(m) * 4));
-                t.stage_cap = kTcStageCap;
-                t.stage = static_cast<uint4*>(w_tc_stage_.ensure(static_cast<size_t>(num_sms_) * kTcStageCap * 16));
-                t.stage_n = static_cast<unsigned int*>(w_tc_stage_n_.ensure(static_cast<size_t>(num_sms_) * 4));
-                t.work = w_work_.as<unsigned int>();
-                t.scanned = a.scanned;
-                if (!w_tc_err_.get()) {
-                    w_tc_err_.ensure(4);
-                    B200_CUDA_CHECK(cudaMemsetAsync(w_tc_err_.get(), 0, 4, st));
-                }
-                t.err = tc_err = w_tc_err_.as<unsigned int>();
+        std::memset(hf, 0, static_cast<size_t>(m));
+        unsigned int* tc_err = nullptr;
+        timer_.begin(kStageScan, st);
+        if (tc) {
+            const int64_t npairs = m * nprobe;
+            int32_t* keys = static_cast<int32_t*>(w_tc_keys_.ensure(static_cast<size_t>(npairs) * 4));
+            int32_t* vals = static_cast<int32_t*>(w_tc_vals_.ensure(static_cast<size_t>(npairs) * 4));
+            int32_t* keys2 = static_cast<int32_t*>(w_tc_keys2_.ensure(static_cast<size_t>(npairs) * 4));
+            int32_t* vals2 = static_cast<int32_t*>(w_tc_vals2_.ensure(static_cast<size_t>(npairs) * 4));
+            int32_t* first = static_cast<int32_t*>(w_tc_first_.ensure(static_cast<size_t>(nlist_) * 4));
+            int32_t* last = static_cast<int32_t*>(w_tc_last_.ensure(static_cast<size_t>(nlist_) * 4));
+            B200_CUDA_CHECK(launch_tc_keys(cI, npairs, nlist_, keys, vals, st));
+            int end_bit = 1;
+            while ((1 << end_bit) <= nlist_) ++end_bit;
+            size_t sort_bytes = 0;
+            B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys, keys2, vals, vals2,
+                                                            static_cast<int>(npairs), 0, end_bit, st));
+            void* sort_tmp = w_tc_sort_.ensure(sort_bytes);
+            B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, keys, keys2, vals, vals2,
+                                                            static_cast<int>(npairs), 0, end_bit, st));
+            B200_CUDA_CHECK(launch_tc_bounds(keys2, npairs, nlist_, first, last, st));
+            // lists with the most probing queries are handed out first, so that no long list is
+            // left for the end of the launch
+            int32_t* okeys = static_cast<int32_t*>(w_tc_okeys_.ensure(static_cast<size_t>(nlist_) * 16));
+            int32_t* ovals = okeys + nlist_;
+            int32_t* okeys2 = ovals + nlist_;
+            int32_t* order = okeys2 + nlist_;
+            B200_CUDA_CHECK(launch_tc_order_keys(first, last, nlist_, okeys, ovals, st));
+            size_t osort_bytes = 0;
+            B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, osort_bytes, okeys, okeys2, ovals, order, nlist_, 0, 31, st));
+            void* osort_tmp = w_tc_osort_.ensure(osort_bytes);
+            B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(osort_tmp, osort_bytes, okeys, okeys2, ovals, order, nlist_, 0, 31, st));
+            float* tau = static_cast<float*>(w_tc_tau_.ensure(static_cast<size_t>(m) * 4));
+            TcScanArgs t{};
+            t.cb16 = cb16_.as<uint16_t>();
+            t.cbnorm = cbnorm_.as<float>();
+            t.xq = xp;
+            t.centroids = coarse_->rows_f32();
+            t.cD = cD;
+            t.nprobe = nprobe;
+            t.nlist = nlist_;
+            t.nq = m;
+            t.sorted_pair = vals2;
+            t.first = first;
+            t.last = last;
+            t.order = order;
+            t.offsets = offsets_.as<int64_t>();
+            t.lens = lens_.as<int64_t>();
+            t.codes = codes_.as<uint8_t>();
+            t.tau = tau;
+            t.cap = 256;
+            t.cb_bound = a.cb_bound;
+            t.cand_d = static_cast<float*>(w_tc_cd_.ensure(static_cast<size_t>(m) * t.cap * 4));
+            t.cand_p = static_cast<uint32_t*>(w_tc_cp_.ensure(static_cast<size_t>(m) * t.cap * 4));
+            t.cand_n = static_cast<unsigned int*>(w_tc_cn_.ensure(static_cast<size_t>(m) * 4));
+            t.stage_cap = kTcStageCap;
+            t.stage = static_cast<uint4*>(w_tc_stage_.ensure(static_cast<size_t>(num_sms_) * kTcStageCap * 16));
+            t.stage_n = static_cast<unsigned int*>(w_tc_stage_n_.ensure(static_cast<size_t>(num_sms_) * 4));
+            t.work = w_work_.as<unsigned int>();
+            t.scanned = a.scanned;
+            if (!w_tc_err_.get()) {
+                w_tc_err_.ensure(4);
+                B200_CUDA_CHECK(cudaMemsetAsync(w_tc_err_.get(), 0, 4, st));
+            }
+            t.err = tc_err = w_tc_err_.as<unsigned int>();
 #ifdef B200IDX_DEV_PROF
-                const char* pe = std::getenv("B200IDX_PROF");
-                const bool tc_prof = pe && std::strcmp(pe, "1") == 0;
+            const char* pe = std::getenv("B200IDX_PROF");
+            const bool tc_prof = pe && std::strcmp(pe, "1") == 0;
 #else
-                const bool tc_prof = false;
+            const bool tc_prof = false;
 #endif
-                if (tc_prof) {
-                    w_tc_prof_.ensure(64 + static_cast<size_t>(m) * 4);
-                    B200_CUDA_CHECK(cudaMemsetAsync(w_tc_prof_.get(), 0, 64, st));
-                    t.prof = w_tc_prof_.as<unsigned long long>();
-                }
-                // threshold: one warp per query over the codes of its nearest list
-                B200_CUDA_CHECK(launch_tc_head_tau(t, cI, a.err_rel, a.t2_bound, tau, st));
-                B200_CUDA_CHECK(launch_tc_scan(t, num_sms_, st));
-                B200_CUDA_CHECK(launch_tc_select(t, a.fd, a.fp, a.fth, st));
-                if (tc_prof) {   // development aid: phase cycles of thread 0 (sum over CTAs), candidates per query
-                    unsigned long long hp[8];
-                    std::vector<unsigned int> cn(static_cast<size_t>(m));
-                    B200_CUDA_CHECK(cudaMemcpyAsync(hp, t.prof, 64, cudaMemcpyDeviceToHost, st));
-                    B200_CUDA_CHECK(cudaMemcpyAsync(cn.data(), t.cand_n, cn.size() * 4, cudaMemcpyDeviceToHost, st));
-                    B200_CUDA_CHECK(cudaStreamSynchronize(st));
-                    unsigned long long tot = 0, mx = 0;
-                    for (unsigned int c : cn) { tot += c; mx = std::max<unsigned long long>(mx, c); }
-                    std::fprintf(stderr, "[tc scan] per-CTA kcycles: ctx_wait %.0f decode %.0f barrier %.0f issue %.0f mma_wait %.0f "
-                                 "epilogue %.0f release %.0f; tiles/CTA %.0f; candidates/query avg %.1f max %llu\n",
-                                 hp[0] / 1e3 / num_sms_, hp[1] / 1e3 / num_sms_, hp[2] / 1e3 / num_sms_, hp[3] / 1e3 / num_sms_,
-                                 hp[4] / 1e3 / num_sms_, hp[5] / 1e3 / num_sms_, hp[6] / 1e3 / num_sms_,
-                                 static_cast<double>(hp[7]) / num_sms_, static_cast<double>(tot) / m, mx);
-                }
-                a.tc_rel = kTcErrRel;
-                a.tc_abs = kTcErrAbs;
-                stats_.kernel_launches += 8;
-            } else if (persist) {
-                a.work = w_work_.as<unsigned int>();
+            if (tc_prof) {
+                w_tc_prof_.ensure(64 + static_cast<size_t>(m) * 4);
+                B200_CUDA_CHECK(cudaMemsetAsync(w_tc_prof_.get(), 0, 64, st));
+                t.prof = w_tc_prof_.as<unsigned long long>();
+            }
+            // threshold: one warp per query over the codes of its nearest list
+            B200_CUDA_CHECK(launch_tc_head_tau(t, cI, a.err_rel, a.t2_bound, tau, st));
+            B200_CUDA_CHECK(launch_tc_scan(t, num_sms_, st));
+            B200_CUDA_CHECK(launch_tc_select(t, a.fd, a.fp, a.fth, st));
+            if (tc_prof) {   // development aid: phase cycles of thread 0 (sum over CTAs), candidates per query
+                unsigned long long hp[8];
+                std::vector<unsigned int> cn(static_cast<size_t>(m));
+                B200_CUDA_CHECK(cudaMemcpyAsync(hp, t.prof, 64, cudaMemcpyDeviceToHost, st));
+                B200_CUDA_CHECK(cudaMemcpyAsync(cn.data(), t.cand_n, cn.size() * 4, cudaMemcpyDeviceToHost, st));
+                B200_CUDA_CHECK(cudaStreamSynchronize(st));
+                unsigned long long tot = 0, mx = 0;
+                for (unsigned int c : cn) { tot += c; mx = std::max<unsigned long long>(mx, c); }
+                std::fprintf(stderr, "[tc scan] per-CTA kcycles: ctx_wait %.0f decode %.0f barrier %.0f issue %.0f mma_wait %.0f "
+                             "epilogue %.0f release %.0f; tiles/CTA %.0f; candidates/query avg %.1f max %llu\n",
+                             hp[0] / 1e3 / num_sms_, hp[1] / 1e3 / num_sms_, hp[2] / 1e3 / num_sms_, hp[3] / 1e3 / num_sms_,
+                             hp[4] / 1e3 / num_sms_, hp[5] / 1e3 / num_sms_, hp[6] / 1e3 / num_sms_,
+                             static_cast<double>(hp[7]) / num_sms_, static_cast<double>(tot) / m, mx);
+            }
+            a.tc_rel = kTcErrRel;
+            a.tc_abs = kTcErrAbs;
+            stats_.kernel_launches += 8;
+        } else if (persist) {
+            a.work = w_work_.as<unsigned int>();
 #ifdef B200IDX_DEV_PROF
-                a.prof = static_cast<unsigned long long*>(w_tc_prof_.ensure(128));
-                B200_CUDA_CHECK(cudaMemsetAsync(a.prof, 0, 128, st));
+            a.prof = static_cast<unsigned long long*>(w_tc_prof_.ensure(128));
+            B200_CUDA_CHECK(cudaMemsetAsync(a.prof, 0, 128, st));
 #endif
-                B200_CUDA_CHECK(launch_persist(a, kpt, num_sms_, st));
+            B200_CUDA_CHECK(launch_persist(a, kpt, num_sms_, st));
 #ifdef B200IDX_DEV_PROF
-                {
-                    unsigned long long hp[16];
-                    B200_CUDA_CHECK(cudaMemcpyAsync(hp, a.prof, 128, cudaMemcpyDeviceToHost, st));
-                    B200_CUDA_CHECK(cudaStreamSynchronize(st));
-                    const double nq_s = hp[9] ? static_cast<double>(hp[9]) : 1.0;
-                    std::fprintf(stderr, "[persist scan] cycles per query of a slot -- warp 1: build %.0f wait %.0f scan %.0f wait %.0f | "
-                                 "warp 0: build %.0f wait %.0f scan %.0f wait %.0f merge %.0f\n", hp[0] / nq_s, hp[1] / nq_s,
-                                 hp[2] / nq_s, hp[3] / nq_s, hp[4] / nq_s, hp[5] / nq_s, hp[6] / nq_s, hp[7] / nq_s, hp[8] / nq_s);
-                }
+            {
+                unsigned long long hp[16];
+                B200_CUDA_CHECK(cudaMemcpyAsync(hp, a.prof, 128, cudaMemcpyDeviceToHost, st));
+                B200_CUDA_CHECK(cudaStreamSynchronize(st));
+                const double nq_s = hp[9] ? static_cast<double>(hp[9]) : 1.0;
+                std::fprintf(stderr, "[persist scan] cycles per query of a slot -- warp 1: build %.0f wait %.0f scan %.0f wait %.0f | "
+                             "warp 0: build %.0f wait %.0f scan %.0f wait %.0f merge %.0f\n", hp[0] / nq_s, hp[1] / nq_s,
+                             hp[2] / nq_s, hp[3] / nq_s, hp[4] / nq_s, hp[5] / nq_s, hp[6] / nq_s, hp[7] / nq_s, hp[8] / nq_s);
+            }
 #endif
-            } else {
-                B200_CUDA_CHECK(launch_fast(a, kpt, st));
-            }
-            timer_.end(st);
-            timer_.begin(kStageMerge, st);
-            const int P = pow2_ceil_int(std::max(kprime, 32));
-            const size_t rsmem = static_cast<size_t>(P) * 12 + static_cast<size_t>(kprime) * 4;
-            if (S * kprime == 32 && k <= 32 && nprobe <= kRefMaxProbe) {
-                ivfpq_refine_warp_kernel<<<blocks_for(m, kRefWarpsPerBlock), kRefWarpsPerBlock * 32, 0, st>>>(a);
-            } else {
-                B200_CUDA_CHECK(allow_max_smem(ivfpq_refine_kernel));
-                ivfpq_refine_kernel<<<static_cast<unsigned>(m), kScanThreads, rsmem, st>>>(a, P);
-            }
-            B200_CUDA_CHECK(cudaGetLastError());
-            timer_.end(st);
-            stats_.kernel_launches += 3;
-            idle = false;
-            if (tc_err) B200_CUDA_CHECK(cudaMemcpyAsync(&tc_err_host, tc_err, 4, cudaMemcpyDeviceToHost, st));
-            B200_CUDA_CHECK(cudaStreamSynchronize(st));
-            idle = true;
-            if (tc_err_host) cudaMemsetAsync(tc_err, 0, 4, st);
-            if (tc_err_host & 2u)                       // a staging area overflowed: candidates were lost,
-                std::memset(hf, 1, static_cast<size_t>(m));   // every query of the page takes the exact path
-            if (tc_err_host & 1u) {
-                throw std::runtime_error("IVFPQ tensor-core scan reported error word " + std::to_string(tc_err_host) +
-                                         " (bounded wait ran out)");
-            }
-            if (probes_stand()) break;
+        } else {
+            B200_CUDA_CHECK(launch_fast(a, kpt, st));
+        }
+        timer_.end(st);
+        timer_.begin(kStageMerge, st);
+        const int P = pow2_ceil_int(std::max(kprime, 32));
+        const size_t rsmem = static_cast<size_t>(P) * 12 + static_cast<size_t>(kprime) * 4;
+        if (S * kprime == 32 && k <= 32 && nprobe <= kRefMaxProbe) {
+            ivfpq_refine_warp_kernel<<<blocks_for(m, kRefWarpsPerBlock), kRefWarpsPerBlock * 32, 0, st>>>(a);
+        } else {
+            B200_CUDA_CHECK(allow_max_smem(ivfpq_refine_kernel));
+            ivfpq_refine_kernel<<<static_cast<unsigned>(m), kScanThreads, rsmem, st>>>(a, P);
+        }
+        B200_CUDA_CHECK(cudaGetLastError());
+        timer_.end(st);
+        stats_.kernel_launches += 3;
+        if (tc_err) B200_CUDA_CHECK(cudaMemcpyAsync(&tc_err_host, tc_err, 4, cudaMemcpyDeviceToHost, st));
+        B200_CUDA_CHECK(cudaStreamSynchronize(st));
+        if (tc_err_host) cudaMemsetAsync(tc_err, 0, 4, st);
+        if (tc_err_host & 2u)                       // a staging area overflowed: candidates were lost,
+            std::memset(hf, 1, static_cast<size_t>(m));   // every query of the page takes the exact path
+        if (tc_err_host & 1u) {
+            throw std::runtime_error("IVFPQ tensor-core scan reported error word " + std::to_string(tc_err_host) +
+                                     " (bounded wait ran out)");
         }
         std::vector<int32_t> bad;
         for (int64_t i = 0; i < m; ++i)
@@ -2524,13 +2550,10 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
             B200_CUDA_CHECK(cudaStreamSynchronize(st));
             stats_.kernel_launches += 1;
         }
+        idle = true;
+        search_left();
     }
-    if (!idle) B200_CUDA_CHECK(cudaStreamSynchronize(st));
-    timer_.collect(stats_);
-    stats_.kernel_launches += coarse_->stats().kernel_launches;
-    stats_.gemm_launches += coarse_->stats().gemm_launches;
-    coarse_->stats().kernel_launches = 0;
-    coarse_->stats().gemm_launches = 0;
+    return idle;
 }
 
 void IvfpqIndex::search_host(int64_t nq, const float* xq, int k, float* D, int64_t* I) {

@@ -83,6 +83,18 @@ private:
     float t2_bound() const;
     void search_stages(int64_t nq, const float* xq, int k, float* D, int64_t* I, const float* pre_cD,
                        const int64_t* pre_cI);
+    // How queries go through the stages.
+    struct Route {
+        bool ahead = true;   // probes are queued ahead of their statuses
+        int depth = 0;       // how often these queries are searched again
+    };
+    bool search_pages(int64_t nq, const float* xq, int k, float* D, int64_t* I, const float* pre_cD,
+                      const int64_t* pre_cI, Route r);
+    void search_again(const std::vector<int32_t>& which, const float* xq, int k, float* D, int64_t* I, Route r);
+    struct Again {
+        DeviceBuffer idx, x, D, I;
+    };
+    Again again_[1];         // queries that are searched again, by depth
     bool has_centroids_ = false, has_codebooks_ = false;
     bool no_persist_ = false;
     bool tc_scan_ = false;                // list-major tensor-core filter scan (large batches, residual encoding)

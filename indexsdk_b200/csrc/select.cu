@@ -435,7 +435,8 @@ select_emit_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixe
             if (overflow) overflow[q] = 1;
             if (any_overflow) *any_overflow = 1u;
         }
-        n = cap;
+        for (uint32_t i = threadIdx.x; i < k; i += NT) emit_one(e, q, static_cast<int>(i), kCandInvalid);
+        return;
     }
     uint64_t* sorted = sel_sm;
     uint64_t* held = sel_sm + P;
@@ -1110,6 +1111,14 @@ __global__ void gather_rows_kernel(const uint32_t* src, const int32_t* idx, int 
     for (int i = threadIdx.x; i < row_words; i += blockDim.x) d[i] = s[i];
 }
 
+__global__ void scatter_rows_kernel(const uint32_t* src, const int32_t* idx, int n, int row_words, uint32_t* dst) {
+    const int r = blockIdx.x;
+    if (r >= n) return;
+    const uint32_t* s = src + static_cast<int64_t>(r) * row_words;
+    uint32_t* d = dst + static_cast<int64_t>(idx[r]) * row_words;
+    for (int i = threadIdx.x; i < row_words; i += blockDim.x) d[i] = s[i];
+}
+
 inline int next_pow2(int v) {
     int p = 1;
     while (p < v) p <<= 1;
@@ -1313,6 +1322,13 @@ cudaError_t launch_gather_rows(const void* src, const int32_t* idx, int n, int r
     if (n <= 0) return cudaSuccess;
     gather_rows_kernel<<<n, 128, 0, stream>>>(static_cast<const uint32_t*>(src), idx, n, row_bytes / 4,
                                               static_cast<uint32_t*>(dst));
+    return cudaGetLastError();
+}
+cudaError_t launch_scatter_rows(const void* src, const int32_t* idx, int n, int row_bytes, void* dst,
+                                cudaStream_t stream) {
+    if (n <= 0) return cudaSuccess;
+    scatter_rows_kernel<<<n, 128, 0, stream>>>(static_cast<const uint32_t*>(src), idx, n, row_bytes / 4,
+                                               static_cast<uint32_t*>(dst));
     return cudaGetLastError();
 }
 

@@ -70,8 +70,8 @@ struct EmitArgs {
 };
 // Per query: the k smallest of cand[q][0..min(counts[q],cap)) in ascending order as results (FLT_MAX / -1
 // where there are fewer).  counts == nullptr means every row holds n_fixed candidates.  overflow[q] is
-// set to 1 when counts[q] > cap (the row's result is then not trustworthy and the caller re-runs it
-// without a threshold), and so is *any_overflow; neither is written otherwise.  D, I, overflow and
+// set to 1 when counts[q] > cap (the row's results are then padding and the caller searches for the query
+// again, without a threshold), and so is *any_overflow; neither is written otherwise.  D, I, overflow and
 // any_overflow may lie in pinned host memory: stores there cost no copy and no wait of their own.
 cudaError_t launch_select_emit(const uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap,
                                uint8_t* overflow, uint32_t* any_overflow, const EmitArgs& e, cudaStream_t stream);
@@ -124,5 +124,8 @@ cudaError_t launch_iota_i64(int64_t* p, int64_t count, int64_t start, cudaStream
 // dst[i] = src[idx[i]] for rows of row_bytes bytes (row_bytes a multiple of 4).
 cudaError_t launch_gather_rows(const void* src, const int32_t* idx, int n, int row_bytes, void* dst,
                                cudaStream_t stream);
+// dst[idx[i]] = src[i], the other way round.
+cudaError_t launch_scatter_rows(const void* src, const int32_t* idx, int n, int row_bytes, void* dst,
+                                cudaStream_t stream);
 
 }  // namespace b200
