@@ -2567,18 +2567,16 @@ void IvfpqIndex::search_host(int64_t nq, const float* xq, int k, float* D, int64
     out.deliver(D, I, st);
 }
 
-// The counter of visited codes lives on the device and is read when somebody asks.
+// The counter of visited codes lives on the device and is read when somebody asks (under the handle's mutex,
+// like a search).
 SearchStats& IvfpqIndex::stats() {
     if (!scanned_known_ && w_tmp_.get()) {
         DeviceGuard g(device_);
-        unsigned long long v = 0;   // (no exception leaves here: the C entry that asks is not guarded)
-        if (cudaMemcpyAsync(&v, w_tmp_.get(), 8, cudaMemcpyDeviceToHost, stream()) == cudaSuccess &&
-            cudaStreamSynchronize(stream()) == cudaSuccess) {
-            stats_.scan_codes = v;
-            scanned_known_ = true;
-        } else {
-            cudaGetLastError();
-        }
+        unsigned long long v = 0;
+        B200_CUDA_CHECK(cudaMemcpyAsync(&v, w_tmp_.get(), 8, cudaMemcpyDeviceToHost, stream()));
+        B200_CUDA_CHECK(cudaStreamSynchronize(stream()));
+        stats_.scan_codes = v;
+        scanned_known_ = true;
     }
     return stats_;
 }

@@ -82,3 +82,33 @@ def test_two_indexes_share_their_kernels(b200, which):
                         "-L", build, "-lb200idx", "-Wl,-rpath," + build, "-lpthread"], check=True)
     r = subprocess.run([exe, which], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "0 failed" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def test_statistics_are_read_between_searches_not_inside_them(b200):
+    """A thread that asks for the statistics while another searches sees whole searches: the codes visited
+    belong to the queries counted, in between and at the end."""
+    d, nlist, M, k, n = 32, 16, 8, 10, 20000
+    rng = np.random.default_rng(4)
+    ix = b200.IndexIVFPQ(d, nlist, M, 8, by_residual=False)
+    ix.set_centroids(datasets.gaussian(nlist, d, seed=2))
+    ix.set_codebooks(rng.standard_normal((M, 256, d // M)).astype(np.float32))
+    ix.add_codes(rng.integers(0, nlist, size=n).astype(np.int32), rng.integers(0, 256, size=(n, M), dtype=np.uint8))
+    ix.nprobe = nlist                                          # every query visits every vector
+    xq = datasets.gaussian(40000, d, seed=1)                   # three pages
+    stop, wrong = threading.Event(), []
+
+    def watch():
+        while not stop.is_set():
+            s = ix.stats()
+            if s["scan_codes"] != s["queries"] * n:
+                wrong.append((s["queries"], s["scan_codes"]))
+
+    t = threading.Thread(target=watch)
+    t.start()
+    for _ in range(8):
+        ix.search(xq, k)
+    stop.set()
+    t.join()
+    s = ix.stats()
+    assert s["queries"] == 8 * len(xq) and s["scan_codes"] == s["queries"] * n
+    assert not wrong, wrong[:3]
