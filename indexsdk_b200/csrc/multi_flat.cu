@@ -167,11 +167,12 @@ void FlatGroup::search_device(const std::vector<FlatIndex*>& members, int64_t nq
     // help pass at most 9 k (the k-th of B minima admits B ln(1 / (1 - k / B)) keys, and B < 1.1 k
     // means fewer than 9 k rows), which the candidate rows have room for.
     const bool thresholded = static_cast<int64_t>(cap_) / 8 >= 4LL * k;
-    // [0] error word, [1] a candidate row was left (overflow, or too long): pinned, written by the kernels
-    volatile uint32_t* h = static_cast<uint32_t*>(h_flags_.ensure(8));
-    for (bool with_tau = thresholded;; with_tau = false) {
-        h[0] = h[1] = 0u;
-        run_passes(with_tau, nq, xq, xq_op, map_a, qnorm, k, D, I, st);
+    // [0] error word, [1] a candidate row overflowed, [2] a list was too long for the fused tail: pinned,
+    // written by the kernels
+    volatile uint32_t* h = static_cast<uint32_t*>(h_flags_.ensure(12));
+    for (Pass pass = thresholded ? kPassThresholds : kPassEveryKey;;) {
+        h[0] = h[1] = h[2] = 0u;
+        run_passes(pass, nq, xq, xq_op, map_a, qnorm, k, D, I, st);
         if (then) then();
         B200_CUDA_CHECK(cudaStreamSynchronize(st));
         if (h[0]) {
@@ -179,13 +180,15 @@ void FlatGroup::search_device(const std::vector<FlatIndex*>& members, int64_t nq
             B200_CUDA_CHECK(cudaMemsetAsync(w_err_.get(), 0, sizeof(int), st));
             throw std::runtime_error("device pipeline reported error word " + std::to_string(err) + " (bounded wait ran out)");
         }
-        if (!h[1]) return;
+        if (h[1]) pass = kPassEveryKey;
+        else if (h[2]) pass = kPassLongLists;
+        else return;
     }
 }
 
-void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq_op, const CUtensorMap& map_a,
+void FlatGroup::run_passes(Pass pass, int nq, const void* xq, const void* xq_op, const CUtensorMap& map_a,
                            const void* qnorm, int k, float* D, int64_t* I, cudaStream_t st) {
-    const bool is_int = dtype_ == kI8;
+    const bool is_int = dtype_ == kI8, with_tau = pass != kPassEveryKey;
     const uint32_t tau_all = is_int ? 0xFFFFFFFFu : 0xFF800000u;
     const size_t nm = cur_.size();
     const int n_qb = (nq + kTileQ - 1) / kTileQ;
@@ -249,7 +252,12 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
         L.kind = kind_;
         L.simt = use_simt_ ? 1 : 0;
         L.num_sms = num_sms_;
-        if (with_tau) {
+        // Lists that turned out too long for the fused tail are still there when one pass covers all members.
+        const bool listed = pass == kPassLongLists && nm <= per_pass;
+        a.counts = counts;
+        if (listed) {
+            // nothing to find
+        } else if (with_tau) {
             // bursts that a shorter member does not have never win
             B200_CUDA_CHECK(cudaMemsetAsync(mins, 0xFF, static_cast<size_t>(rows) * mins_stride * 4, st));
             a.mins = mins;
@@ -272,7 +280,6 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
             }
             B200_CUDA_CHECK(launch_kth_threshold(mins, mins_stride, mins_stride, rows, k, dtype_ == kF32 ? w_eps_.as<float>() : nullptr,
                                                  tau_all, tau, fold, st));
-            a.counts = counts;
             launches_ += 2;
         } else {
             B200_CUDA_CHECK(cudaMemsetAsync(cand, 0xFF, static_cast<size_t>(rows) * cap * 8, st));
@@ -280,7 +287,10 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
         }
         L.mode = kModeAppend;
         L.burst = 32;
-        B200_CUDA_CHECK(launch_dist_gemm(L, a, &map_a, &map_b_, st));
+        if (!listed) {
+            B200_CUDA_CHECK(launch_dist_gemm(L, a, &map_a, &map_b_, st));
+            ++launches_;
+        }
         EmitArgs e{};
         e.nq = rows;
         e.k = k;
@@ -295,8 +305,8 @@ void FlatGroup::run_passes(bool with_tau, int nq, const void* xq, const void* xq
         uint32_t* any_left = h_flags_.as<uint32_t>() + 1;
         e.err = w_err_.as<int>();
         e.err_host = h_flags_.as<int>();
-        launches_ += 2;
-        if (with_tau && dtype_ == kF32 && k <= kFinishMaxK) {
+        ++launches_;
+        if (pass == kPassThresholds && dtype_ == kF32 && k <= kFinishMaxK) {
             B200_CUDA_CHECK(launch_finish_f32(cand, counts, cap, d_, w_eps_.as<float>(), static_cast<const float*>(xq), nullptr,
                                               nullptr, any_left, e, false, st));
             continue;

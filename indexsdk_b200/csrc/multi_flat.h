@@ -31,7 +31,7 @@ public:
     // xq: device pointer, float rows (kF32 / kF16 members) or int8 rows.  D / I: device pointers
     // [members][nq][k].  Work is queued on `stream`; returns after synchronising it.  `then` may queue
     // what follows on the stream: it is called before that synchronisation (and again in the rare case
-    // that the search has to be repeated without thresholds).
+    // that lists were too long, or the search has to be repeated without thresholds).
     void search_device(const std::vector<FlatIndex*>& members, int64_t nq, const void* xq, int k, float* D, int64_t* I,
                        cudaStream_t stream, const std::function<void()>& then = nullptr);
     uint64_t launches() const { return launches_; }   // kernels launched by searches so far
@@ -39,8 +39,10 @@ public:
 
 private:
     void refresh(const std::vector<FlatIndex*>& members, cudaStream_t stream);
-    // All members' passes, with a threshold per (member, query) or with every key kept.
-    void run_passes(bool with_tau, int nq, const void* xq, const void* xq_op, const CUtensorMap& map_a, const void* qnorm,
+    // All members' passes: with a threshold per (member, query); the same with every list refined and ordered by
+    // kernels of their own, for when one is too long for the fused tail; or with every key kept.
+    enum Pass { kPassThresholds, kPassLongLists, kPassEveryKey };
+    void run_passes(Pass pass, int nq, const void* xq, const void* xq_op, const CUtensorMap& map_a, const void* qnorm,
                     int k, float* D, int64_t* I, cudaStream_t stream);
 
     int device_;

@@ -758,7 +758,7 @@ finish_f32_kernel(const uint64_t* cand, const uint32_t* counts, uint32_t cap, ui
     auto leave = [&](uint8_t why) {
         if (threadIdx.x == 0) {
             if (status) status[q] = why;
-            if (any_status) *any_status = 1u;
+            if (any_status) any_status[why - 1] = 1u;
         }
         // (a caller that goes on before it looks at the status finds no results, not stale ones)
         for (uint32_t i = threadIdx.x; i < k; i += kFinThreads) emit_one(e, q, static_cast<int>(i), kCandInvalid);

@@ -77,8 +77,8 @@ cudaError_t launch_select_emit(const uint64_t* cand, const uint32_t* counts, uin
                                uint8_t* overflow, uint32_t* any_overflow, const EmitArgs& e, cudaStream_t stream);
 // fp32 indexes: pruning, exact distances, selection and results of short candidate lists in one launch.
 // status[q], written when it is not 0: 1 row overflowed, 2 list too long for it (prune, refine and select it
-// instead; the candidates are unchanged, the results are padding); *any_status is set to 1 when any row is
-// left.  k <= kFinishMaxK.  few: lists of little
+// instead; the candidates are unchanged, the results are padding); any_status[0] is set to 1 when any row
+// overflowed, any_status[1] when any list is too long.  k <= kFinishMaxK.  few: lists of little
 // more than k candidates are expected (a threshold over the whole base), no need to prune them first.
 constexpr int kFinishMaxK = 256;
 cudaError_t launch_finish_f32(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int d, const float* eps,

@@ -72,3 +72,28 @@ def test_infinite_distances_fill_up_a_short_member(b200):
     x = datasets.gaussian(400, 64, seed=1)
     x[5:] = 3e19                                  # squared norm 5.8e40: not finite in fp32
     _check(b200, "f32_l2", [x, datasets.gaussian(700, 64, seed=2)], datasets.gaussian(3, 64, seed=3), 10)
+
+
+@pytest.mark.parametrize("metric", [L2, IP])
+def test_a_list_too_long_for_the_fused_tail_costs_its_own_kernels_only(b200, metric):
+    """1 100 rows of one member closer together than the bf16 filter can tell apart all survive the pruning.
+    The candidates are complete, so nothing has to be searched again: two kernels more (exact distances, order)
+    than a call without such rows."""
+    k, d = 100, 64
+    rng = np.random.default_rng(5)
+    plain = [datasets.gaussian(n, d, seed=i) for i, n in enumerate((12000, 9000, 11000))]
+    near = plain[1].copy()
+    near[rng.permutation(9000)[:1100]] = 3 * near[:1] + np.float32(1e-4) * datasets.gaussian(1100, d, seed=8)
+    xq = datasets.gaussian(6, d, seed=9)
+    xq[2] = 3 * near[0]
+    launches = []
+    for bases in (plain, [plain[0], near, plain[2]]):
+        ix, ref = _group(b200, "f32_l2" if metric == L2 else "f32_ip", bases)
+        b200.search_multi(ix, xq, k, merged=False)
+        before = b200.search_multi_stats()["group_launches"]
+        D, I = b200.search_multi(ix, xq, k, merged=False)
+        launches.append(b200.search_multi_stats()["group_launches"] - before)
+        for i, x in enumerate(bases):
+            Dr, Ir = oracle.flat_search(metric, x, xq, k)
+            assert_exact(D[i], I[i], Dr, Ir)
+    assert launches[1] == launches[0] + 2
