@@ -2138,19 +2138,37 @@ void IvfpqIndex::search_preassigned_device(int64_t nq, const float* xq, int k, c
     search_stages(nq, xq, k, D, I, cD, cI);
 }
 
-// The scan with a bound (ivfpq_short_scan.cu): the queries of a page in groups whose candidate rows fit 1 GB.
-// Returns the queries that need the exact scan (more candidates than a row holds).
-std::vector<int32_t> IvfpqIndex::search_short(const ShortScanArgs& a, int64_t m, cudaStream_t st) {
+// The scan with a bound (ivfpq_short_scan.cu): the queries of a page in groups whose scratch fits 256 MB.
+// row: candidates a query may collect; 0: the number to be expected.  Queries with more of them come back in
+// *longer or, where no row is long enough, *too_many.
+void IvfpqIndex::search_short(const ShortScanArgs& a, int64_t m, uint32_t row, std::vector<int32_t>* longer,
+                              std::vector<int32_t>* too_many) {
+    cudaStream_t st = stream();
     int64_t longest = 0;
-    for (int64_t l : lens_host_) longest = std::max(longest, l);
+    int64_t squares = 0;   // (at most vectors * longest list: below 2^62)
+    for (int64_t l : lens_host_) {
+        longest = std::max(longest, l);
+        squares += l * l;
+    }
     ShortScanArgs s = a;
-    s.cap = static_cast<uint32_t>(std::min<int64_t>(kShortMaxCap, std::max<int64_t>(32, longest * a.nprobe)));
     const int64_t visited = longest * a.nprobe;
     // (a query's nearest sixteenth, so far as it fits; more for a large k, whose candidates have to fit a row)
     const int64_t most = std::max<int64_t>(a.rotated ? kShortMaxBound / 2 : kShortMaxBound, 16LL * a.k);
     s.n1_max = static_cast<uint32_t>(std::min(most, std::max<int64_t>(1, std::min(visited, std::max<int64_t>({visited / 16, 4LL * a.k, 2048})))));
+    if (row == 0) {
+        // If the nearest lists are no better than the others, k of the n1 vectors the bound is taken from lie
+        // below it and k visited / n1 of all: sixteen k unless n1 is at its limit.  Clustered data brings far
+        // fewer.  Queries visit lists as often as vectors lie in them, or oftener, so a list counts with its own
+        // length, and there is room for twice that.  1 000 queries, M = 48, nprobe 128, k = 100: rows for the worst
+        // case took 456 MB, these take 96.  Raw short codes are equal by the thousand, of which the nearest
+        // sixteenth shows up to 1 024 before their labels are looked at: rows for the worst case.
+        const double many = 2.0 * a.nprobe * static_cast<double>(squares) / static_cast<double>(std::max<int64_t>(n_, 1));
+        const double want = 1.25 * a.k * std::max(16.0, many / s.n1_max) + 512.0;
+        row = !a.rotated && !a.by_residual ? kShortMaxCap : static_cast<uint32_t>(std::min<double>(kShortMaxCap, want));
+    }
+    s.cap = (static_cast<uint32_t>(std::min<int64_t>(row, std::max<int64_t>(32, visited))) + 31u) / 32u * 32u;
     const int64_t per_query = static_cast<int64_t>(s.cap) * 10 + static_cast<int64_t>(a.M) * kKsub * 4;
-    const int64_t group = std::min<int64_t>(4096, std::max<int64_t>(1, (int64_t(1) << 30) / per_query));
+    const int64_t group = std::min<int64_t>(4096, std::max<int64_t>(1, (int64_t(256) << 20) / per_query));
     const int64_t g = std::min(group, m);
     s.cand = static_cast<uint2*>(w_cpos_.ensure(static_cast<size_t>(g) * s.cap * 8));
     s.lut = static_cast<float*>(w_fd_.ensure(static_cast<size_t>(g) * a.M * kKsub * 4));
@@ -2173,10 +2191,9 @@ std::vector<int32_t> IvfpqIndex::search_short(const ShortScanArgs& a, int64_t m,
         stats_.kernel_launches += 3;
     }
     B200_CUDA_CHECK(cudaStreamSynchronize(st));
-    std::vector<int32_t> bad;
+    const bool longest_row = s.cap >= kShortMaxCap;
     for (int64_t i = 0; i < m; ++i)
-        if (flag[i]) bad.push_back(static_cast<int32_t>(i));
-    return bad;
+        if (flag[i]) (flag[i] == 1 && !longest_row ? longer : too_many)->push_back(static_cast<int32_t>(i));
 }
 
 // Error bound of the filter arithmetic relative to the canonical value:
@@ -2212,8 +2229,12 @@ void IvfpqIndex::search_stages(int64_t nq, const float* xq, int k, float* D, int
 
 // Some queries of a page once more, on another route: they are gathered, searched by themselves, and their
 // results take the place of what the page left for them.  Queued on the stream.
-void IvfpqIndex::search_again(const std::vector<int32_t>& which, const float* xq, int k, float* D, int64_t* I, Route r) {
+// cD, cI: the page's probes, or nullptr to select these queries' probes anew.
+void IvfpqIndex::search_again(const std::vector<int32_t>& which, const float* xq, int k, float* D, int64_t* I,
+                              const float* cD, const int64_t* cI, Route r) {
+    if (which.empty()) return;
     cudaStream_t st = stream();
+    const int nprobe = std::max(1, std::min(nprobe_, nlist_));
     Again& w = again_[r.depth++];
     const int n = static_cast<int>(which.size());
     int32_t* idx = static_cast<int32_t*>(w.idx.ensure(static_cast<size_t>(n) * 4));
@@ -2222,7 +2243,15 @@ void IvfpqIndex::search_again(const std::vector<int32_t>& which, const float* xq
     B200_CUDA_CHECK(launch_gather_rows(xq, idx, n, d_ * 4, x, st));
     float* rD = static_cast<float*>(w.D.ensure(static_cast<size_t>(n) * k * 4));
     int64_t* rI = static_cast<int64_t*>(w.I.ensure(static_cast<size_t>(n) * k * 8));
-    search_pages(n, x, k, rD, rI, nullptr, nullptr, r);
+    if (cI) {
+        float* gD = static_cast<float*>(w.cD.ensure(static_cast<size_t>(n) * nprobe * 4));
+        int64_t* gI = static_cast<int64_t*>(w.cI.ensure(static_cast<size_t>(n) * nprobe * 8));
+        B200_CUDA_CHECK(launch_gather_rows(cD, idx, n, nprobe * 4, gD, st));
+        B200_CUDA_CHECK(launch_gather_rows(cI, idx, n, nprobe * 8, gI, st));
+        cD = gD;
+        cI = gI;
+    }
+    search_pages(n, x, k, rD, rI, cD, cI, r);
     B200_CUDA_CHECK(launch_scatter_rows(rD, idx, n, k * 4, D, st));
     B200_CUDA_CHECK(launch_scatter_rows(rI, idx, n, k * 8, I, st));
     stats_.kernel_launches += 3;
@@ -2239,7 +2268,7 @@ bool IvfpqIndex::search_pages(int64_t nq, const float* xq, int k, float* D, int6
     while (kpt * 32 < k + 16) kpt <<= 1;
     const bool fast = rotated_ && !force_exact_ && kpt <= 32;
     const double visited = static_cast<double>(nprobe) * n_ / nlist_;   // vectors a query meets on average
-    const bool bounded = !force_exact_ && (rotated_ ? use_bounded_scan(M_, visited, nprobe, k, nq)
+    const bool bounded = r.bounded && !force_exact_ && (rotated_ ? use_bounded_scan(M_, visited, nprobe, k, nq)
                                                     : use_short_scan(M_, by_residual_, visited, nprobe, k));
     const int kprime = 32 * kpt;
     const int64_t page = 16384;
@@ -2274,7 +2303,7 @@ bool IvfpqIndex::search_pages(int64_t nq, const float* xq, int k, float* D, int6
             if (left.empty()) return;
             Route again = r;
             again.ahead = false;
-            search_again(left, xp, k, outD, outI, again);
+            search_again(left, xp, k, outD, outI, nullptr, nullptr, again);
             idle = false;
         };
 
@@ -2332,17 +2361,30 @@ bool IvfpqIndex::search_pages(int64_t nq, const float* xq, int k, float* D, int6
             s.outD = a.outD;
             s.outI = a.outI;
             s.scanned = a.scanned;
-            const std::vector<int32_t> bad = search_short(s, m, st);
-            idle = bad.empty();
-            if (!bad.empty()) {
-                stats_.fallback_queries += bad.size();
-                int32_t* ql = static_cast<int32_t*>(w_qlist_.ensure(bad.size() * 4));
-                B200_CUDA_CHECK(cudaMemcpyAsync(ql, bad.data(), bad.size() * 4, cudaMemcpyHostToDevice, st));
+            std::vector<int32_t> longer, too_many;
+            search_short(s, m, r.row, &longer, &too_many);
+            timer_.end(st);
+            idle = longer.empty() && too_many.empty();
+            Route again = r;
+            again.row = kShortMaxCap;
+            search_again(longer, xp, k, outD, outI, cD, cI, again);
+            if (fast && static_cast<int>(too_many.size()) < num_sms_) {
+                // The filter, whose lists have a fixed length, rather than one block per query: for as many queries as
+                // there are SMs the latter is no slower (512 queries, k = 1 000, 1 M vectors each without list
+                // structure: 28.8 ms for the 412 queries left over, the filter 44.2; 64 queries, 51 left
+                // over: 16.2 ms against 9.0; k = 300, 36 of 512: 19.0 against 9.5).
+                again.bounded = false;
+                search_again(too_many, xp, k, outD, outI, cD, cI, again);
+            } else if (!too_many.empty()) {
+                stats_.fallback_queries += too_many.size();
+                int32_t* ql = static_cast<int32_t*>(w_qlist_.ensure(too_many.size() * 4));
+                B200_CUDA_CHECK(cudaMemcpyAsync(ql, too_many.data(), too_many.size() * 4, cudaMemcpyHostToDevice, st));
                 a.qlist = ql;
-                B200_CUDA_CHECK(launch_exact(a, static_cast<int>(bad.size()), st));
+                timer_.begin(kStageScan, st);
+                B200_CUDA_CHECK(launch_exact(a, static_cast<int>(too_many.size()), st));
+                timer_.end(st);
                 stats_.kernel_launches += 1;
             }
-            timer_.end(st);
             search_left();
             continue;
         }

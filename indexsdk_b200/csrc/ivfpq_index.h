@@ -78,7 +78,8 @@ private:
     int nprobe_ = 1;
     int64_t n_ = 0;                       // vectors stored
     int64_t n_pad_ = 0;                   // storage slots in use: every list padded to a multiple of 32
-    std::vector<int32_t> search_short(const ShortScanArgs& a, int64_t m, cudaStream_t st);
+    void search_short(const ShortScanArgs& a, int64_t m, uint32_t row, std::vector<int32_t>* longer,
+                      std::vector<int32_t>* too_many);
     float filter_err_rel() const;
     float t2_bound() const;
     void search_stages(int64_t nq, const float* xq, int k, float* D, int64_t* I, const float* pre_cD,
@@ -86,15 +87,18 @@ private:
     // How queries go through the stages.
     struct Route {
         bool ahead = true;   // probes are queued ahead of their statuses
+        bool bounded = true; // the scan with a bound may be taken
+        uint32_t row = 0;    // ... with candidate rows of this length (0: see search_short)
         int depth = 0;       // how often these queries are searched again
     };
     bool search_pages(int64_t nq, const float* xq, int k, float* D, int64_t* I, const float* pre_cD,
                       const int64_t* pre_cI, Route r);
-    void search_again(const std::vector<int32_t>& which, const float* xq, int k, float* D, int64_t* I, Route r);
+    void search_again(const std::vector<int32_t>& which, const float* xq, int k, float* D, int64_t* I, const float* cD,
+                      const int64_t* cI, Route r);
     struct Again {
-        DeviceBuffer idx, x, D, I;
+        DeviceBuffer idx, x, D, I, cD, cI;
     };
-    Again again_[1];         // queries that are searched again, by depth
+    Again again_[3];         // queries that are searched again, by depth: probes, a longer row, another scan
     bool has_centroids_ = false, has_codebooks_ = false;
     bool no_persist_ = false;
     bool tc_scan_ = false;                // list-major tensor-core filter scan (large batches, residual encoding)

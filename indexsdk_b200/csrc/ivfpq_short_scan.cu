@@ -22,8 +22,8 @@
 // within twice the error of the k-th get their canonical distance.
 // Wide codes: wide_scan_kernel takes the place of short_scan_kernel, with the table rows of the wide-code filter
 // (ivfpq_index.cu); what they measured stands at use_bounded_scan.
-// A query with more than `cap` vectors under its bound (tens of thousands of equal codes) is flagged
-// and scanned exactly by the caller.
+// A query with more than `cap` vectors under its bound is flagged, and the caller searches for it with a longer
+// row or another scan.
 // What bounds it (64 queries, 10 M vectors, M = 4, 64 of 1024 lists, k = 300; the exact scan this
 // replaces took 2.14 ms): the bound takes 41 us (64 blocks, one step
 // after the other inside), the scan 65 (issue slots: about 40 instructions a vector, and two table fills per
@@ -680,7 +680,7 @@ short_select_kernel(const ShortScanArgs a) {
     const int64_t q = blockIdx.x;
     const uint32_t n = a.count[q];
     if (n > a.cap) {
-        if (threadIdx.x == 0) a.flag[q] = 1;
+        if (threadIdx.x == 0) a.flag[q] = n > kShortMaxCap ? 2 : 1;
         return;
     }
     uint2* row = a.cand + q * a.cap;
