@@ -81,7 +81,9 @@ int FlatIndex::gemm_kind() const {
 
 void FlatIndex::reserve(int64_t n) {
     if (n <= cap_rows_) return;
-    generation_ = next_generation();   // the rows move: tables that point at them are out of date even if the add fails
+    // the rows move: what points at them is out of date even if an allocation below fails and the add with it
+    generation_ = next_generation();
+    map_b_valid_ = false;
     int64_t want = std::max<int64_t>(n, cap_rows_ + cap_rows_ / 2);
     want = round_up(want, kTileB);
     const size_t row_op = static_cast<size_t>(op_cols()) * op_elem_bytes();
@@ -92,7 +94,6 @@ void FlatIndex::reserve(int64_t n) {
     norms_.grow_keep(static_cast<size_t>(want) * 4, static_cast<size_t>(n_) * 4, stream_);
     labels_.grow_keep(static_cast<size_t>(want) * 8, static_cast<size_t>(n_) * 8, stream_);
     cap_rows_ = want;
-    map_b_valid_ = false;
 }
 
 void FlatIndex::add(int64_t n, const void* x, bool x_is_f16, const int64_t* ids, bool x_on_device) {

@@ -169,3 +169,32 @@ def test_argument_errors(b200):
     with pytest.raises(b200.B200IdxError) as e:
         b200.IndexFlat(100, L2)
     assert "Unsupported dims" in e.value.msg
+
+
+def test_search_after_an_add_that_ran_out_of_memory(b200):
+    """An add whose growth fails half way (the rows' copy has moved, their labels do not fit any more) leaves
+    the index as it was."""
+    import torch
+    d, k, n = 16, 10, 2_000_000
+    ix = b200.IndexFlat(d, L2, dtype=b200.F16)
+    xb, xq = datasets.gaussian(5000, d, seed=1), datasets.gaussian(7, d, seed=2)
+    ix.add(xb)
+    D, I = ix.search(xq, k)
+    more = torch.zeros(n, d, device="cuda")
+    torch.cuda.synchronize()
+    # room for the operand rows (32 bytes each) and the norms (4), not for the labels (8)
+    room = n * 36 + (8 << 20)
+    held = []
+    for _ in range(4):
+        spare = torch.cuda.mem_get_info()[0] - room
+        if spare > 4 << 20:
+            held.append(torch.empty(spare, dtype=torch.uint8, device="cuda"))
+    with pytest.raises(b200.B200IdxError):
+        ix.add_device(more.data_ptr(), n)
+    held.clear()
+    torch.cuda.empty_cache()
+    assert ix.ntotal == len(xb)
+    D2, I2 = ix.search(xq, k)
+    assert_exact(D2, I2, D, I)
+    ix.add_device(more.data_ptr(), n)
+    assert ix.ntotal == len(xb) + n
