@@ -78,6 +78,7 @@ public:
         if (bytes > bytes_) {
             if (ptr_) cudaFreeHost(ptr_);
             ptr_ = nullptr;
+            bytes_ = 0;   // (the allocation may fail)
             size_t want = (bytes + bytes / 4 + 255) & ~size_t(255);
             B200_CUDA_CHECK(cudaMallocHost(&ptr_, want));
             bytes_ = want;
