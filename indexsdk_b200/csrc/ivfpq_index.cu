@@ -50,6 +50,7 @@
 #include "kmeans.h"
 #include "ptx_sm100.cuh"
 #include "smem_limit.h"
+#include "spare_pool.h"
 #include "select.cuh"
 
 namespace b200 {
@@ -1724,6 +1725,7 @@ IvfpqIndex::IvfpqIndex(int d, int nlist, int M, int nbits, bool by_residual, int
     if (M <= 0 || d % M != 0) throw std::invalid_argument("d must be a multiple of M");
     DeviceGuard g(device_);
     B200_CUDA_CHECK(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device_));
+    spare_user_.join(device_);
     coarse_.reset(new FlatIndex(d, kMetricL2, kF32, device));
     offsets_.ensure(static_cast<size_t>(nlist_ + 1) * 8);
     B200_CUDA_CHECK(cudaMemset(offsets_.get(), 0, static_cast<size_t>(nlist_ + 1) * 8));
@@ -1940,36 +1942,53 @@ void IvfpqIndex::add_codes(int64_t n, const int32_t* list_no, const uint8_t* cod
 // Stable merge of a batch into the CSR lists: existing entries keep their order, new entries
 // follow in arrival order (the order the reference's per-list append produces).  Codes are
 // re-rotated for their new positions on the way.
+namespace {
+// The arrays of one merge; they go to the spare ones when it is over.
+class MergeArrays {
+public:
+    MergeArrays(int device, cudaStream_t st) : pool_(SparePool::of(device)), st_(st) {}
+    ~MergeArrays() {
+        cudaStreamSynchronize(st_);
+        for (int i = 0; i < used_; ++i) pool_.give(b_[i]);
+    }
+    DeviceBuffer& get() { return b_[used_++]; }
+    void* get(size_t bytes) { return pool_.take(get(), bytes); }
+
+private:
+    SparePool& pool_;
+    cudaStream_t st_;
+    DeviceBuffer b_[12];
+    int used_ = 0;
+};
+}  // namespace
+
 void IvfpqIndex::merge_new(int64_t n, const int32_t* ln, const uint8_t* cd, const float* t2, const int64_t* idd) {
     cudaStream_t st = stream();
     const int64_t n_new_total = n_ + n;
     // upper bound of the padded size; the exact value is known after the scan below
     const int64_t pad_bound = n_new_total + static_cast<int64_t>(kListPad) * (nlist_ + 1);
     if (pad_bound > 0x7FFFFFF0ll) throw std::invalid_argument("a single-device IVFPQ index holds at most 2^31 - 16 vectors (padding included)");
-    // The work arrays of a merge and the spare set the lists change places with are kept while they
-    // are small (allocating and freeing the thirteen of them was 12 of the 22 ms that adding 300 000
-    // vectors took).
-    DeviceBuffer &hist = w_m_[0], &new_len = w_m_[1], &padded = w_m_[2], &new_off = w_m_[3], &new_first = w_m_[4],
-                 &keys_out = w_m_[5], &vals_in = w_m_[6], &vals_out = w_m_[7], &cub_tmp = w_m_[8];
-    DeviceBuffer &ncodes = w_m_[9], &nids = w_m_[10], &nt2 = w_m_[11];
-    int64_t* h = static_cast<int64_t*>(hist.ensure(static_cast<size_t>(nlist_ + 1) * 8));
+    MergeArrays w(device_, st);
+    DeviceBuffer &new_len = w.get(), &new_off = w.get(), &ncodes = w.get(), &nids = w.get(), &nt2 = w.get();
+    SparePool& pool = SparePool::of(device_);
+    int64_t* h = static_cast<int64_t*>(w.get(static_cast<size_t>(nlist_ + 1) * 8));
     B200_CUDA_CHECK(cudaMemsetAsync(h, 0, static_cast<size_t>(nlist_ + 1) * 8, st));
     hist_kernel<<<blocks_for(n, 256), 256, 0, st>>>(ln, n, h);
-    int64_t* nlen = static_cast<int64_t*>(new_len.ensure(static_cast<size_t>(nlist_ + 1) * 8));
-    int64_t* pad = static_cast<int64_t*>(padded.ensure(static_cast<size_t>(nlist_ + 1) * 8));
+    int64_t* nlen = static_cast<int64_t*>(pool.take(new_len, static_cast<size_t>(nlist_ + 1) * 8));
+    int64_t* pad = static_cast<int64_t*>(w.get(static_cast<size_t>(nlist_ + 1) * 8));
     add_counts_kernel<<<blocks_for(nlist_ + 1, 256), 256, 0, st>>>(lens_.as<int64_t>(), h, nlist_, nlen, pad);
-    int64_t* noff = static_cast<int64_t*>(new_off.ensure(static_cast<size_t>(nlist_ + 1) * 8));
-    int64_t* nfirst = static_cast<int64_t*>(new_first.ensure(static_cast<size_t>(nlist_ + 1) * 8));
+    int64_t* noff = static_cast<int64_t*>(pool.take(new_off, static_cast<size_t>(nlist_ + 1) * 8));
+    int64_t* nfirst = static_cast<int64_t*>(w.get(static_cast<size_t>(nlist_ + 1) * 8));
     size_t tmp_bytes = 0, tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, pad, noff, nlist_ + 1, st);
-    int32_t* kout = static_cast<int32_t*>(keys_out.ensure(static_cast<size_t>(n) * 4));
-    int32_t* vin = static_cast<int32_t*>(vals_in.ensure(static_cast<size_t>(n) * 4));
-    int32_t* vout = static_cast<int32_t*>(vals_out.ensure(static_cast<size_t>(n) * 4));
+    int32_t* kout = static_cast<int32_t*>(w.get(static_cast<size_t>(n) * 4));
+    int32_t* vin = static_cast<int32_t*>(w.get(static_cast<size_t>(n) * 4));
+    int32_t* vout = static_cast<int32_t*>(w.get(static_cast<size_t>(n) * 4));
     int end_bit = 1;
     while ((1 << end_bit) < nlist_) ++end_bit;
     cub::DeviceRadixSort::SortPairs(nullptr, tb, ln, kout, vin, vout, static_cast<int>(n), 0, end_bit, st);
     tmp_bytes = std::max(tmp_bytes, tb);
-    void* tmp = cub_tmp.ensure(tmp_bytes + 16);
+    void* tmp = w.get(tmp_bytes + 16);
     size_t tsz = tmp_bytes;
     B200_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(tmp, tsz, pad, noff, nlist_ + 1, st));
     tsz = tmp_bytes;
@@ -1977,9 +1996,9 @@ void IvfpqIndex::merge_new(int64_t n, const int32_t* ln, const uint8_t* cd, cons
     iota_i32_kernel<<<blocks_for(n, 256), 256, 0, st>>>(vin, n);
     tsz = tmp_bytes;
     B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(tmp, tsz, ln, kout, vin, vout, static_cast<int>(n), 0, end_bit, st));
-    uint8_t* nc = static_cast<uint8_t*>(ncodes.ensure(static_cast<size_t>(pad_bound) * M_ + 64));
-    int64_t* ni = static_cast<int64_t*>(nids.ensure(static_cast<size_t>(pad_bound) * 8));
-    float* nt = static_cast<float*>(nt2.ensure(static_cast<size_t>(pad_bound) * 4));
+    uint8_t* nc = static_cast<uint8_t*>(pool.take(ncodes, static_cast<size_t>(pad_bound) * M_ + 64));
+    int64_t* ni = static_cast<int64_t*>(pool.take(nids, static_cast<size_t>(pad_bound) * 8));
+    float* nt = static_cast<float*>(pool.take(nt2, static_cast<size_t>(pad_bound) * 4));
     if (n_pad_ > 0)
         scatter_old_kernel<<<blocks_for(n_pad_, 256), 256, 0, st>>>(n_pad_, nlist_, offsets_.as<int64_t>(),
                                                                     lens_.as<int64_t>(), noff, M_, rotated_ ? 1 : 0,
@@ -2000,9 +2019,6 @@ void IvfpqIndex::merge_new(int64_t n, const int32_t* ln, const uint8_t* cd, cons
     codes_.swap(ncodes);
     ids_.swap(nids);
     t2_.swap(nt2);
-    constexpr size_t kSpareBytes = size_t(64) << 20;
-    for (DeviceBuffer& w : w_m_)
-        if (w.bytes() > kSpareBytes) w.release();
     n_ = n_new_total;
     n_pad_ = offsets_host_[static_cast<size_t>(nlist_)];
 }

@@ -16,6 +16,7 @@
 
 #include "flat_index.h"
 #include "ivfpq_short_scan.cuh"
+#include "spare_pool.h"
 
 namespace b200 {
 
@@ -107,6 +108,7 @@ private:
     float cb_norm_bound_ = 0.f;           // sqrt(sum_m max_j |cb[m][j]|^2), for the filter's error bound
     bool force_exact_ = false;            // B200IDX_IVFPQ_EXACT=1: always use the exact scan kernels
 
+    SparePool::User spare_user_;          // (first: it leaves after the arrays below are freed)
     std::unique_ptr<FlatIndex> coarse_;   // nlist centroids, fp32, L2
     DeviceBuffer codebooks_;              // [M][256][dsub] float
     DeviceBuffer codebooks_t_;            // the same regrouped [M / 16][256][16][dsub] (M % 16 == 0)
@@ -119,7 +121,6 @@ private:
     // scratch
     DeviceBuffer w_work_, w_cD_, w_cI_, w_fd_, w_fp_, w_fth_, w_qlist_, w_q_, w_D_, w_I_, w_assign_D_,
         w_assign_I_, w_list_, w_codes_, w_t2_, w_ids_, w_x_, w_tmp_, w_vflag_, w_cpos_, w_ccount_;
-    DeviceBuffer w_m_[12];           // merge_new: work arrays and the spare list arrays
     mutable PinnedBuffer h_list_;    // get_list: a stretch of a list on its way out
     DeviceBuffer w_tc_keys_, w_tc_vals_, w_tc_keys2_, w_tc_vals2_, w_tc_first_, w_tc_last_, w_tc_cI0_, w_tc_cD0_,
         w_tc_fd0_, w_tc_fp0_, w_tc_fth0_, w_tc_tau_, w_tc_cd_, w_tc_cp_, w_tc_cn_, w_tc_sort_, w_tc_err_, w_tc_prof_, w_tc_stage_, w_tc_stage_n_, w_tc_okeys_, w_tc_osort_;
