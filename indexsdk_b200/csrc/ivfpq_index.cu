@@ -2156,9 +2156,9 @@ void IvfpqIndex::search_preassigned_device(int64_t nq, const float* xq, int k, c
 
 // The scan with a bound (ivfpq_short_scan.cu): the queries of a page in groups whose scratch fits 256 MB.
 // row: candidates a query may collect; 0: the number to be expected.  Queries with more of them come back in
-// *longer or, where no row is long enough, *too_many.
+// *longer or, where no row is long enough, *too_many, and queries beyond the range of floats in *exact.
 void IvfpqIndex::search_short(const ShortScanArgs& a, int64_t m, uint32_t row, std::vector<int32_t>* longer,
-                              std::vector<int32_t>* too_many) {
+                              std::vector<int32_t>* too_many, std::vector<int32_t>* exact) {
     cudaStream_t st = stream();
     int64_t longest = 0;
     int64_t squares = 0;   // (at most vectors * longest list: below 2^62)
@@ -2209,7 +2209,7 @@ void IvfpqIndex::search_short(const ShortScanArgs& a, int64_t m, uint32_t row, s
     B200_CUDA_CHECK(cudaStreamSynchronize(st));
     const bool longest_row = s.cap >= kShortMaxCap;
     for (int64_t i = 0; i < m; ++i)
-        if (flag[i]) (flag[i] == 1 && !longest_row ? longer : too_many)->push_back(static_cast<int32_t>(i));
+        if (flag[i]) (flag[i] == 3 ? exact : flag[i] == 1 && !longest_row ? longer : too_many)->push_back(static_cast<int32_t>(i));
 }
 
 // Error bound of the filter arithmetic relative to the canonical value:
@@ -2377,10 +2377,10 @@ bool IvfpqIndex::search_pages(int64_t nq, const float* xq, int k, float* D, int6
             s.outD = a.outD;
             s.outI = a.outI;
             s.scanned = a.scanned;
-            std::vector<int32_t> longer, too_many;
-            search_short(s, m, r.row, &longer, &too_many);
+            std::vector<int32_t> longer, too_many, exact;
+            search_short(s, m, r.row, &longer, &too_many, &exact);
             timer_.end(st);
-            idle = longer.empty() && too_many.empty();
+            idle = longer.empty() && too_many.empty() && exact.empty();
             Route again = r;
             again.row = kShortMaxCap;
             search_again(longer, xp, k, outD, outI, cD, cI, again);
@@ -2391,13 +2391,16 @@ bool IvfpqIndex::search_pages(int64_t nq, const float* xq, int k, float* D, int6
                 // over: 16.2 ms against 9.0; k = 300, 36 of 512: 19.0 against 9.5).
                 again.bounded = false;
                 search_again(too_many, xp, k, outD, outI, cD, cI, again);
-            } else if (!too_many.empty()) {
-                stats_.fallback_queries += too_many.size();
-                int32_t* ql = static_cast<int32_t*>(w_qlist_.ensure(too_many.size() * 4));
-                B200_CUDA_CHECK(cudaMemcpyAsync(ql, too_many.data(), too_many.size() * 4, cudaMemcpyHostToDevice, st));
+            } else {
+                exact.insert(exact.end(), too_many.begin(), too_many.end());
+            }
+            if (!exact.empty()) {
+                stats_.fallback_queries += exact.size();
+                int32_t* ql = static_cast<int32_t*>(w_qlist_.ensure(exact.size() * 4));
+                B200_CUDA_CHECK(cudaMemcpyAsync(ql, exact.data(), exact.size() * 4, cudaMemcpyHostToDevice, st));
                 a.qlist = ql;
                 timer_.begin(kStageScan, st);
-                B200_CUDA_CHECK(launch_exact(a, static_cast<int>(too_many.size()), st));
+                B200_CUDA_CHECK(launch_exact(a, static_cast<int>(exact.size()), st));
                 timer_.end(st);
                 stats_.kernel_launches += 1;
             }

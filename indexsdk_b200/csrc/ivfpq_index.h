@@ -80,7 +80,7 @@ private:
     int64_t n_ = 0;                       // vectors stored
     int64_t n_pad_ = 0;                   // storage slots in use: every list padded to a multiple of 32
     void search_short(const ShortScanArgs& a, int64_t m, uint32_t row, std::vector<int32_t>* longer,
-                      std::vector<int32_t>* too_many);
+                      std::vector<int32_t>* too_many, std::vector<int32_t>* exact);
     float filter_err_rel() const;
     float t2_bound() const;
     void search_stages(int64_t nq, const float* xq, int k, float* D, int64_t* I, const float* pre_cD,

@@ -112,7 +112,7 @@ short_bound_kernel(const ShortScanArgs a) {
     float* base = reinterpret_cast<float*>(beg + kShortMaxProbe);
     float* qs = base + kShortMaxProbe;                                      // [d]
     uint32_t* dist = reinterpret_cast<uint32_t*>(qs + a.d);                 // [a.n1_max] bits of the distances
-    __shared__ uint32_t s_warp[32], s_lo, s_hi, s_bin, s_below, s_in;
+    __shared__ uint32_t s_warp[32], s_lo, s_hi, s_bin, s_below, s_in, s_base;
     __shared__ unsigned long long s_llo, s_lhi;
     __shared__ float s_qn2;
     const int64_t q = blockIdx.x;
@@ -120,6 +120,7 @@ short_bound_kernel(const ShortScanArgs a) {
     if (tid == 0) {
         s_lo = kInfBits;
         s_hi = 0u;
+        s_base = 0u;
         a.count[q] = 0u;
     }
     for (int t = tid; t < a.d; t += kBoundThreads) qs[t] = a.xq[q * a.d + t];
@@ -131,6 +132,10 @@ short_bound_kernel(const ShortScanArgs a) {
         if (p < a.nprobe) pr = load_probe(a, q, p);
         uint32_t sum;
         const uint32_t ex = block_exclusive(pr.len, s_warp, &sum);
+        if (a.by_residual) {   // largest magnitude (a NaN is larger still)
+            const uint32_t far = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(pr.base)));
+            if ((tid & 31) == 0) atomicMax(&s_base, far);
+        }
         if (p < a.nprobe) {
             pre[p] = total + ex;
             beg[p] = pr.begin;
@@ -396,9 +401,15 @@ short_bound_kernel(const ShortScanArgs a) {
         float thr = __uint_as_float(tb);
         // scanned distances of raw short codes are the canonical ones; the others are off by eps at most
         float eps = 0.f;
-        if (a.by_residual && tb != kInfBits) {
-            const float coarse_max = a.cD[q * a.nprobe + a.nprobe - 1];
-            eps = a.err_rel * (fabsf(coarse_max) + a.t2_bound + 2.f * sqrtf(s_qn2) * a.cb_bound + thr);
+        if (a.by_residual) {
+            const float mag = __uint_as_float(s_base) + a.t2_bound + 2.f * sqrtf(s_qn2) * a.cb_bound;
+            if (tb != kInfBits) eps = a.err_rel * (mag + thr);
+            // A query whose terms leave the range of a float (or hold a NaN): their sum may be NaN where the
+            // canonical distance is a number.  It collects nothing and is left to the exact scan.
+            if (!(mag < kPadDist)) {
+                thr = __int_as_float(0x7fc00000);
+                a.count[q] = kShortExact;
+            }
         } else if (wide<M>() && tb != kInfBits) {
             eps = a.err_rel * thr;
         }
@@ -680,7 +691,7 @@ short_select_kernel(const ShortScanArgs a) {
     const int64_t q = blockIdx.x;
     const uint32_t n = a.count[q];
     if (n > a.cap) {
-        if (threadIdx.x == 0) a.flag[q] = n > kShortMaxCap ? 2 : 1;
+        if (threadIdx.x == 0) a.flag[q] = n == kShortExact ? 3 : n > kShortMaxCap ? 2 : 1;
         return;
     }
     uint2* row = a.cand + q * a.cap;

@@ -8,6 +8,7 @@ namespace b200 {
 constexpr int kShortMaxProbe = 1024;     // probes whose metadata a block stages in shared memory
 constexpr uint32_t kShortMaxBound = 16384;   // vectors the bound is taken from (wide codes: half as many)
 constexpr uint32_t kShortMaxCap = 32768; // most candidates a query may collect; more take another scan
+constexpr uint32_t kShortExact = 0xFFFFFFFFu;   // count of a query that needs the exact scan
 
 struct ShortScanArgs {
     const int64_t* cI;       // [nq][nprobe] probed list ids (-1 = none), nearest first
@@ -39,7 +40,8 @@ struct ShortScanArgs {
     // results
     float* outD;             // [nq][k]
     int64_t* outI;
-    uint8_t* flag;           // [nq] written when the query has more than cap candidates: 1, or 2 for more than kShortMaxCap
+    uint8_t* flag;           // [nq] written when the query has more than cap candidates: 1, or 2 for more than kShortMaxCap;
+                             // 3 = exact scan
     unsigned long long* scanned;
 };
 

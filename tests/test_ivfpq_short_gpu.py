@@ -77,3 +77,26 @@ def test_queries_that_hold_nan_or_infinity_find_what_the_exact_scan_finds(b200, 
         ix.nprobe = 4
         out.append(ix.search(xq, 20))
     assert_exact(out[0][0], out[0][1], out[1][0], out[1][1])
+
+
+@pytest.mark.parametrize("M,d,k", [(4, 64, 300), (8, 64, 20), (16, 64, 60), (48, 96, 100)])
+def test_residual_queries_beyond_the_range_of_floats_find_what_the_exact_scan_finds(b200, monkeypatch, M, d, k):
+    """With a component or a norm that overflows, |q - c|^2 + t2 - 2 q.cb can be NaN where the canonical distance
+    is infinite."""
+    nlist = 8
+    xb, _ = datasets.mixture(4000, d, 8, seed=4)
+    cent, cb = datasets.train_ivfpq(xb, nlist, M, True, niter=3)
+    xq = xb[:9].copy()
+    xq[1, 3], xq[2, 5], xq[3] = np.nan, np.inf, 1e30
+    xq[4], xq[5, 7], xq[6] = 1e18, 3e38, np.inf
+    xq[7, 1], xq[8, 2] = -1e19, 1e19
+    out = []
+    for exact in ("0", "1"):
+        monkeypatch.setenv("B200IDX_IVFPQ_EXACT", exact)
+        ix = b200.IndexIVFPQ(d, nlist, M, 8, by_residual=True)
+        ix.set_centroids(cent)
+        ix.set_codebooks(cb)
+        ix.add(xb)
+        ix.nprobe = nlist
+        out.append(ix.search(xq, k))
+    assert_exact(out[0][0], out[0][1], out[1][0], out[1][1])
