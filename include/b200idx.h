@@ -173,8 +173,9 @@ int b200idx_ivfpq_train(b200idx_t* h, int64_t n, const float* x, int niter, uint
  * the queries, exchange them, and scan their shard for all queries.
  *   coarse      : probe_distances_dev / probe_lists_dev [n][nprobe] <- the nprobe nearest centroids
  *                 (canonical fp32 distances, ascending; list -1 = none)
- *   preassigned : searches the given probes; same results as b200idx_search_device when they come
- *                 from coarse on the same queries */
+ *   preassigned : searches the given probes, in any order (list -1 = none); same results as
+ *                 b200idx_search_device when they come from coarse on the same queries.  Raw encoding,
+ *                 and residual encoding with M other than 16, 32, 48 and 64, do not read the distances */
 int b200idx_ivfpq_coarse_device(b200idx_t* h, int64_t n, const float* x_dev, float* probe_distances_dev,
                                 int64_t* probe_lists_dev);
 int b200idx_ivfpq_search_preassigned_device(b200idx_t* h, int64_t n, const float* x_dev, int k,

@@ -225,6 +225,23 @@ __global__ void i64_to_i32_kernel(const int64_t* in, int64_t n, int32_t* out) {
     if (i < n) out[i] = static_cast<int32_t>(in[i]);
 }
 
+// |q - c|^2 of every probe, a warp each (0 where there is none).
+__global__ void probe_distance_kernel(const float* xq, int d, const float* centroids, const int64_t* cI, int64_t n, int nprobe,
+                                      int nlist, float* cD) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t list = cI[i];
+    float s = 0.f;
+    if (list >= 0 && list < nlist)
+        for (int t = lane; t < d; t += 32) {
+            const float df = xq[i / nprobe * d + t] - centroids[list * d + t];
+            s = fmaf(df, df, s);
+        }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) cD[i] = s;
+}
+
 // ---- list maintenance ----
 __global__ void hist_kernel(const int32_t* list_no, int64_t n, int64_t* hist) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -2354,6 +2371,15 @@ bool IvfpqIndex::search_pages(int64_t nq, const float* xq, int k, float* D, int6
             ShortScanArgs s{};
             s.cI = a.cI;
             s.cD = a.cD;
+            if (pre_cI && by_residual_ && !rotated_ && r.depth == 0) {
+                // The exact scan, which short codes come from, has no use for the caller's probe distances, so
+                // nothing is known about them.
+                float* pD = static_cast<float*>(w_pD_.ensure(static_cast<size_t>(m) * nprobe * 4));
+                probe_distance_kernel<<<blocks_for(m * nprobe, 8), 256, 0, st>>>(xp, d_, a.centroids, cI, m * nprobe, nprobe, nlist_, pD);
+                B200_CUDA_CHECK(cudaGetLastError());
+                stats_.kernel_launches += 1;
+                s.cD = cD = pD;
+            }
             s.nprobe = nprobe;
             s.nlist = nlist_;
             s.k = k;

@@ -119,7 +119,7 @@ private:
     std::vector<int64_t> offsets_host_, lens_host_;
     DeviceBuffer codes_, ids_, t2_;
     // scratch
-    DeviceBuffer w_work_, w_cD_, w_cI_, w_fd_, w_fp_, w_fth_, w_qlist_, w_q_, w_D_, w_I_, w_assign_D_,
+    DeviceBuffer w_work_, w_cD_, w_cI_, w_pD_, w_fd_, w_fp_, w_fth_, w_qlist_, w_q_, w_D_, w_I_, w_assign_D_,
         w_assign_I_, w_list_, w_codes_, w_t2_, w_ids_, w_x_, w_tmp_, w_vflag_, w_cpos_, w_ccount_;
     mutable PinnedBuffer h_list_;    // get_list: a stretch of a list on its way out
     DeviceBuffer w_tc_keys_, w_tc_vals_, w_tc_keys2_, w_tc_vals2_, w_tc_first_, w_tc_last_, w_tc_cI0_, w_tc_cD0_,

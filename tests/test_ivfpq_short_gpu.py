@@ -100,3 +100,42 @@ def test_residual_queries_beyond_the_range_of_floats_find_what_the_exact_scan_fi
         ix.nprobe = nlist
         out.append(ix.search(xq, k))
     assert_exact(out[0][0], out[0][1], out[1][0], out[1][1])
+
+
+# short codes: the distances that come with the probes are not what decides; wide codes scan with them
+@pytest.mark.parametrize("M,d,k,how", [(4, 64, 10, "reversed"), (4, 64, 10, "zero"), (8, 64, 300, "zero"), (8, 64, 10, "nan"),
+                                       (16, 64, 60, "reversed"), (16, 64, 60, "some"), (8, 64, 10, "some"), (64, 64, 300, "reversed")])
+def test_given_probes_in_any_order(b200, M, d, k, how):
+    import torch
+    nlist, nprobe, nq = 32, 20, 50
+    xb, _ = datasets.mixture(30000, d, nlist, seed=4, sigma=0.5)
+    cent, cb = datasets.train_ivfpq(xb[:6000], nlist, M, True, niter=2)
+    ix = b200.IndexIVFPQ(d, nlist, M, 8, by_residual=True)
+    ix.set_centroids(cent)
+    ix.set_codebooks(cb)
+    ix.add(xb)
+    ix.nprobe = nprobe
+    xq = torch.from_numpy(datasets.mixture(nq, d, nlist, seed=5, centers_seed=4, sigma=0.5)[0]).cuda()
+    cD = torch.empty(nq, nprobe, device="cuda")
+    cI = torch.empty(nq, nprobe, device="cuda", dtype=torch.int64)
+    D, I = torch.empty(nq, k, device="cuda"), torch.empty(nq, k, device="cuda", dtype=torch.int64)
+    ix.coarse_device(xq.data_ptr(), nq, cD.data_ptr(), cI.data_ptr())
+    if how == "some":                       # every other probe is none, the last one too
+        cI[:, 1::2] = -1
+        cD[:, 1::2] = float("nan")
+    lists = cI.cpu().numpy()
+    if how == "reversed":
+        cD, cI = cD.flip(1).contiguous(), cI.flip(1).contiguous()
+    elif how == "zero":
+        cD.zero_()
+    elif how == "nan":
+        cD.fill_(float("nan"))
+    torch.cuda.synchronize()
+    ix.search_preassigned_device(xq.data_ptr(), nq, k, cD.data_ptr(), cI.data_ptr(), D.data_ptr(), I.data_ptr())
+    ln = oracle.ivf_assign(cent, xb)
+    codes = oracle.pq_encode(cb, xb, True, cent, ln)
+    for q in range(0, nq, 7):               # the oracle over the vectors of the given lists
+        rows = np.flatnonzero(np.isin(ln, lists[q]))
+        off, cs, ids = oracle.build_lists(ln[rows], codes[rows], rows.astype(np.int64), nlist)
+        Dr, Ir = oracle.ivfpq_search(cent, cb, True, off, cs, ids, xq[q:q + 1].cpu().numpy(), nlist, k)
+        assert_exact(D[q:q + 1].cpu().numpy(), I[q:q + 1].cpu().numpy(), Dr, Ir)
