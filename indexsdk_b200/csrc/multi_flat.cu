@@ -1,6 +1,7 @@
 #include "multi_flat.h"
 
 #include <algorithm>
+#include <limits>
 #include <stdexcept>
 #include <string>
 
@@ -71,7 +72,9 @@ void FlatGroup::refresh(const std::vector<FlatIndex*>& members, cudaStream_t st)
         const int64_t p = pad_tile(members[i]->ntotal());
         seg_start_[i + 1] = seg_start_[i] + p;
         cap_ = std::max<uint32_t>(cap_, static_cast<uint32_t>(p));
-        max_norm_ = std::max(max_norm_, members[i]->raw_view().max_norm);
+        const float norm = members[i]->raw_view().max_norm;
+        // (a member with rows whose norm is not a number has no error bound: infinity keeps every key)
+        max_norm_ = norm == norm ? std::max(max_norm_, norm) : std::numeric_limits<float>::infinity();
     }
     total_rows_ = seg_start_.back();
     // Everything a pass needs to know about its members travels in one copy.  Their data is not

@@ -97,3 +97,17 @@ def test_a_list_too_long_for_the_fused_tail_costs_its_own_kernels_only(b200, met
             Dr, Ir = oracle.flat_search(metric, x, xq, k)
             assert_exact(D[i], I[i], Dr, Ir)
     assert launches[1] == launches[0] + 2
+
+
+@pytest.mark.parametrize("metric", [L2, IP])
+@pytest.mark.parametrize("nq,k", [(20, 1), (300, 10)])
+def test_a_member_without_an_error_bound(b200, metric, nq, k):
+    """A row with a NaN leaves a member's largest norm undefined; the other members' norms say nothing about
+    its rows, of which one is near the largest float."""
+    bases = [datasets.gaussian(n, 64, seed=i) for i, n in enumerate((1, 40, 300))]
+    bases[1][7], bases[1][9, 2], bases[1][11], bases[1][13] = np.inf, np.nan, -np.inf, 3e38
+    ix, _ = _group(b200, "f32_l2" if metric == L2 else "f32_ip", bases)
+    xq = datasets.gaussian(nq, 64, seed=9)
+    D, I = b200.search_multi(ix, xq, k, merged=False)
+    for i in range(3):
+        assert_exact(D[i], I[i], *ix[i].search(xq, k))     # few rows: every key is looked at
