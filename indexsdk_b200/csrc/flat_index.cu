@@ -142,7 +142,7 @@ void FlatIndex::add(int64_t n, const void* x, bool x_is_f16, const int64_t* ids,
         float m2 = 0.f;
         B200_CUDA_CHECK(cudaMemcpyAsync(&m2, maxnorm_.get(), 4, cudaMemcpyDeviceToHost, stream_));
         B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
-        max_norm_ = std::sqrt(m2) * 1.0001f;
+        max_norm_ = std::sqrt(m2 + kNormFloor) * 1.0001f;
     }
     B200_CUDA_CHECK(cudaStreamSynchronize(stream_));
     n_ += n;
@@ -228,7 +228,9 @@ FlatIndex::Plan FlatIndex::make_plan(int k, int64_t nq) const {
     const int64_t n_tiles = (n_ + kTileB - 1) / kTileB;
     const int64_t need = std::max<int64_t>(4LL * k, 1024);
     p.sampled = false;
-    if (n_tiles <= 256) {
+    // a row whose norm is infinite or no number leaves fp32 keys without an error bound, for every query
+    const bool bounded = dtype_ != kF32 || max_norm_ <= 1e38f;
+    if (bounded && n_tiles <= 256) {
         // Small base (e.g. an IVF coarse quantizer): the "sample" is the whole base, so the k-th
         // smallest burst minimum is a certain upper bound of the k-th smallest key and admits
         // little more than k candidates as long as bursts are plentiful against k (with k / bursts
@@ -245,7 +247,7 @@ FlatIndex::Plan FlatIndex::make_plan(int k, int64_t nq) const {
         if (p.sampled) p.s_tiles = static_cast<int>(n_tiles);
     }
     for (int burst : {32, 8}) {
-        if (p.sampled) break;
+        if (p.sampled || !bounded) break;
         const int bpt = kTileB / burst;
         const int64_t s = std::max<int64_t>((n_tiles + 15) / 16, (need + bpt - 1) / bpt);
         if (s * 2 <= n_tiles) {

@@ -42,12 +42,19 @@ __device__ __forceinline__ void store_tau(int q, uint32_t ord, uint32_t* tau, co
     if (!fold.qnorm) return;
     const float t = ord_to_float(ord);
     const float qn = fold.qnorm[fold.q_mod > 0 ? q % fold.q_mod : q];
-    const float m = sqrtf(qn) * fold.ymax + 0.5f * fold.ymax * fold.ymax + fabsf(t);
-    float c = t + 0.000244140625f * m;
+    const float reach = sqrtf(qn) * fold.ymax + 0.5f * fold.ymax * fold.ymax;
+    float c = t + 0.000244140625f * (reach + fabsf(t));
     if (fold.metric == kMetricL2) c *= 0.5f;
     if (fold.bias) {
         fold.bias[q] = c;
     } else {
+        // A query whose terms may leave the range of a float (0 x infinity included): with a threshold among
+        // them a sum may be NaN where the key is a number.  Nothing passes, and the row counts as overflowed: the
+        // caller searches for it without a threshold.
+        if (!(reach <= 1e38f)) {
+            c = __int_as_float(0xff800000);
+            if (fold.counts) fold.counts[q] = 0x80000000u;
+        }
         const int dp = fold.d + kFoldCols;
         // columns d + 3 .. d + 5 lie in one 8-column group (d is a multiple of 16), so they are
         // consecutive in the packed layout as well
@@ -686,8 +693,8 @@ refine_f32_kernel(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint
     // candidate row q_first + q holds the candidates of query (q_first + q) % q_mod (several indexes
     // searched with the same queries) or of query q_first + q (q_mod = 0)
     const int qrow = q_mod > 0 ? (q_first + q) % q_mod : q_first + q;
-    uint32_t n = counts ? counts[q] : n_fixed;
-    if (n > cap) n = cap;
+    const uint32_t n = counts ? counts[q] : n_fixed;
+    if (n > cap) return;   // overflowed: what its slots hold is not looked at
     if (blockIdx.x * kRefWindow >= n) return;
     uint32_t pos_first = 0;   // position of xb's first row
     if (members) {
@@ -994,7 +1001,7 @@ __global__ void prep_queries_f32_kernel(const float* xq, int nq, int d, int metr
         // 2^-8 (1 + 2^-10) relatively, so |dot~ - dot| <= c |q||y| with the accumulation slack
         // folded into c; the second term covers the fp32 rounding of norms and of the canonical
         // distance itself.
-        const float qn = sqrtf(s) * 1.0001f;
+        const float qn = sqrtf(s + kNormFloor) * 1.0001f;
         const float c = 0.00390625f * 1.01f + static_cast<float>(d) * 4.76837158203125e-07f;
         const float g = static_cast<float>(d + 4) * 2.384185791015625e-07f;
         float e;

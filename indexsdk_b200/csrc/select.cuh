@@ -53,6 +53,9 @@ cudaError_t launch_refine_f32(uint64_t* cand, const uint32_t* counts, uint32_t n
                               int metric, const float* xq, const float* xb, cudaStream_t stream, int q_mod = 0,
                               const MemberView* members = nullptr);
 
+// Added to squared norms that error bounds are formed from: the squares of components below about 1e-19 vanish.
+constexpr float kNormFloor = 1e-30f;
+
 struct EmitArgs {
     int nq, k;
     int metric;

@@ -72,3 +72,51 @@ def test_filter_that_leaves_fewer_rows_than_k(b200, keep):
             if keep:
                 Dr, Ir = oracle.int8_search(metric, xb[rows], xq[q:q + 1], got, labels=rows)
                 assert_exact(D[q:q + 1, :got], I[q:q + 1, :got], Dr, Ir)
+
+
+def _odd_queries(nq, d):
+    xq = datasets.gaussian(nq, d, seed=7)
+    one = [np.nan, np.inf, -np.inf, 1e15, 1e18, 1e20, 1e30, 3e38]
+    whole = [1e18, 1e20, 3e38, 0.0, 1e-30, np.inf, np.nan]
+    xq[np.arange(len(one)), 3] = one
+    for i, v in enumerate(whole):
+        xq[len(one) + i] = v
+    return xq
+
+
+# what the smallest base thresholds are taken from, one and several tiles, and larger ones
+@pytest.mark.parametrize("metric", [L2, IP])
+@pytest.mark.parametrize("n,d", [(1, 64), (40, 64), (300, 64), (2100, 80), (20000, 64)])
+@pytest.mark.parametrize("rows", ["plain", "no number", "huge", "tiny", "equal"])
+def test_without_an_error_bound_every_key_is_looked_at(b200, metric, n, d, rows):
+    """Queries and rows whose norms overflow, vanish or are no numbers find what the search without thresholds
+    finds (the entry point without allocations)."""
+    import torch
+    xb = datasets.gaussian(n, d, seed=n)
+    if rows == "no number" and n > 20:
+        xb[7], xb[9, 2], xb[11], xb[13] = np.inf, np.nan, -np.inf, 3e38
+    elif rows == "huge":
+        xb[n // 4:n // 2] = 3e19
+    elif rows == "tiny":
+        xb *= np.float32(1e-25)
+    elif rows == "equal":
+        xb[n // 2:] = xb[0]
+    ix = b200.IndexFlat(d, metric)
+    ix.add(xb)
+    for nq, k in ((20, 1), (20, 10), (20, 300), (45, 100), (2000, 1)):
+        if nq * ((n + 255) // 256 * 256) > 1 << 20:
+            continue
+        xq = _odd_queries(nq, d)
+        xt = torch.from_numpy(xq).cuda()
+        out = []
+        for f in (ix.search_device, ix.search_device_noalloc):
+            for q0 in range(0, nq, nq if f == ix.search_device else 1000):
+                m = min(nq - q0, nq if f == ix.search_device else 1000)
+                if q0 == 0:
+                    D, I = torch.empty(nq, k, device="cuda"), torch.empty(nq, k, device="cuda", dtype=torch.int64)
+                torch.cuda.synchronize()
+                f(xt[q0:].data_ptr(), m, k, D[q0:].data_ptr(), I[q0:].data_ptr())
+            torch.cuda.synchronize()
+            out.append((D.cpu().numpy(), I.cpu().numpy()))
+        np.testing.assert_array_equal(out[0][1], out[1][1])
+        np.testing.assert_array_equal(out[0][0], out[1][0])
