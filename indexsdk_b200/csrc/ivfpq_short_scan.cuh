@@ -51,6 +51,9 @@ struct ShortScanArgs {
 // 15 600 321 against 327, 62 500 474 against 642; M = 8, 780 vectors 217 against 195, 3 100 256 against 272), or
 // fewer when k is large (k = 100: 265 against 355 at 3 100 vectors).  The exact scan of residual codes
 // builds a table per list: two lists are enough (4 lists of 50 vectors, M = 8: 231 us against 353).
+// There is no line above: in clustered data the exact scan is ten times slower at any size (M = 4, 512 queries of
+// 1 M vectors, k = 900: 8.1 ms against 0.84), and where lists are no better than one another and most queries of a
+// large k end up with it after all, bound and scan come on top of it (23.3 ms against 28.3).
 inline bool use_short_scan(int M, bool residual, double visited, int nprobe, int k) {
     if ((M != 4 && M != 8) || nprobe > kShortMaxProbe || k > 1024) return false;
     if (residual && nprobe > 1) return true;
@@ -66,10 +69,19 @@ inline bool use_short_scan(int M, bool residual, double visited, int nprobe, int
 //   k = 10,  31 000, 2 048 queries: M = 16 375 / 645, M = 32 859 / 886, M = 48 1 036 / 1 202, M = 64 2 020 / 1 646
 // Below about 2 000 vectors a query the bound is not worth its launch.  16-byte codes with k <= 48 stay with the
 // lists: their tables are small, and the persistent kernel takes over from 1 184 queries on.
+// The other way round, once the lists are full, hardly a vector gets past them, and the filter's loop is the
+// faster one (4 M vectors, 1 024 lists, us before / this way; vectors near their centroids, and without structure):
+//   k = 10,  M = 48, 64 queries of 1.0 M: 1 324 / 1 045 and 4 491 / 2 140;  of 3.0 M: 2 537 / 2 903 and 5 922 / 3 613
+//   k = 10,  M = 48, 512 queries of 102 k: 1 032 / 863 and 5 377 / 3 074;   of 500 k: 2 969 / 3 565 and 11 385 / 9 881
+//   k = 100, M = 16, 512 queries of 500 k: 1 805 / 1 452 and 5 147 / 4 234; of 1.0 M: 2 778 / 2 950, of 3.0 M: 6 773 / 8 526
+//   k = 100, M = 48, 512 queries of 500 k: 3 736 / 3 577 and 12 869 / 9 909; of 1.0 M: 5 809 / 7 191
+// so the product of queries and vectors has a limit.  Longer lists (k > 112: k' of 256 and more) never catch up
+// in that range (k = 300, M = 48, 512 queries of 102 k: 10 692 / 905 and 24 182 / 4 029).
 inline bool use_bounded_scan(int M, double visited, int nprobe, int k, int64_t nq) {
     if (M % 16 != 0 || M > 64 || k > 1024 || nprobe > kShortMaxProbe || visited < 2048.0) return false;
-    if (k > 48) return true;
-    if (M == 16) return false;
+    const double all = visited * static_cast<double>(nq);
+    if (k > 48) return k > 112 || all <= 3e8;
+    if (M == 16 || all > 1.3e8) return false;
     if (nq <= 64) return true;
     return visited >= 16384.0 && (nq <= 1024 || M == 64);
 }
