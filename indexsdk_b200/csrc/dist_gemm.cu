@@ -1179,8 +1179,14 @@ cudaError_t launch_one(const GemmLaunch& L, GemmArgs a, const CUtensorMap* mapA,
         if (worst <= 1.06 * ideal + 1.0) a.aligned_ranges = 1;
     }
     // In a short run most threads never see a candidate, and the blocks they reserved would be what the
-    // selection reads: 9 472 slots for the 150 candidates of one query against 100 003 rows.
-    a.eager = total >= 16LL * grid ? 1 : 0;
+    // selection reads: 9 472 slots for the 150 candidates of one query against 100 003 rows.  The same holds for
+    // one query block, whose rows every CTA has a share in.  us of a search on demand / ahead, fp32, d 128:
+    //   one query block, k = 10:  4 items a CTA 87 / 103, 16 items 115 / 129, 64 items 203 / 220; k = 100: 106 / 114, 142 / 144, 228 / 236
+    //   two, 32 items a CTA: k = 10 133 / 138, k = 100 170 / 160;  eight, 32 items: k = 10 151 / 148, k = 100 200 / 191
+    //   eight, 211 items (1 M rows): k = 10 389 / 366, k = 100 510 / 493;  79, 34 items (16 384 rows), k = 64: 324 / 312
+    //   below 16 items the two differ by less than 4 us from two query blocks on
+    // The rows of a segmented base belong to a few CTAs each, however few the query blocks.
+    a.eager = total >= 16LL * grid && (n_qb > 1 || a.seg_index) ? 1 : 0;
     kern<<<grid, gemm_threads(KIND), smem, stream>>>(*mapA, *mapB, a);
     return cudaGetLastError();
 }

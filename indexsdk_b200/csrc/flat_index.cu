@@ -272,9 +272,10 @@ FlatIndex::Plan FlatIndex::make_plan(int k, int64_t nq) const {
         p.cap = pow2_ceil(std::max<uint64_t>(whole ? 256 : 2048, want));
         // Candidate rows as long as the base itself save nothing in memory; they pay all the same once
         // there are many keys that would otherwise be refined and selected from one by one (300 000 queries
-        // against 256 rows of d 128, k = 1: 8.6 -> 0.8 ms; the second GEMM pass and the threshold cost a
-        // small call about 10 us, as much as 0.5 M keys do).
-        if (p.cap >= static_cast<uint64_t>(n_pad) && !(whole && nq * n_pad >= (int64_t(1) << 19))) p.sampled = false;
+        // against 256 rows of d 128, k = 1: 8.6 -> 0.8 ms).  us without / with a threshold, d 128, k = 1:
+        //   40 rows: 512 queries 50 / 54, 1 024 53 / 50, 2 048 60 / 51;  100 rows: 64 queries 50 / 52, 256 55 / 54, 1 024 65 / 50
+        //   256 rows: 16 queries 53 / 51, 64 60 / 51, 256 77 / 53, 2 048 127 / 52;  int8: 64 queries 46 / 40, 2 048 89 / 46
+        if (p.cap >= static_cast<uint64_t>(n_pad) && !(whole && nq * n_ >= (int64_t(1) << 14))) p.sampled = false;
     }
     if (!p.sampled) {
         p.burst = 32;
@@ -471,7 +472,11 @@ void FlatIndex::run_tail(const PageTail& t, bool fused) {
     const uint32_t n_fixed = static_cast<uint32_t>(n_);
     if (fused) {
         timer_.begin(kStageRefine, stream_);
-        B200_CUDA_CHECK(launch_finish_f32(cand, counts, t.cap, d_, eps, t.xq, x32_.as<float>(), over, nullptr, t.e, !t.prune && t.nq >= 4 * num_sms_, stream_));
+        // Short lists, a warp per query instead of a block: us block / warp, 16 384 rows,
+        //   k = 1: 148 queries 53 / 51, 1 184 70 / 62, 2 960 98 / 80;  k = 8: 148 55 / 53, 592 63 / 62, 2 960 108 / 88
+        //   k = 32: 148 queries 59 / 67, 592 63 / 68, 888 67 / 71, 1 184 78 / 75, 2 960 116 / 103
+        const bool few = !t.prune && t.nq >= (t.k <= 8 ? 1 : 8) * num_sms_;
+        B200_CUDA_CHECK(launch_finish_f32(cand, counts, t.cap, d_, eps, t.xq, x32_.as<float>(), over, nullptr, t.e, few, stream_));
         timer_.end(stream_);
         stats_.kernel_launches += 1;
         return;

@@ -120,3 +120,11 @@ def test_without_an_error_bound_every_key_is_looked_at(b200, metric, n, d, rows)
             out.append((D.cpu().numpy(), I.cpu().numpy()))
         np.testing.assert_array_equal(out[0][1], out[1][1])
         np.testing.assert_array_equal(out[0][0], out[1][0])
+
+
+# both sides of the lines by number of queries: thresholds for bases of one tile (2^14 keys), the warp form
+# (one query per SM up to k = 8, eight beyond)
+@pytest.mark.parametrize("n,d,nq,k", [(40, 64, 409, 1), (40, 64, 410, 1), (256, 64, 63, 1), (256, 64, 64, 1), (5000, 64, 147, 8),
+                                      (5000, 64, 148, 8), (5000, 64, 1183, 9), (5000, 64, 1184, 9)])
+def test_lines_by_number_of_queries(b200, n, d, nq, k):
+    _flat(b200, L2, datasets.gaussian(n, d, seed=1), datasets.gaussian(nq, d, seed=2), k)
