@@ -2301,7 +2301,8 @@ bool IvfpqIndex::search_pages(int64_t nq, const float* xq, int k, float* D, int6
     while (kpt * 32 < k + 16) kpt <<= 1;
     const bool fast = rotated_ && !force_exact_ && kpt <= 32;
     const double visited = static_cast<double>(nprobe) * n_ / nlist_;   // vectors a query meets on average
-    const bool bounded = r.bounded && !force_exact_ && (rotated_ ? use_bounded_scan(M_, visited, nprobe, k, nq)
+    const bool countable = !pre_cI || counts_fit(lens_host_.empty() ? 0 : *std::max_element(lens_host_.begin(), lens_host_.end()), nprobe);
+    const bool bounded = r.bounded && countable && !force_exact_ && (rotated_ ? use_bounded_scan(M_, visited, nprobe, k, nq)
                                                     : use_short_scan(M_, by_residual_, visited, nprobe, k));
     const int kprime = 32 * kpt;
     const int64_t page = 16384;

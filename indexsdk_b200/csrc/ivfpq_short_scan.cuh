@@ -85,6 +85,8 @@ inline bool use_bounded_scan(int M, double visited, int nprobe, int k, int64_t n
     if (nq <= 64) return true;
     return visited >= 16384.0 && (nq <= 1024 || M == 64);
 }
+// Given probes may name a list as often as they like, and a query's vectors are counted in 32 bits.
+inline bool counts_fit(int64_t longest_list, int nprobe) { return longest_list * nprobe <= 0xFFFFFFFFll; }
 cudaError_t launch_short_scan(const ShortScanArgs& a, int num_sms, cudaStream_t st);
 
 }  // namespace b200

@@ -42,6 +42,11 @@ int main() {
     small(false, 8, true, 1e6, 1025, 10);
     small(false, 8, true, 1e6, 8, 1025);
     small(false, 12, true, 1e6, 8, 10);
+    // given probes that all name one list of 2^22 vectors
+    if (!b200::counts_fit(1 << 22, 1023) || b200::counts_fit(1 << 22, 1024) || b200::counts_fit(int64_t(1) << 30, 1024)) {
+        std::printf("FAILED: counts of repeated lists\n");
+        ++failed;
+    }
     std::printf("%d failed\n", failed);
     return failed != 0;
 }
