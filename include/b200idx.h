@@ -108,11 +108,12 @@ int b200idx_search_multi(b200idx_t* const* hs, int nh, int64_t n, const void* x,
                          int64_t* labels, int merged);
 
 /* Counters of the segmented path of b200idx_search_multi on one device: small Flat / Int8Flat
- * indexes of a device are searched in one pass over their concatenated bases, the counterpart of
+ * indexes of a device are searched in one pass over all their bases, the counterpart of
  * the reference's single top-k operator over the blocks of all indexes
  * (FR/ops/cpukernel/impl/topk_multisearch_cpu_kernel.cpp:316-430).  group_launches: kernels
  * launched by that path so far (per call it does not depend on the number of indexes);
- * group_rebuilds: times the concatenated copy was (re)built -- it is kept until a member changes. */
+ * group_rebuilds: times the tables of the members (for row-major operands also a gathered copy of those)
+ * were (re)built -- they are kept until a member changes. */
 int b200idx_search_multi_stats(int device, uint64_t* group_launches, uint64_t* group_rebuilds);
 
 /* Merge of nsrc sorted per-shard results resident on one device: Din/Iin [nsrc][n][k] ->

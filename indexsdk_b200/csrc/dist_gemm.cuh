@@ -78,7 +78,7 @@ struct GemmArgs {
     uint32_t* counts;     // [nq] slots reserved (blocks of 8 per thread and query block run): >= candidates
     uint32_t cap;
     int eager;            // threshold mode: a thread reserves its first candidate block before it has a candidate
-                          // (filled in by launch_dist_gemm)
+                          // (filled in by launch_dist_gemm, where the rule stands)
     int direct;           // 1: slot = position (cap >= N, no atomics); 0: slot = atomic counter
     // optional per-(query, base row) filter: bit (row % 32) of qmask[q * qmask_stride + row / 32] = 1
     // lets the row take part (nullptr: every row does)
@@ -88,7 +88,7 @@ struct GemmArgs {
     // same queries in ONE pass (multi-index search).  A tile belongs to exactly one index (segments
     // start on tile boundaries); per tile:
     //   seg_index: which index; the candidates of (index i, query q) go to row
-    //              (i - seg_first) * nq + q of cand / tau (direct mode only)
+    //              (i - seg_first) * nq + q of cand / tau
     //   seg_col0 : position of the index's first base row (the slot of a
     //              candidate is its position minus this; burst minima count their slots from it too)
     //   seg_end  : position one past the index's last real base row

@@ -75,6 +75,7 @@ inline bool use_short_scan(int M, bool residual, double visited, int nprobe, int
 //   k = 10,  M = 48, 512 queries of 102 k: 1 032 / 863 and 5 377 / 3 074;   of 500 k: 2 969 / 3 565 and 11 385 / 9 881
 //   k = 100, M = 16, 512 queries of 500 k: 1 805 / 1 452 and 5 147 / 4 234; of 1.0 M: 2 778 / 2 950, of 3.0 M: 6 773 / 8 526
 //   k = 100, M = 48, 512 queries of 500 k: 3 736 / 3 577 and 12 869 / 9 909; of 1.0 M: 5 809 / 7 191
+//   k = 100, M = 48, 10 000 queries of 781 k (100 M vectors, 16 384 lists): 20.9 ms / 26.9
 // so the product of queries and vectors has a limit.  Longer lists (k > 112: k' of 256 and more) never catch up
 // in that range (k = 300, M = 48, 512 queries of 102 k: 10 692 / 905 and 24 182 / 4 029).
 inline bool use_bounded_scan(int M, double visited, int nprobe, int k, int64_t nq) {

@@ -25,8 +25,8 @@ class FlatGroup {
 public:
     explicit FlatGroup(int device) : device_(device) {}
     // Can these members (one device; same d / metric / dtype is the caller's contract) be searched
-    // as one group with nq queries?  Small indexes only: without thresholds every key of a member is
-    // written once.
+    // as one group with nq queries?  Small indexes only: tiny ones are searched without thresholds, and so is a
+    // call in which a row overflows, and then every key of a member is written once.
     static bool eligible(const std::vector<FlatIndex*>& members, int64_t nq, int k);
     // xq: device pointer, float rows (kF32 / kF16 members) or int8 rows.  D / I: device pointers
     // [members][nq][k].  Work is queued on `stream`; returns after synchronising it.  `then` may queue

@@ -35,9 +35,6 @@ struct TauFold {
 cudaError_t launch_kth_threshold(const uint32_t* mins, int stride, int n, int nq, int k, const float* eps,
                                  uint32_t tau_all, uint32_t* tau, const TauFold& fold, cudaStream_t stream);
 
-// fp32 refinement: replaces the key of every candidate by the canonical fp32 distance
-// (sequential fmaf over the dimension) computed from the fp32 rows; L2 -> distance,
-// IP -> negated dot product.
 // thresholded path, between two stretches of the full pass: tau[row] = min(tau[row], k-th smallest
 // key among the row's candidates so far (+ 2 eps[row] where eps is given: approximate keys))
 cudaError_t launch_tighten_tau(const uint64_t* cand, const uint32_t* counts, uint32_t cap, int nq, int k,
@@ -47,6 +44,9 @@ cudaError_t launch_tighten_tau(const uint64_t* cand, const uint32_t* counts, uin
 // is compacted and counts[row] updated
 cudaError_t launch_prune_candidates(uint64_t* cand, uint32_t* counts, uint32_t cap, int nq, int k,
                                     const float* eps, cudaStream_t stream);
+// fp32 refinement: replaces the key of every candidate by the canonical fp32 distance
+// (sequential fmaf over the dimension) computed from the fp32 rows; L2 -> distance,
+// IP -> negated dot product.  Overflowed rows are left alone.
 // q_mod > 0: candidate row r belongs to query r % q_mod (rows = [index][query] of a multi-index search)
 // and, where members (a device array) is given instead of xb, to member r / q_mod
 cudaError_t launch_refine_f32(uint64_t* cand, const uint32_t* counts, uint32_t n_fixed, uint32_t cap, int nq, int d,
