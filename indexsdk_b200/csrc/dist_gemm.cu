@@ -1185,8 +1185,10 @@ cudaError_t launch_one(const GemmLaunch& L, GemmArgs a, const CUtensorMap* mapA,
     //   two, 32 items a CTA: k = 10 133 / 138, k = 100 170 / 160;  eight, 32 items: k = 10 151 / 148, k = 100 200 / 191
     //   eight, 211 items (1 M rows): k = 10 389 / 366, k = 100 510 / 493;  79, 34 items (16 384 rows), k = 64: 324 / 312
     //   below 16 items the two differ by less than 4 us from two query blocks on
-    // The rows of a segmented base belong to a few CTAs each, however few the query blocks.
-    a.eager = total >= 16LL * grid && (n_qb > 1 || a.seg_index) ? 1 : 0;
+    // With many candidates a thread it turns round there, too (three and more: 41 queries, 831 508 x 128 int8,
+    // k = 113, 129 / 126).  The rows of a segmented base belong to a few CTAs each, however few the query blocks.
+    const bool shared = n_qb == 1 && !a.seg_index && a.row_cands < 3LL * 4 * grid;   // (four threads a row and CTA)
+    a.eager = total >= 16LL * grid && !shared ? 1 : 0;
     kern<<<grid, gemm_threads(KIND), smem, stream>>>(*mapA, *mapB, a);
     return cudaGetLastError();
 }

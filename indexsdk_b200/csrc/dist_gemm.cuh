@@ -77,6 +77,7 @@ struct GemmArgs {
     uint64_t* cand;       // [nq][cap] packed (ordered key, position); reserved but unused slots hold "invalid"
     uint32_t* counts;     // [nq] slots reserved (blocks of 8 per thread and query block run): >= candidates
     uint32_t cap;
+    int row_cands;        // threshold mode: candidates a row is to expect (0: unknown), for the rule of eager
     int eager;            // threshold mode: a thread reserves its first candidate block before it has a candidate
                           // (filled in by launch_dist_gemm, where the rule stands)
     int direct;           // 1: slot = position (cap >= N, no atomics); 0: slot = atomic counter

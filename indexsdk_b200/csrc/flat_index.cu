@@ -382,6 +382,7 @@ FlatIndex::PageTail FlatIndex::run_page(int nq, const void* xq_raw, const void* 
         stats_.gemm_launches += 1;
         stats_.kernel_launches += 2;
         a.direct = 0;
+        a.row_cands = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(k) * a.n_tiles_total / plan.s_tiles, int64_t(1) << 30));
     } else {
         B200_CUDA_CHECK(launch_fill_u32(tau, nq, tau_all, stream_));
         B200_CUDA_CHECK(cudaMemsetAsync(cand, 0xFF, static_cast<size_t>(nq) * plan.cap * 8, stream_));

@@ -206,9 +206,10 @@ void FlatGroup::run_passes(Pass pass, int nq, const void* xq, const void* xq_op,
         // 38 -> 14 us, the end 26 -> 34).  How many depends on the queries, whose candidates all have to be
         // refined.  us with every tile / every fourth, 32 members, by bursts / k:
         //   1 query:     8: 136 / 129 (5 000 rows: 100 / 104), 16: 124 / 114, 30: 160 / 138, 61: 152 / 131
-        //   64 queries:  8: 177 / 188, 16: 158 / 167, 30: 189 / 188, 61: 181 / 166;  of 16 members: 62: 175 / 160
+        //   64 queries:  8: 177 / 188, 16: 158 / 167, 30: 189 / 188, 61: 181 / 166;  of 16 members: 62: 175 / 160;
+        //                74 of 59 members of 5 400 x 256: 32: 312 / 298
         //   512 queries: 16: 402 / 516, 32: 368 / 404, 61: 480 / 497;  of 16 members: 62: 431 / 423, 125: 404 / 387
-        const int64_t per_k = std::max(8, std::min(64, nq / 2));
+        const int64_t per_k = std::max(8, std::min(64, nq / 3));
         if ((least / kTileB) / 4 * (kTileB / 8) >= per_k * k) step = 4;
         if (least / kTileB / step * (kTileB / 32) < 8LL * k) burst = 8;
         // Room for 9 k keys, and for the slots the epilogue's threads reserve in blocks of 8 and leave
